@@ -9,4 +9,6 @@ namespace atag {
 atag_status set_error(atag_status s, const char* msg);
 // Adds one to the launch counter reported by atag_launch_count().
 void count_launch();
+// SMs of the calling thread's current device (0 before atag_init succeeded on it).
+int device_sms();
 }  // namespace atag

@@ -269,6 +269,10 @@ StageClusterLayout layout_stage_cluster(char* base, uint32_t w, uint32_t h, uint
 namespace atag {
 atag_status set_error(atag_status s, const char* msg) { return fail(s, "%s", msg); }
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
+int device_sms() {
+    DeviceInfo* d;
+    return ensure_device(&d) ? 0 : d->num_sms;
+}
 }  // namespace atag
 
 // ===========================================================================

@@ -22,7 +22,18 @@
 // intensities per quad; backward recomputes the forward and propagates
 // dL/d(refined corners) and dL/d(residuals) to dL/d(corners), dL/d(samples)
 // and, optionally, dL/d(image) (scattered through the bilinear weights).
-// One 128-thread CTA per quad, one warp per edge, two samples per lane.
+//
+// A warp takes an edge (two samples per lane); the FP64 part of an edge (the
+// eigen-solve, the intersections and their adjoints) has no lane-level
+// parallelism, and on this GPU FP64 issues at 2 lanes per clock and SM
+// whether a warp's lanes do different work or the same.  So the edges' moments
+// go through shared memory, and one warp of the CTA takes all of its edges'
+// FP64 parts at once, lane = edge (up to 32 edges of 8 quads).  With every
+// lane of every edge's warp solving its own edge redundantly, the FP64 pipe
+// was 80-85% busy: 4,096 quads took 167 us forward and 339 us backward, and
+// take 22 and 64 us now (single launches, cold caches).
+#include <algorithm>
+
 #include "atag_internal.h"
 #include "atag_kernels.cuh"
 
@@ -75,30 +86,41 @@ __device__ __forceinline__ void bilinear_scatter(float* __restrict__ gimg, int w
     atomicAdd(gimg + (size_t)(y0 + 1) * w + x0 + 1, g * fx * fy);
 }
 
-// Per-edge geometry and the line fit of one warp.
+constexpr int RF_WARPS = 4, RF_QUADS = 8, RF_EDGES = 4 * RF_QUADS;
+
+// The fitted line of an edge, FP64.
 struct EdgeLine {
-    double mx, my, ux, uy, r;                       // line and residual
+    double mx, my, ux, uy;                          // line
     double S0, Sx, Sy, Sxx, Syy, Sxy;               // moments about (ox, oy)
-    double ox, oy;
-    double cxx, cyy, cxy, phi, R, lam;
+    double cxx, cyy, cxy;
+};
+
+// What an edge's warp hands to the FP64 lane, and what it gets back.
+struct EdgeSums {
+    float m6[6], ox, oy, dx, dy, nx, ny;
+    float pad_;  // 13 words: lanes of the FP64 warp read distinct banks
+};
+struct EdgeFit {
+    float cs, cn, c0;      // distance of q_j to the line: sa cs + o cn - c0
+    float nux, nuy;        // its normal
 };
 
 struct LaneState {
     // position j = lane / 2 owns taps 2*(lane&1) .. +1
-    float ax, ay, bx, by, dx, dy, nx, ny, len, t;
+    float dx, dy, nx, ny, len, t;
     Bilinear s[2];
     float sx[2], sy[2];
     // position-level values (valid on even lanes)
     float v[4], gd[3], w[3], Om, Nn, o, W;
     float sa;              // (t_j - 1/2) |b - a|: q_j - midpoint = sa d + o n
-    float nux, nuy, dist;  // normal of the fitted line, distance of q_j to it
 };
 
+// FP32 part of an edge on its warp: samples, edge points and the moments of
+// the line fit (in S, written by lane 0).
 template <class Img>
-__device__ __forceinline__ void edge_forward(const Img& img, int iw, int ih, float ax, float ay, float bx,
-                                             float by, LaneState& L, EdgeLine& E) {
+__device__ __forceinline__ void edge_samples(const Img& img, int iw, int ih, float ax, float ay, float bx, float by,
+                                             LaneState& L, EdgeSums& S) {
     const int lane = threadIdx.x & 31, j = lane >> 1, half = lane & 1;
-    L.ax = ax; L.ay = ay; L.bx = bx; L.by = by;
     const float Dx = bx - ax, Dy = by - ay;
     L.len = fmaxf(sqrtf(Dx * Dx + Dy * Dy), 1e-6f);
     L.dx = Dx / L.len;
@@ -142,82 +164,131 @@ __device__ __forceinline__ void edge_forward(const Img& img, int iw, int ih, flo
     for (int k = 0; k < 6; k++)
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) m6[k] += __shfl_xor_sync(0xffffffffu, m6[k], off);
-    // FP64 eigen-solve of the 2x2 covariance (every lane, identical values)
-    E.ox = ox; E.oy = oy;
-    E.S0 = fmax((double)m6[0], 1e-30);
-    E.Sx = m6[1]; E.Sy = m6[2]; E.Sxx = m6[3]; E.Syy = m6[4]; E.Sxy = m6[5];
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < 6; k++) S.m6[k] = m6[k];
+        S.ox = ox; S.oy = oy;
+        S.dx = L.dx; S.dy = L.dy; S.nx = L.nx; S.ny = L.ny;
+    }
+}
+
+// FP64 part of an edge on one lane: the eigen-solve of the 2x2 covariance.
+// The direction of the larger eigenvalue, (cos phi, sin phi) with phi =
+// atan2(2 cxy, cxx - cyy) / 2, follows without trigonometry from the
+// eigenvector (R + h, cxy) or, for h < 0, (|cxy|, +-(R - h)), h = (cxx - cyy)
+// / 2, R = sqrt(h^2 + cxy^2): both components are sums of terms of one sign.
+__device__ __forceinline__ void solve_line(const EdgeSums& S, EdgeLine& E, EdgeFit& fit) {
+    E.S0 = fmax((double)S.m6[0], 1e-30);
+    E.Sx = S.m6[1]; E.Sy = S.m6[2]; E.Sxx = S.m6[3]; E.Syy = S.m6[4]; E.Sxy = S.m6[5];
     const double mx = E.Sx / E.S0, my = E.Sy / E.S0;
     E.cxx = E.Sxx / E.S0 - mx * mx;
     E.cyy = E.Syy / E.S0 - my * my;
     E.cxy = E.Sxy / E.S0 - mx * my;
-    E.phi = 0.5 * atan2(2.0 * E.cxy, E.cxx - E.cyy);
-    const double h2 = 0.5 * (E.cxx - E.cyy);
-    E.R = sqrt(h2 * h2 + E.cxy * E.cxy);
-    E.lam = 0.5 * (E.cxx + E.cyy) - E.R;
-    E.mx = (double)ox + mx;
-    E.my = (double)oy + my;
-    E.ux = cos(E.phi);
-    E.uy = sin(E.phi);
+    const double h = 0.5 * (E.cxx - E.cyy);
+    const double R = sqrt(h * h + E.cxy * E.cxy);
+    const double vx = h >= 0.0 ? R + h : fabs(E.cxy), vy = h >= 0.0 ? E.cxy : copysign(R - h, E.cxy);
+    const double len = sqrt(vx * vx + vy * vy);
+    E.mx = (double)S.ox + mx;
+    E.my = (double)S.oy + my;
+    E.ux = len == 0.0 ? 1.0 : vx / len;
+    E.uy = len == 0.0 ? 0.0 : vy / len;
     // residual sum W_j d_j^2 of the perpendicular distances to the fitted
     // line, in a second pass (S0 * lambda_min from the moments would
     // cancel), in the edge frame: d_j = sa (d.nu) + o (n.nu) - (m.nu), whose
     // terms are small where the line runs along the edge
     const double nux = -E.uy, nuy = E.ux;
-    L.nux = (float)nux;
-    L.nuy = (float)nuy;
-    const float cs = (float)((double)L.dx * nux + (double)L.dy * nuy);
-    const float cn = (float)((double)L.nx * nux + (double)L.ny * nuy);
-    const float c0 = (float)(mx * nux + my * nuy);
-    L.dist = L.sa * cs + L.o * cn - c0;
-    float rr = half ? 0.0f : L.W * L.dist * L.dist;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) rr += __shfl_xor_sync(0xffffffffu, rr, off);
-    E.r = rr;
+    fit.nux = (float)nux;
+    fit.nuy = (float)nuy;
+    fit.cs = (float)((double)S.dx * nux + (double)S.dy * nuy);
+    fit.cn = (float)((double)S.nx * nux + (double)S.ny * nuy);
+    fit.c0 = (float)(mx * nux + my * nuy);
 }
 
 // Intersection of line A (m_A + alpha u_A) with line B, FP64.
-__device__ __forceinline__ void intersect(const EdgeLine& A, const EdgeLine& B, double& cx, double& cy, double& alpha,
-                                          double& P, double& Q) {
-    const double Dx = B.mx - A.mx, Dy = B.my - A.my;
-    P = B.ux * Dy - B.uy * Dx;
-    Q = B.ux * A.uy - B.uy * A.ux;
-    alpha = P / Q;
-    cx = A.mx + alpha * A.ux;
-    cy = A.my + alpha * A.uy;
+struct Crossing {
+    double cx, cy, alpha, P, Q, Dx, Dy;
+};
+__device__ __forceinline__ Crossing intersect(double amx, double amy, double aux, double auy, const EdgeLine& B) {
+    Crossing X;
+    X.Dx = B.mx - amx;
+    X.Dy = B.my - amy;
+    X.P = B.ux * X.Dy - B.uy * X.Dx;
+    X.Q = B.ux * auy - B.uy * aux;
+    X.alpha = X.P / X.Q;
+    X.cx = amx + X.alpha * aux;
+    X.cy = amy + X.alpha * auy;
+    return X;
+}
+// Lane 4 q + i of the FP64 warp: corner i of quad q, the crossing of lines
+// i - 1 (A, fetched from its lane) and i (B, this lane's).
+__device__ __forceinline__ Crossing corner_of(const EdgeLine& E, double* aux, double* auy) {
+    const int lane = threadIdx.x & 31, prev = (lane & ~3) | ((lane + 3) & 3);
+    const double amx = __shfl_sync(0xffffffffu, E.mx, prev), amy = __shfl_sync(0xffffffffu, E.my, prev);
+    *aux = __shfl_sync(0xffffffffu, E.ux, prev);
+    *auy = __shfl_sync(0xffffffffu, E.uy, prev);
+    return intersect(amx, amy, *aux, *auy, E);
+}
+
+// Quads per CTA: four CTAs per SM put one FP64 warp on each of its four
+// schedulers (the FP64 warp's index turns with the CTA), and few quads spread
+// over the SMs one by one.
+inline unsigned refine_quads_per_cta(size_t n) {
+    const size_t slots = 4 * (size_t)device_sms();
+    return (unsigned)std::min<size_t>(RF_QUADS, (n + slots - 1) / slots);
 }
 
 }  // namespace
 
-__global__ void __launch_bounds__(128) k_refine_forward(const float* __restrict__ img, int iw, int ih,
-                                                        const float* __restrict__ corners, int nq,
+__global__ void __launch_bounds__(32 * RF_WARPS) k_refine_forward(const float* __restrict__ img, int iw, int ih,
+                                                        const float* __restrict__ corners, int nq, int qpc,
                                                         float* __restrict__ refined, float* __restrict__ residual,
                                                         float* __restrict__ samples) {
-    __shared__ EdgeLine lines[4];
-    const int q = blockIdx.x;
-    if (q >= nq) return;
-    const int e = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const float* c = corners + (size_t)q * 8;
-    const int e1 = (e + 1) & 3;
-    LaneState L;
-    EdgeLine E;
-    edge_forward(F32Image{img}, iw, ih, c[2 * e], c[2 * e + 1], c[2 * e1], c[2 * e1 + 1], L, E);
-    if (samples) {
-        const int j = lane >> 1, half = lane & 1;
-        float* s = samples + ((size_t)q * 4 + e) * (RF_POS * RF_TAPS) + j * RF_TAPS + 2 * half;
-        s[0] = L.s[0].v;
-        s[1] = L.s[1].v;
-    }
-    if (lane == 0) {
-        lines[e] = E;
-        if (residual) residual[(size_t)q * 4 + e] = (float)E.r;
+    __shared__ EdgeSums sums[RF_EDGES];
+    __shared__ EdgeFit fits[RF_EDGES];
+    __shared__ float pos[RF_EDGES][RF_POS][3];  // sa, o, W of each position
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t q0 = (size_t)blockIdx.x * qpc;
+    const int ne = 4 * min(qpc, nq - (int)q0);
+    for (int k = warp; k < ne; k += RF_WARPS) {
+        const int e = k & 3, e1 = (e + 1) & 3, j = lane >> 1, half = lane & 1;
+        const float* c = corners + (q0 + (k >> 2)) * 8;
+        LaneState L;
+        edge_samples(F32Image{img}, iw, ih, c[2 * e], c[2 * e + 1], c[2 * e1], c[2 * e1 + 1], L, sums[k]);
+        if (samples) {
+            float* s = samples + (q0 * 4 + k) * (RF_POS * RF_TAPS) + j * RF_TAPS + 2 * half;
+            s[0] = L.s[0].v;
+            s[1] = L.s[1].v;
+        }
+        if (!half) {
+            pos[k][j][0] = L.sa;
+            pos[k][j][1] = L.o;
+            pos[k][j][2] = L.W;
+        }
     }
     __syncthreads();
-    if (threadIdx.x < 4) {
-        const int i = threadIdx.x;
-        double cx, cy, alpha, P, Q;
-        intersect(lines[(i + 3) & 3], lines[i], cx, cy, alpha, P, Q);
-        refined[(size_t)q * 8 + 2 * i] = (float)cx;
-        refined[(size_t)q * 8 + 2 * i + 1] = (float)cy;
+    if (warp == (blockIdx.x & (RF_WARPS - 1))) {
+        EdgeLine E;
+        EdgeFit fit;
+        solve_line(sums[min(lane, ne - 1)], E, fit);
+        double aux, auy;
+        const Crossing X = corner_of(E, &aux, &auy);
+        if (lane < ne) {
+            fits[lane] = fit;
+            refined[q0 * 8 + 2 * lane] = (float)X.cx;
+            refined[q0 * 8 + 2 * lane + 1] = (float)X.cy;
+        }
+    }
+    if (!residual) return;
+    __syncthreads();
+    for (int k = warp; k < ne; k += RF_WARPS) {
+        const int j = lane >> 1, half = lane & 1;
+        const float sa = pos[k][j][0], o = pos[k][j][1], W = pos[k][j][2];
+        const EdgeFit f = fits[k];
+        const float dist = sa * f.cs + o * f.cn - f.c0;
+        float rr = half ? 0.0f : W * dist * dist;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) rr += __shfl_xor_sync(0xffffffffu, rr, off);
+        if (lane == 0) residual[q0 * 4 + k] = rr;
     }
 }
 
@@ -227,182 +298,200 @@ __global__ void __launch_bounds__(128) k_refine_forward(const float* __restrict_
 // A corner whose two edge lines are nearly parallel (|sin| of their angle
 // at most 1e-3) keeps its unrefined position.  Frame blockIdx.x; its quads
 // blockIdx.y, blockIdx.y + gridDim.y, ...
-__global__ void __launch_bounds__(128) k_refine_detected(const __grid_constant__ FrameSet fs) {
-    __shared__ EdgeLine lines[4];
-    __shared__ float s_c[8];
+__global__ void __launch_bounds__(32 * RF_WARPS) k_refine_detected(const __grid_constant__ FrameSet fs) {
+    __shared__ EdgeSums sums[4];
     const FrameDesc& F = fs.get(blockIdx.x);
     const uint32_t nq = min(F.stats->n_quads, F.quad_cap);
     const U8Image img{F.grey};
     const int e = threadIdx.x >> 5, lane = threadIdx.x & 31, e1 = (e + 1) & 3;
     for (uint32_t q = blockIdx.y; q < nq; q += gridDim.y) {
         atag_quad_corners* qc = F.quads + q;
-        if (threadIdx.x < 8) s_c[threadIdx.x] = qc->corners[threadIdx.x >> 1][threadIdx.x & 1];
-        __syncthreads();
+        const float ax = qc->corners[e][0], ay = qc->corners[e][1], bx = qc->corners[e1][0], by = qc->corners[e1][1];
         LaneState L;
-        EdgeLine E;
-        edge_forward(img, (int)F.width, (int)F.height, s_c[2 * e], s_c[2 * e + 1], s_c[2 * e1], s_c[2 * e1 + 1], L, E);
-        if (lane == 0) lines[e] = E;
-        __syncthreads();
-        if (threadIdx.x < 4) {
-            const int i = threadIdx.x;
-            double cx, cy, alpha, P, Q;
-            intersect(lines[(i + 3) & 3], lines[i], cx, cy, alpha, P, Q);
-            if (fabs(Q) > 1e-3 && isfinite(cx) && isfinite(cy)) {
-                qc->corners[i][0] = (float)cx;
-                qc->corners[i][1] = (float)cy;
+        edge_samples(img, (int)F.width, (int)F.height, ax, ay, bx, by, L, sums[e]);
+        __syncthreads();  // also: every warp has read the corners
+        if (e == (int)(blockIdx.y & (RF_WARPS - 1))) {
+            EdgeLine E;
+            EdgeFit fit;
+            solve_line(sums[lane & 3], E, fit);
+            double aux, auy;
+            const Crossing X = corner_of(E, &aux, &auy);
+            if (lane < 4 && fabs(X.Q) > 1e-3 && isfinite(X.cx) && isfinite(X.cy)) {
+                qc->corners[lane][0] = (float)X.cx;
+                qc->corners[lane][1] = (float)X.cy;
             }
         }
         __syncthreads();
     }
 }
 
-__global__ void __launch_bounds__(128) k_refine_backward(const float* __restrict__ img, int iw, int ih,
-                                                         const float* __restrict__ corners, int nq,
+// What the FP64 lane of an edge hands back for the adjoint: the adjoints of
+// its moments, of the origin (through the centroid) and of its residual.
+struct EdgeAdjoint {
+    double gS0, gSx, gSy, gSxx, gSyy, gSxy;
+    float gox, goy, gr;
+};
+
+__global__ void __launch_bounds__(32 * RF_WARPS) k_refine_backward(const float* __restrict__ img, int iw, int ih,
+                                                         const float* __restrict__ corners, int nq, int qpc,
                                                          const float* __restrict__ g_refined,
                                                          const float* __restrict__ g_residual,
                                                          float* __restrict__ g_corners, float* __restrict__ g_samples,
                                                          float* __restrict__ g_image) {
-    __shared__ EdgeLine lines[4];
-    __shared__ double gm[4][2], gu[4][2];   // adjoints of each line's centroid and direction
-    __shared__ float gc[4][2];              // adjoints of the input corners
-    const int q = blockIdx.x;
-    if (q >= nq) return;
-    const int e = threadIdx.x >> 5, lane = threadIdx.x & 31, j = lane >> 1, half = lane & 1;
-    const float* c = corners + (size_t)q * 8;
-    const int e1 = (e + 1) & 3;
-    LaneState L;
-    EdgeLine E;
-    edge_forward(F32Image{img}, iw, ih, c[2 * e], c[2 * e + 1], c[2 * e1], c[2 * e1 + 1], L, E);
-    if (lane == 0) lines[e] = E;
-    if (threadIdx.x < 8) {
-        (&gm[0][0])[threadIdx.x] = 0.0;
-        (&gu[0][0])[threadIdx.x] = 0.0;
-        (&gc[0][0])[threadIdx.x] = 0.0f;
-    }
-    __syncthreads();
-    // corner i = intersection(line i-1 (A), line i (B))
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < 4; i++) {
-            const int a = (i + 3) & 3, b = i;
-            const EdgeLine &A = lines[a], &B = lines[b];
-            double cx, cy, alpha, P, Q;
-            intersect(A, B, cx, cy, alpha, P, Q);
-            const double gcx = g_refined ? (double)g_refined[(size_t)q * 8 + 2 * i] : 0.0;
-            const double gcy = g_refined ? (double)g_refined[(size_t)q * 8 + 2 * i + 1] : 0.0;
-            gm[a][0] += gcx;
-            gm[a][1] += gcy;
-            gu[a][0] += alpha * gcx;
-            gu[a][1] += alpha * gcy;
-            const double ga = gcx * A.ux + gcy * A.uy;
-            const double gP = ga / Q, gQ = -ga * P / (Q * Q);
-            const double Dx = B.mx - A.mx, Dy = B.my - A.my;
-            // P = uBx Dy - uBy Dx
-            gu[b][0] += gP * Dy;
-            gu[b][1] += -gP * Dx;
-            const double gDx = -gP * B.uy, gDy = gP * B.ux;
-            // Q = uBx uAy - uBy uAx
-            gu[b][0] += gQ * A.uy;
-            gu[b][1] += -gQ * A.ux;
-            gu[a][0] += -gQ * B.uy;
-            gu[a][1] += gQ * B.ux;
-            gm[b][0] += gDx;
-            gm[b][1] += gDy;
-            gm[a][0] -= gDx;
-            gm[a][1] -= gDy;
+    __shared__ EdgeSums sums[RF_EDGES];
+    __shared__ EdgeFit fits[RF_EDGES];
+    __shared__ EdgeAdjoint adj[RF_EDGES];
+    __shared__ float gc[RF_EDGES][2];       // adjoints of the input corners
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, j = lane >> 1, half = lane & 1;
+    const size_t q0 = (size_t)blockIdx.x * qpc;
+    const int ne = 4 * min(qpc, nq - (int)q0);
+    if (threadIdx.x < 2 * RF_EDGES) (&gc[0][0])[threadIdx.x] = 0.0f;
+    // pass 0 gathers the moments of the CTA's edges; pass 1, with their
+    // adjoints, repeats an edge's FP32 forward (its pixels are in L1) rather
+    // than keeping its lanes' states
+#pragma unroll 1
+    for (int pass = 0; pass < 2; pass++) {
+        for (int k = warp; k < ne; k += RF_WARPS) {
+            const int e = k & 3, e1 = (e + 1) & 3;
+            const float* c = corners + (q0 + (k >> 2)) * 8;
+            LaneState L;
+            edge_samples(F32Image{img}, iw, ih, c[2 * e], c[2 * e + 1], c[2 * e1], c[2 * e1 + 1], L, sums[k]);
+            if (pass == 0) continue;
+            const EdgeFit f = fits[k];
+            const EdgeAdjoint& G = adj[k];
+            const float dist = L.sa * f.cs + L.o * f.cn - f.c0;
+            // moments -> edge point q_j and weight W_j (even lanes own position j)
+            const float X = L.sa * L.dx + L.o * L.nx, Y = L.sa * L.dy + L.o * L.ny;
+            const float grf = G.gr;
+            float gW = (float)(G.gS0 + G.gSx * X + G.gSy * Y + G.gSxx * X * X + G.gSyy * Y * Y + G.gSxy * X * Y) +
+                       grf * dist * dist;
+            float gqx = (float)(L.W * (G.gSx + 2.0 * G.gSxx * X + G.gSxy * Y)) + grf * 2.0f * L.W * dist * f.nux;
+            float gqy = (float)(L.W * (G.gSy + 2.0 * G.gSyy * Y + G.gSxy * X)) + grf * 2.0f * L.W * dist * f.nuy;
+            // X = q_x - o_x with q = p + o n and o the midpoint (the forward
+            // evaluates the same quantity as sa d_x + o n_x)
+            float gox = -gqx, goy = -gqy;
+            float gpx = gqx, gpy = gqy;
+            const float go = gqx * L.nx + gqy * L.ny;
+            float gnx = L.o * gqx, gny = L.o * gqy;
+            const float den_o = L.Om + RF_EPS;
+            const float gN = go / den_o;
+            const float gOm = gW - go * L.Nn / (den_o * den_o);
+            float gv[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int m = 0; m < 3; m++) {
+                const float gw = gN * (float)(m - 1) + gOm;
+                const float ggd = 2.0f * L.gd[m] * gw;
+                gv[m + 1] += ggd;
+                gv[m] -= ggd;
+            }
+            if (half) {  // only even lanes carry position-level adjoints
+                gpx = gpy = gnx = gny = gox = goy = 0.0f;
+                gv[0] = gv[1] = gv[2] = gv[3] = 0.0f;
+            }
+            if (lane == 0) {  // the line's centroid is origin + S_x / S_0: direct path to the origin
+                gox += G.gox;
+                goy += G.goy;
+            }
+            // hand the adjoints of taps 2, 3 to the odd lane
+            const float t2 = __shfl_xor_sync(0xffffffffu, gv[2], 1), t3 = __shfl_xor_sync(0xffffffffu, gv[3], 1);
+            const float gs0 = half ? t2 : gv[0], gs1 = half ? t3 : gv[1];
+            if (g_samples) {
+                float* s = g_samples + (q0 * 4 + k) * (RF_POS * RF_TAPS) + j * RF_TAPS + 2 * half;
+                s[0] = gs0;
+                s[1] = gs1;
+            }
+            // samples -> sample positions -> p_j, n
+            const float gsv[2] = {gs0, gs1};
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const float u = RF_U[2 * half + i];
+                const float gx = gsv[i] * L.s[i].gx, gy = gsv[i] * L.s[i].gy;
+                gpx += gx;
+                gpy += gy;
+                gnx += u * gx;
+                gny += u * gy;
+                if (g_image) bilinear_scatter(g_image, iw, ih, L.sx[i], L.sy[i], gsv[i]);
+            }
+            // p = a + t (b - a); origin = (a + b) / 2; n = (-d_y, d_x), d = (b - a) / |b - a|
+            float gax = (1.0f - L.t) * gpx + 0.5f * gox, gay = (1.0f - L.t) * gpy + 0.5f * goy;
+            float gbx = L.t * gpx + 0.5f * gox, gby = L.t * gpy + 0.5f * goy;
+            const float gdx = gny, gdy = -gnx;
+            const float dd = L.dx * gdx + L.dy * gdy;
+            const float gDx = (gdx - L.dx * dd) / L.len, gDy = (gdy - L.dy * dd) / L.len;
+            gax -= gDx; gay -= gDy; gbx += gDx; gby += gDy;
+            float acc[4] = {gax, gay, gbx, gby};
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], off);
+            if (lane == 0) {  // two edges add to each corner
+                atomicAdd(&gc[k][0], acc[0]);
+                atomicAdd(&gc[k][1], acc[1]);
+                atomicAdd(&gc[(k & ~3) | e1][0], acc[2]);
+                atomicAdd(&gc[(k & ~3) | e1][1], acc[3]);
+            }
+        }
+        __syncthreads();
+        if (pass == 0) {
+            if (warp == (blockIdx.x & (RF_WARPS - 1))) {
+                EdgeLine E;
+                EdgeFit fit;
+                const int k = min(lane, ne - 1);
+                solve_line(sums[k], E, fit);
+                // adjoint of corner i (this lane), the crossing of lines A = i - 1
+                // (the lane before in its quad) and B = i (this lane's own)
+                double aux, auy;
+                const Crossing C = corner_of(E, &aux, &auy);
+                const double gcx = g_refined ? (double)g_refined[q0 * 8 + 2 * k] : 0.0;
+                const double gcy = g_refined ? (double)g_refined[q0 * 8 + 2 * k + 1] : 0.0;
+                const double ga = gcx * aux + gcy * auy;
+                const double gP = ga / C.Q, gQ = -ga * C.P / (C.Q * C.Q);
+                const double gDx = -gP * E.uy, gDy = gP * E.ux;
+                // Q = uBx uAy - uBy uAx, P = uBx Dy - uBy Dx
+                double gmx_a = gcx - gDx, gmy_a = gcy - gDy;
+                double gux_a = C.alpha * gcx - gQ * E.uy, guy_a = C.alpha * gcy + gQ * E.ux;
+                // line i's adjoints: as B of its own corner, as A of the next lane's
+                const int next = (lane & ~3) | ((lane + 1) & 3);
+                gmx_a = __shfl_sync(0xffffffffu, gmx_a, next);
+                gmy_a = __shfl_sync(0xffffffffu, gmy_a, next);
+                gux_a = __shfl_sync(0xffffffffu, gux_a, next);
+                guy_a = __shfl_sync(0xffffffffu, guy_a, next);
+                const double gmx0 = gDx + gmx_a, gmy0 = gDy + gmy_a;
+                const double gux = gP * C.Dy + gQ * auy + gux_a, guy = -gP * C.Dx - gQ * aux + guy_a;
+                // line adjoint -> moment adjoints
+                const double gphi = -E.uy * gux + E.ux * guy;
+                const double Xc = E.cxx - E.cyy, Yc = 2.0 * E.cxy, den = Xc * Xc + Yc * Yc;
+                double gcxx = 0, gcyy = 0, gcxy = 0;
+                if (den > 1e-300) {
+                    const double s = gphi / den;
+                    gcxy = s * Xc;
+                    gcxx = -0.5 * s * Yc;
+                    gcyy = 0.5 * s * Yc;
+                }
+                // the residual's gradient needs no path through the line: the line
+                // minimises sum W d^2, so only q_j and W_j move it (envelope theorem)
+                const double is = 1.0 / E.S0, mx = E.Sx * is, my = E.Sy * is;
+                const double gmx = gmx0 - 2.0 * mx * gcxx - my * gcxy;
+                const double gmy = gmy0 - 2.0 * my * gcyy - mx * gcxy;
+                if (lane < ne) {
+                    fits[lane] = fit;
+                    EdgeAdjoint G;
+                    G.gSxx = gcxx * is;
+                    G.gSyy = gcyy * is;
+                    G.gSxy = gcxy * is;
+                    G.gSx = gmx * is;
+                    G.gSy = gmy * is;
+                    G.gS0 = -(E.Sxx * gcxx + E.Syy * gcyy + E.Sxy * gcxy + E.Sx * gmx + E.Sy * gmy) * (is * is);
+                    G.gox = (float)gmx0;
+                    G.goy = (float)gmy0;
+                    G.gr = g_residual ? g_residual[q0 * 4 + lane] : 0.0f;
+                    adj[lane] = G;
+                }
+            }
+            __syncthreads();
         }
     }
-    __syncthreads();
-    // line adjoint -> moment adjoints (all lanes compute the same doubles)
-    const double gr = g_residual ? (double)g_residual[(size_t)q * 4 + e] : 0.0;
-    const double gphi = -sin(E.phi) * gu[e][0] + cos(E.phi) * gu[e][1];
-    const double Xc = E.cxx - E.cyy, Yc = 2.0 * E.cxy, den = Xc * Xc + Yc * Yc;
-    double gcxx = 0, gcyy = 0, gcxy = 0;
-    if (den > 1e-300) {
-        gcxy += gphi * Xc / den;
-        gcxx += -0.5 * gphi * Yc / den;
-        gcyy -= -0.5 * gphi * Yc / den;
-    }
-    // the residual's gradient needs no path through the line: the line
-    // minimises sum W d^2, so only q_j and W_j move it (envelope theorem)
-    double gS0 = 0.0;
-    const double mx = E.Sx / E.S0, my = E.Sy / E.S0;
-    const double gmx = gm[e][0] - 2.0 * mx * gcxx - my * gcxy;
-    const double gmy = gm[e][1] - 2.0 * my * gcyy - mx * gcxy;
-    const double gSxx = gcxx / E.S0, gSyy = gcyy / E.S0, gSxy = gcxy / E.S0;
-    const double gSx = gmx / E.S0, gSy = gmy / E.S0;
-    gS0 += -(E.Sxx * gcxx + E.Syy * gcyy + E.Sxy * gcxy + E.Sx * gmx + E.Sy * gmy) / (E.S0 * E.S0);
-    // moments -> edge point q_j and weight W_j (even lanes own position j)
-    const float X = L.sa * L.dx + L.o * L.nx, Y = L.sa * L.dy + L.o * L.ny;
-    const float grf = (float)gr;
-    float gW = (float)(gS0 + gSx * X + gSy * Y + gSxx * X * X + gSyy * Y * Y + gSxy * X * Y) +
-               grf * L.dist * L.dist;
-    float gqx = (float)(L.W * (gSx + 2.0 * gSxx * X + gSxy * Y)) + grf * 2.0f * L.W * L.dist * L.nux;
-    float gqy = (float)(L.W * (gSy + 2.0 * gSyy * Y + gSxy * X)) + grf * 2.0f * L.W * L.dist * L.nuy;
-    // X = q_x - o_x with q = p + o n and o the midpoint (the forward
-    // evaluates the same quantity as sa d_x + o n_x)
-    float gox = -gqx, goy = -gqy;
-    float gpx = gqx, gpy = gqy;
-    const float go = gqx * L.nx + gqy * L.ny;
-    float gnx = L.o * gqx, gny = L.o * gqy;
-    const float den_o = L.Om + RF_EPS;
-    const float gN = go / den_o;
-    const float gOm = gW - go * L.Nn / (den_o * den_o);
-    float gv[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (int m = 0; m < 3; m++) {
-        const float gw = gN * (float)(m - 1) + gOm;
-        const float ggd = 2.0f * L.gd[m] * gw;
-        gv[m + 1] += ggd;
-        gv[m] -= ggd;
-    }
-    if (half) {  // only even lanes carry position-level adjoints
-        gpx = gpy = gnx = gny = gox = goy = 0.0f;
-        gv[0] = gv[1] = gv[2] = gv[3] = 0.0f;
-    }
-    if (lane == 0) {  // the line's centroid is origin + S_x / S_0: direct path to the origin
-        gox += (float)gm[e][0];
-        goy += (float)gm[e][1];
-    }
-    // hand the adjoints of taps 2, 3 to the odd lane
-    const float t2 = __shfl_xor_sync(0xffffffffu, gv[2], 1), t3 = __shfl_xor_sync(0xffffffffu, gv[3], 1);
-    const float gs0 = half ? t2 : gv[0], gs1 = half ? t3 : gv[1];
-    if (g_samples) {
-        float* s = g_samples + ((size_t)q * 4 + e) * (RF_POS * RF_TAPS) + j * RF_TAPS + 2 * half;
-        s[0] = gs0;
-        s[1] = gs1;
-    }
-    // samples -> sample positions -> p_j, n
-    const float gsv[2] = {gs0, gs1};
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-        const float u = RF_U[2 * half + i];
-        const float gx = gsv[i] * L.s[i].gx, gy = gsv[i] * L.s[i].gy;
-        gpx += gx;
-        gpy += gy;
-        gnx += u * gx;
-        gny += u * gy;
-        if (g_image) bilinear_scatter(g_image, iw, ih, L.sx[i], L.sy[i], gsv[i]);
-    }
-    // p = a + t (b - a); origin = (a + b) / 2; n = (-d_y, d_x), d = (b - a) / |b - a|
-    float gax = (1.0f - L.t) * gpx + 0.5f * gox, gay = (1.0f - L.t) * gpy + 0.5f * goy;
-    float gbx = L.t * gpx + 0.5f * gox, gby = L.t * gpy + 0.5f * goy;
-    const float gdx = gny, gdy = -gnx;
-    const float dd = L.dx * gdx + L.dy * gdy;
-    const float gDx = (gdx - L.dx * dd) / L.len, gDy = (gdy - L.dy * dd) / L.len;
-    gax -= gDx; gay -= gDy; gbx += gDx; gby += gDy;
-    float acc[4] = {gax, gay, gbx, gby};
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
-    if (lane == 0) {
-        atomicAdd(&gc[e][0], acc[0]);
-        atomicAdd(&gc[e][1], acc[1]);
-        atomicAdd(&gc[e1][0], acc[2]);
-        atomicAdd(&gc[e1][1], acc[3]);
-    }
-    __syncthreads();
-    if (threadIdx.x < 8) g_corners[(size_t)q * 8 + threadIdx.x] = (&gc[0][0])[threadIdx.x];
+    if (threadIdx.x < 2 * ne) g_corners[q0 * 8 + threadIdx.x] = (&gc[0][0])[threadIdx.x];
 }
 
 }  // namespace atag
@@ -418,8 +507,9 @@ extern "C" atag_status atag_refine_forward(const float* d_image, size_t width, s
     if (width < 2 || height < 2) return set_error(ATAG_ERR_INVALID_ARGUMENT, "refine_forward: image smaller than 2x2");
     if (n_quads == 0) return ATAG_OK;
     if (n_quads > (size_t)INT32_MAX) return set_error(ATAG_ERR_INVALID_ARGUMENT, "refine_forward: too many quads");
-    k_refine_forward<<<(unsigned)n_quads, 128, 0, (cudaStream_t)stream>>>(d_image, (int)width, (int)height, d_corners,
-                                                                          (int)n_quads, d_refined, d_residual, d_samples);
+    const unsigned qpc = refine_quads_per_cta(n_quads);
+    k_refine_forward<<<(unsigned)((n_quads + qpc - 1) / qpc), 32 * RF_WARPS, 0, (cudaStream_t)stream>>>(
+        d_image, (int)width, (int)height, d_corners, (int)n_quads, (int)qpc, d_refined, d_residual, d_samples);
     count_launch();
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? ATAG_OK : set_error(ATAG_ERR_CUDA, cudaGetErrorString(e));
@@ -436,10 +526,10 @@ extern "C" atag_status atag_refine_backward(const float* d_image, size_t width, 
     if (width < 2 || height < 2) return set_error(ATAG_ERR_INVALID_ARGUMENT, "refine_backward: image smaller than 2x2");
     if (n_quads == 0) return ATAG_OK;
     if (n_quads > (size_t)INT32_MAX) return set_error(ATAG_ERR_INVALID_ARGUMENT, "refine_backward: too many quads");
-    k_refine_backward<<<(unsigned)n_quads, 128, 0, (cudaStream_t)stream>>>(d_image, (int)width, (int)height,
-                                                                           d_corners, (int)n_quads, d_grad_refined,
-                                                                           d_grad_residual, d_grad_corners,
-                                                                           d_grad_samples, d_grad_image);
+    const unsigned qpc = refine_quads_per_cta(n_quads);
+    k_refine_backward<<<(unsigned)((n_quads + qpc - 1) / qpc), 32 * RF_WARPS, 0, (cudaStream_t)stream>>>(
+        d_image, (int)width, (int)height, d_corners, (int)n_quads, (int)qpc, d_grad_refined, d_grad_residual,
+        d_grad_corners, d_grad_samples, d_grad_image);
     count_launch();
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? ATAG_OK : set_error(ATAG_ERR_CUDA, cudaGetErrorString(e));
