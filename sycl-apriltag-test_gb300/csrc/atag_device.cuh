@@ -545,35 +545,13 @@ __device__ __forceinline__ void bitonic_sort_u64(unsigned long long* keys, uint3
     }
 }
 
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = w > v ? w : v;
-    }
-    return v;
-}
 __device__ __forceinline__ uint32_t warp_sum_u32(uint32_t v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
-// Block reductions through a caller-provided shared array of 32 slots.
-__device__ __forceinline__ unsigned long long block_max_u64(unsigned long long v, unsigned long long* red) {
-    v = warp_max_u64(v);
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    __syncthreads();
-    if (lane == 0) red[wid] = v;
-    __syncthreads();
-    if (wid == 0) {
-        unsigned long long x = lane < nw ? red[lane] : 0ull;
-        x = warp_max_u64(x);
-        if (lane == 0) red[0] = x;
-    }
-    __syncthreads();
-    return red[0];
-}
+// Block reduction through a caller-provided shared array of 32 slots.
 __device__ __forceinline__ uint32_t block_sum_u32(uint32_t v, uint32_t* red) {
     v = warp_sum_u32(v);
     int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
@@ -617,266 +595,6 @@ __device__ __forceinline__ uint32_t block_exclusive_scan_u32(uint32_t v, uint32_
     uint32_t r = red[wid] + x - v;
     *total = red[32];
     return r;
-}
-
-// Shared-memory key arrays of the cluster sorts keep one spare slot after
-// every 16 keys: a warp whose lanes touch 2 to 16 consecutive keys each
-// (sorted runs, per-lane segments) then hits distinct banks.
-__host__ __device__ constexpr uint32_t kpad(uint32_t i) { return i + (i >> 4); }
-__host__ __device__ constexpr uint32_t kpad_size(uint32_t n) { return n + n / 16; }
-
-// ---------------------------------------------------------------------------
-// Bitonic sort of T*K 64-bit keys held K per thread in registers.  On exit
-// thread t holds elements [t K, t K + K) of the ascending order.  Element e
-// lives in register e % K of thread e / K: compare distances below K are
-// register swaps, distances up to a warp are shuffles, longer ones go
-// through `xch` (T*K keys of shared memory, laid out r * T + t).
-// ---------------------------------------------------------------------------
-template <int K, int J>
-__device__ __forceinline__ void bitonic_regs_stage(unsigned long long (&v)[K], int base, int k) {
-#pragma unroll
-    for (int r = 0; r < K; r++) {
-        if ((r ^ J) > r) {
-            const int p = r ^ J;
-            const bool asc = ((base + r) & k) == 0;
-            const unsigned long long a = v[r], b = v[p];
-            const bool sw = (a > b) == asc;
-            v[r] = sw ? b : a;
-            v[p] = sw ? a : b;
-        }
-    }
-}
-
-template <int T, int K>
-__device__ __forceinline__ void bitonic_sort_regs(unsigned long long (&v)[K], unsigned long long* xch) {
-    const int tid = threadIdx.x, base = tid * K;
-    for (int k = 2; k <= T * K; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            if (j >= K) {
-                const int pj = j / K;
-                const bool keep_min = ((tid & pj) == 0) == ((tid & (k / K)) == 0);
-                if (pj < 32) {
-#pragma unroll
-                    for (int r = 0; r < K; r++) {
-                        const unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, v[r], pj);
-                        v[r] = keep_min ? (o < v[r] ? o : v[r]) : (o > v[r] ? o : v[r]);
-                    }
-                } else {
-                    __syncthreads();  // the previous exchange has been read
-#pragma unroll
-                    for (int r = 0; r < K; r++) xch[r * T + tid] = v[r];
-                    __syncthreads();
-#pragma unroll
-                    for (int r = 0; r < K; r++) {
-                        const unsigned long long o = xch[r * T + (tid ^ pj)];
-                        v[r] = keep_min ? (o < v[r] ? o : v[r]) : (o > v[r] ? o : v[r]);
-                    }
-                }
-            } else if (j == 1) {
-                bitonic_regs_stage<K, 1>(v, base, k);
-            } else if (j == 2) {
-                if constexpr (K > 2) bitonic_regs_stage<K, 2>(v, base, k);
-            } else if (j == 4) {
-                if constexpr (K > 4) bitonic_regs_stage<K, 4>(v, base, k);
-            } else if (j == 8) {
-                if constexpr (K > 8) bitonic_regs_stage<K, 8>(v, base, k);
-            } else if (j == 16) {
-                if constexpr (K > 16) bitonic_regs_stage<K, 16>(v, base, k);
-            }
-        }
-    }
-}
-
-// Sorts src[0, n) (global memory, n <= T*K) into dst[kpad(i)] (shared memory
-// of kpad_size(T*K) keys, also used for the exchange); all threads of the
-// CTA call it.
-template <int T, int K>
-__device__ __forceinline__ void sort_keys_regs(const unsigned long long* __restrict__ src, uint32_t n,
-                                               unsigned long long* dst) {
-    static_assert(K <= 32 && (K & (K - 1)) == 0, "K must be a power of two up to 32");
-    unsigned long long v[K];
-#pragma unroll
-    for (int r = 0; r < K; r++) {
-        const uint32_t e = (uint32_t)(r * T) + threadIdx.x;  // coalesced; the order is sorted away
-        v[r] = e < n ? src[e] : ~0ull;
-    }
-    bitonic_sort_regs<T, K>(v, dst);
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < K; r++) {
-        const uint32_t e = threadIdx.x * K + r;
-        if (e < n) dst[kpad(e)] = v[r];
-    }
-    __syncthreads();
-}
-
-// Block merge sort of src[0, n) (global memory, n <= T*K) into dst[kpad(i)]
-// (shared memory of kpad_size(T*K) keys).  Each thread sorts K keys in
-// registers, then log2(T) rounds merge pairs of sorted runs, doubling their
-// length: a thread finds where its K outputs start on the merge path of its
-// two runs (binary search along the diagonal, ties taken from the first
-// run) and merges K keys serially.  Its work is O(n log(n / K)) against the
-// O(n log^2 n) of a bitonic network, which pays from about 8 keys per thread.
-template <int T, int K>
-__device__ __forceinline__ void merge_sort_keys(const unsigned long long* __restrict__ src, uint32_t n,
-                                                unsigned long long* dst) {
-    static_assert(K >= 2 && K <= 32 && (K & (K - 1)) == 0, "K must be a power of two in [2, 32]");
-    unsigned long long v[K];
-#pragma unroll
-    for (int r = 0; r < K; r++) {
-        const uint32_t e = (uint32_t)(r * T) + threadIdx.x;  // coalesced; the order is sorted away
-        v[r] = e < n ? src[e] : ~0ull;
-    }
-#pragma unroll
-    for (int k = 2; k <= K; k <<= 1)
-#pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1)
-#pragma unroll
-            for (int r = 0; r < K; r++) {
-                const int p = r ^ j;
-                if (p > r) {
-                    const unsigned long long a = v[r], b = v[p];
-                    const bool sw = (a > b) == ((r & k) == 0);
-                    v[r] = sw ? b : a;
-                    v[p] = sw ? a : b;
-                }
-            }
-    const uint32_t tid = threadIdx.x;
-    // rounds whose pairs of runs belong to one warp only need that warp
-    // in step; wider rounds synchronise the CTA
-#pragma unroll 1
-    for (uint32_t width = 1; width < (uint32_t)T; width <<= 1) {
-#pragma unroll
-        for (int r = 0; r < K; r++) dst[kpad(tid * K + r)] = v[r];
-        if (2 * width <= 32) __syncwarp();
-        else __syncthreads();
-        const uint32_t g0 = tid & ~(2 * width - 1), L = width * K;
-        const uint32_t a0 = g0 * K, b0 = a0 + L, d = (tid - g0) * K;
-        uint32_t lo = d > L ? d - L : 0u, hi = d < L ? d : L;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (dst[kpad(a0 + mid)] <= dst[kpad(b0 + d - 1 - mid)]) lo = mid + 1;
-            else hi = mid;
-        }
-        uint32_t i = lo, j = d - lo;
-        unsigned long long a = i < L ? dst[kpad(a0 + i)] : 0ull;
-        unsigned long long b = j < L ? dst[kpad(b0 + j)] : 0ull;
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const bool ta = j >= L || (i < L && a <= b);
-            v[k] = ta ? a : b;
-            if (k + 1 < K) {
-                i += ta ? 1u : 0u;
-                j += ta ? 0u : 1u;
-                const uint32_t ni = ta ? i : j;
-                const unsigned long long nv = ni < L ? dst[kpad((ta ? a0 : b0) + ni)] : 0ull;
-                a = ta ? nv : a;
-                b = ta ? b : nv;
-            }
-        }
-        if (2 * width <= 32) __syncwarp();
-        else __syncthreads();
-    }
-#pragma unroll
-    for (int r = 0; r < K; r++) dst[kpad(tid * K + r)] = v[r];
-    __syncthreads();
-}
-
-// Lanes of the warp whose 8-bit digit equals this lane's, among the lanes
-// with `valid` set: eight ballots (match.any on 32 distinct values is much
-// slower on this GPU).
-__device__ __forceinline__ unsigned match_digit8(uint32_t d, bool valid) {
-    unsigned m = __ballot_sync(0xFFFFFFFFu, valid);
-#pragma unroll
-    for (int b = 0; b < 8; b++) {
-        const bool bit = (d >> b) & 1u;
-        const unsigned bb = __ballot_sync(0xFFFFFFFFu, bit);
-        m &= bit ? bb : ~bb;
-    }
-    return m;
-}
-
-// Stable LSD radix sort of n 64-bit keys for a CTA of THREADS threads, 8
-// bits per pass.  Each warp owns a contiguous range of the input so the
-// scatter keeps input order within a digit; passes where every key has the
-// same digit are skipped.  `hist` holds THREADS/32 x 256 counters, `red` 33
-// slots.  Returns the buffer that holds the sorted keys (a or b).  (Sorting
-// on the theta half alone and ordering ties afterwards does not pay: theta
-// carries a quadrant offset of 2^16, so it has 7 fractional bits there and
-// long runs of equal values.)
-template <uint32_t THREADS>
-__device__ __forceinline__ unsigned long long* block_radix_sort_u64(unsigned long long* a, unsigned long long* b,
-                                                                   uint32_t n, uint32_t* hist, uint32_t* red,
-                                                                   uint32_t* s_flag) {
-    constexpr uint32_t W = THREADS / 32;
-    constexpr uint32_t PER = W * 256 / THREADS;  // scan entries per thread
-    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t lo = (uint32_t)((unsigned long long)n * w / W), hi = (uint32_t)((unsigned long long)n * (w + 1) / W);
-    for (int pass = 0; pass < 8; pass++) {
-        const int sh = pass * 8;
-        __syncthreads();  // every thread is done with the previous pass's flag and counters
-        for (uint32_t i = threadIdx.x; i < W * 256; i += THREADS) hist[i] = 0;
-        if (threadIdx.x == 0) *s_flag = 0;
-        __syncthreads();
-        // warp-aggregated counts: lanes with equal digits add once (keys of
-        // one cluster share their high digits, which would serialise)
-        for (uint32_t base = lo; base < hi; base += 32) {
-            const uint32_t i = base + lane;
-            const bool v = i < hi;
-            const uint32_t d = v ? (uint32_t)((a[i] >> sh) & 255) : 0u;
-            const unsigned m = match_digit8(d, v);
-            if (v && (int)lane == __ffs(m) - 1) hist[w * 256 + d] += (uint32_t)__popc(m);
-            __syncwarp();
-        }
-        __syncthreads();
-        for (uint32_t d = threadIdx.x; d < 256; d += THREADS) {
-            uint32_t t = 0;
-#pragma unroll
-            for (uint32_t ww = 0; ww < W; ww++) t += hist[ww * 256 + d];
-            if (t == n) *s_flag = 1;  // all keys share this digit: the pass is the identity
-        }
-        __syncthreads();
-        if (*s_flag) continue;
-        // exclusive scan in (digit, warp) order; PER consecutive entries per thread
-        uint32_t vals[PER], sum = 0;
-        const uint32_t L0 = threadIdx.x * PER;
-#pragma unroll
-        for (uint32_t e = 0; e < PER; e++) {
-            const uint32_t L = L0 + e, d = L / W, ww = L % W;
-            vals[e] = hist[ww * 256 + d];
-            sum += vals[e];
-        }
-        uint32_t total;
-        uint32_t run = block_exclusive_scan_u32(sum, red, &total);
-        __syncthreads();
-#pragma unroll
-        for (uint32_t e = 0; e < PER; e++) {
-            const uint32_t L = L0 + e, d = L / W, ww = L % W;
-            hist[ww * 256 + d] = run;
-            run += vals[e];
-        }
-        __syncthreads();
-        for (uint32_t base = lo; base < hi; base += 32) {
-            const uint32_t i = base + lane;
-            const bool v = i < hi;
-            const unsigned long long key = v ? a[i] : 0ull;
-            const uint32_t d = (uint32_t)((key >> sh) & 255);
-            const unsigned m = match_digit8(d, v);
-            const uint32_t rank = __popc(m & ((1u << lane) - 1u));
-            const uint32_t p = v ? hist[w * 256 + d] : 0u;
-            __syncwarp();
-            if (v) {
-                b[p + rank] = key;
-                if ((int)lane == __ffs(m) - 1) hist[w * 256 + d] = p + __popc(m);
-            }
-            __syncwarp();
-        }
-        __syncthreads();
-        unsigned long long* t = a;
-        a = b;
-        b = t;
-    }
-    return a;
 }
 
 }  // namespace atag

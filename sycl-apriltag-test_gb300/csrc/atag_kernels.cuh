@@ -53,12 +53,14 @@ struct FrameDesc {
     uint32_t* quad_ok;                 // per rank q
     // cluster points
     uint32_t cpoint_cap;
-    unsigned long long* sortbuf;       // (theta key << 32) | packed
+    unsigned long long* sortbuf;       // (theta key << 32) | packed; then the sorted points' line-fit inputs;
+                                       // then the corner candidates
     atag_cluster_point* cluster_points;
     atag_line_fit_point* line_fit;
-    float* errbuf;                     // 2 floats per point (big clusters)
+    float* errbuf;                     // 2 floats per point (sort scratch of clusters past the shared memory)
     uint32_t* cluster_work;            // small clusters from the front, large from the back
     uint32_t* cluster_runs;            // first run (CE_RUN points) of each cluster
+    struct RunInfo* runs;              // per run
     // outputs
     atag_quad_corners* quads;
     uint32_t quad_cap;
@@ -121,25 +123,25 @@ enum Counter : uint32_t {
 constexpr uint32_t DEAD_PAIRS = 2;
 
 // Cluster-sort kernel shapes: most clusters are small and run several per SM
-// on 128 threads (up to 16 keys per thread), large ones get a 512-thread CTA
-// (up to 32 keys per thread); both sort in registers and shared memory (a
-// padded array of kpad_size(cap) keys).  Clusters larger than CF_LARGE_CAP
-// (4K frames only) radix-sort in global memory with per-warp counters.
-constexpr uint32_t CF_SMALL_THREADS = 128, CF_SMALL_CAP = CF_SMALL_THREADS * 16;
-constexpr uint32_t CF_LARGE_THREADS = 512, CF_LARGE_CAP = CF_LARGE_THREADS * 32;
-constexpr uint32_t CF_SMALL_SMEM = kpad_size(CF_SMALL_CAP) * 8;
-constexpr uint32_t CF_LARGE_SMEM = kpad_size(CF_LARGE_CAP) * 8 + (CF_LARGE_THREADS / 32) * 256 * 4;
-// Shared memory of the small-cluster kernel for clusters of at most `cap`
-// points: the sorts work on whole powers of two of at least 2 keys per
-// thread.
-__host__ __device__ constexpr uint32_t cf_small_smem(uint32_t cap) {
-    uint32_t k = CF_SMALL_THREADS * 2;
-    while (k < cap) k <<= 1;
-    return kpad_size(k) * 8;
-}
-// Window errors / filter / peaks: one warp per run of up to CE_RUN
-// consecutive points of one cluster.
+// on 256 threads, large ones get a 1024-thread CTA.  Keys sort in shared
+// memory: a large CTA's is sized for the largest cluster that passes the
+// filter (2 (2 w + 2 h) points, cluster_bounds.h:92-93), up to CF_LARGE_CAP
+// (every frame up to 3840 x 2160).
+constexpr uint32_t CF_SMALL_THREADS = 256, CF_SMALL_CAP = 2048, CF_SMALL_NB = 2048;
+constexpr uint32_t CF_LARGE_THREADS = 1024, CF_LARGE_CAP = 24576, CF_LARGE_NB = 4096;
+__host__ __device__ constexpr uint32_t cf_smem(uint32_t cap, uint32_t nb) { return cap * 8 + nb * 4; }
+constexpr uint32_t CF_LARGE_SMEM = cf_smem(CF_LARGE_CAP, CF_LARGE_NB);
+__host__ __device__ constexpr uint32_t max_cluster_points(uint32_t w, uint32_t h) { return 2 * (2 * w + 2 * h); }
+// A run: up to CE_RUN consecutive points of one cluster, the work item of a
+// warp in the prefix-sum and window-error kernels.
 constexpr uint32_t CE_RUN = 256;
+constexpr uint32_t CF_MAX_RUNS = max_cluster_points(4096, 4096) / CE_RUN;
+struct RunInfo {
+    long long before[6];  // moments (Mx, My, Mxx, Myy, Mxy, W) of the cluster's earlier runs
+    uint32_t cluster, first;  // its cluster and first point in it
+    uint32_t pad_[2];
+};
+__host__ __device__ constexpr size_t max_runs(size_t points, size_t clusters) { return points / CE_RUN + clusters; }
 
 // Batch-wide prefix offsets of up to four per-frame counters.
 struct BatchOffsets {
@@ -197,9 +199,10 @@ __global__ void k_boundaries_pairs_r16(const __grid_constant__ FrameSet fs, uint
 __global__ void k_pairs_finalize(const __grid_constant__ FrameSet fs, PipelineParams p, uint32_t small_max);
 __global__ void k_scatter_points(const __grid_constant__ FrameSet fs);
 __global__ void k_cluster_sort_small(const __grid_constant__ FrameSet fs, const uint32_t* work_offsets,
-                                     uint32_t n_frames, uint32_t* work_counter, uint32_t sort_cap);
+                                     uint32_t n_frames, uint32_t* work_counter, uint32_t cap);
 __global__ void k_cluster_sort_large(const __grid_constant__ FrameSet fs, const uint32_t* work_offsets,
-                                     uint32_t n_frames, uint32_t* work_counter);
+                                     uint32_t n_frames, uint32_t* work_counter, uint32_t cap);
+__global__ void k_cluster_lines(const __grid_constant__ FrameSet fs, const uint32_t* run_offsets, uint32_t n_frames);
 __global__ void k_cluster_errors(const __grid_constant__ FrameSet fs, const uint32_t* run_offsets,
                                  uint32_t n_frames, uint32_t* work_counter);
 __global__ void k_cluster_peaks(const __grid_constant__ FrameSet fs, const uint32_t* cluster_offsets,

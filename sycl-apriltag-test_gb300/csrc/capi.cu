@@ -69,7 +69,6 @@ atag_status ensure_device(DeviceInfo** out) {
         e = cudaFuncGetAttributes(&fa, k_threshold);
         if (e != cudaSuccess) return fail(ATAG_ERR_NO_DEVICE, "kernels do not load: %s", cudaGetErrorString(e));
         CK(cudaFuncSetAttribute(k_cluster_sort_large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF_LARGE_SMEM));
-        CK(cudaFuncSetAttribute(k_cluster_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF_SMALL_SMEM));
         CK(cudaFuncSetAttribute(k_peaks_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PK_SMEM));
         d.num_sms = prop.multiProcessorCount;
         d.smem_optin = prop.sharedMemPerBlockOptin;
@@ -200,6 +199,7 @@ size_t layout_frame(char* base, uint32_t w, uint32_t h, uint32_t factor, bool ow
     f.errbuf = (float*)take(8ull * c.cpoint_cap);
     f.cluster_work = (uint32_t*)take(4ull * c.cluster_cap);
     f.cluster_runs = (uint32_t*)take(4ull * c.cluster_cap);
+    f.runs = (RunInfo*)take(sizeof(RunInfo) * max_runs(c.cpoint_cap, c.cluster_cap));
     f.counters = (uint32_t*)take(4ull * CNT_COUNT);
     f.dead_pairs = (unsigned long long*)take(8ull * DEAD_PAIRS);
     // CCL edge records, sized for the largest of the tile-row choices
@@ -223,7 +223,7 @@ struct StageClusterLayout {
     size_t bytes;
     FrameDesc d;
     atag_frame_stats* stats;
-    uint32_t* work;  // small/large offsets (2 words each), then 2 queue cursors
+    uint32_t* work;  // small/large/run offsets (2 words each), then 3 queue cursors
 };
 StageClusterLayout layout_stage_cluster(char* base, uint32_t w, uint32_t h, uint32_t cluster_cap, uint32_t cpoint_cap) {
     StageClusterLayout L;
@@ -252,13 +252,14 @@ StageClusterLayout layout_stage_cluster(char* base, uint32_t w, uint32_t h, uint
     f.peak_count = (uint32_t*)take(4ull * cluster_cap);
     f.cluster_work = (uint32_t*)take(4ull * cluster_cap);
     f.cluster_runs = (uint32_t*)take(4ull * cluster_cap);
+    f.runs = (RunInfo*)take(sizeof(RunInfo) * max_runs(cpoint_cap, cluster_cap));
     f.cpoint_cap = cpoint_cap;
     f.sortbuf = (unsigned long long*)take(8ull * cpoint_cap);
     f.errbuf = (float*)take(8ull * cpoint_cap);
     f.counters = (uint32_t*)take(4ull * CNT_COUNT);
     f.stage_outputs = 1;
     L.stats = (atag_frame_stats*)take(sizeof(atag_frame_stats));
-    L.work = (uint32_t*)take(4ull * 6);
+    L.work = (uint32_t*)take(4ull * 9);
     L.d = f;
     L.bytes = off;
     return L;
@@ -591,7 +592,8 @@ atag_status atag_cluster(const atag_boundary_point* points, const uint64_t* keys
     const int sms = dev->num_sms;
     uint32_t* off_small = L.work;
     uint32_t* off_large = L.work + 2;
-    uint32_t* wc = L.work + 4;
+    uint32_t* off_runs = L.work + 4;
+    uint32_t* wc = L.work + 6;
     atag_config c;
     atag_config_default(&c);
     const PipelineParams p = make_params(c);
@@ -603,16 +605,21 @@ atag_status atag_cluster(const atag_boundary_point* points, const uint64_t* keys
     k_pairs_finalize<<<1, 1024, 0, s>>>(fs, p, CF_SMALL_CAP);
     LAUNCHED();
     {
-        BatchOffsets bo{{CNT_SMALL, CNT_LARGE, 0, 0}, {off_small, off_large, nullptr, nullptr}, wc};
+        BatchOffsets bo{{CNT_SMALL, CNT_LARGE, CNT_RUNS, 0}, {off_small, off_large, off_runs, nullptr}, wc};
         k_batch_offsets<<<1, 1024, 0, s>>>(fs, 1, bo);
     }
     LAUNCHED();
     k_planes_scatter<<<(unsigned)std::min<size_t>(cdiv(n, 256), (size_t)sms * 8), 256, 0, s>>>(
         fs, reinterpret_cast<const uint32_t*>(points), reinterpret_cast<const unsigned long long*>(keys), n);
     LAUNCHED();
-    k_cluster_sort_large<<<std::max(1, sms / 2), CF_LARGE_THREADS, CF_LARGE_SMEM, s>>>(fs, off_large, 1, wc + 1);
+    const uint32_t cap = std::min(max_cluster_points(d.width, d.height), CF_LARGE_CAP);
+    k_cluster_sort_large<<<std::max(1, sms / 2), CF_LARGE_THREADS, cf_smem(cap, CF_LARGE_NB), s>>>(fs, off_large, 1,
+                                                                                                  wc + 1, cap);
     LAUNCHED();
-    k_cluster_sort_small<<<sms * 8, CF_SMALL_THREADS, CF_SMALL_SMEM, s>>>(fs, off_small, 1, wc, CF_SMALL_CAP);
+    k_cluster_sort_small<<<sms * 8, CF_SMALL_THREADS, cf_smem(CF_SMALL_CAP, CF_SMALL_NB), s>>>(fs, off_small, 1, wc,
+                                                                                              CF_SMALL_CAP);
+    LAUNCHED();
+    k_cluster_lines<<<sms * 8, 128, 0, s>>>(fs, off_runs, 1);
     LAUNCHED();
     k_stage_cluster_out<<<sms * 4, 256, 0, s>>>(fs, o->cluster_indices, (unsigned long long*)o->filtered_keys);
     LAUNCHED();
@@ -884,13 +891,14 @@ static atag_status upload_table(atag_detector* det, const std::vector<FrameDesc>
 static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, const std::vector<FrameDesc>& t,
                                size_t first, size_t last, cudaStream_t s, int lane, bool timed) {
     const size_t n = last - first;
-    size_t mw = 0, mh = 0, max_pair = 0, max_points = 0;
+    size_t mw = 0, mh = 0, max_pair = 0, max_points = 0, max_cluster = 0;
     bool any_decim = false;
     for (size_t i = first; i < last; i++) {
         mw = std::max<size_t>(mw, t[i].width);
         mh = std::max<size_t>(mh, t[i].height);
         max_pair = std::max<size_t>(max_pair, t[i].pair_cap);
         max_points = std::max<size_t>(max_points, t[i].point_cap);
+        max_cluster = std::max<size_t>(max_cluster, max_cluster_points(t[i].width, t[i].height));
         any_decim |= t[i].factor > 1 || t[i].src_format != ATAG_PIX_GREY8;
     }
     FrameSet fs;
@@ -968,19 +976,19 @@ static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, con
     // large clusters on the side stream, concurrently with the small ones
     CK(cudaEventRecord(det->fork[lane], s));
     CK(cudaStreamWaitEvent(side, det->fork[lane], 0));
-    k_cluster_sort_large<<<std::max(1, sms / std::max(1, tu.large_ctas_divisor)), CF_LARGE_THREADS, CF_LARGE_SMEM,
-                           side>>>(fs, off_large, (uint32_t)n, wc + 1);
+    const uint32_t large_cap = (uint32_t)std::min<size_t>(max_cluster, CF_LARGE_CAP);
+    k_cluster_sort_large<<<std::max(1, sms / std::max(1, tu.large_ctas_divisor)), CF_LARGE_THREADS,
+                           cf_smem(large_cap, CF_LARGE_NB), side>>>(fs, off_large, (uint32_t)n, wc + 1, large_cap);
     LAUNCHED();
-    {
-        // the small-cluster kernel's key buffers are sized for the tuned split
-        const uint32_t cap = (uint32_t)tu.small_cluster_max;
-        const uint32_t smem = cf_small_smem(cap);
-        k_cluster_sort_small<<<sms * std::max(1, tu.small_ctas_per_sm), CF_SMALL_THREADS, smem, s>>>(
-            fs, off_small, (uint32_t)n, wc, cap);
-    }
+    // the small-cluster kernel's key buffer is sized for the tuned split
+    k_cluster_sort_small<<<sms * std::max(1, tu.small_ctas_per_sm), CF_SMALL_THREADS,
+                           cf_smem((uint32_t)tu.small_cluster_max, CF_SMALL_NB), s>>>(
+        fs, off_small, (uint32_t)n, wc, (uint32_t)tu.small_cluster_max);
     LAUNCHED();
     CK(cudaEventRecord(det->join[lane], side));
     CK(cudaStreamWaitEvent(s, det->join[lane], 0));
+    k_cluster_lines<<<sms * 8, 128, 0, s>>>(fs, off_runs, (uint32_t)n);
+    LAUNCHED();
     STAGE(10);
     k_cluster_errors<<<sms * 8, 256, 0, s>>>(fs, off_runs, (uint32_t)n, wc + 2);
     LAUNCHED();

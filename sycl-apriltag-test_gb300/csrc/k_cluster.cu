@@ -19,7 +19,8 @@
 //   3. k_scatter_points: points of surviving pairs go straight into their
 //      cluster's segment with their theta key; the rest are dropped;
 //   4. k_cluster_sort: one CTA per cluster sorts by (theta, point) in
-//      shared memory and writes ClusterPoints and the line-fit prefix sums;
+//      shared memory and writes ClusterPoints and the line-fit inputs;
+//      k_cluster_lines: line-fit prefix sums, a warp per run of points;
 //      k_cluster_errors: fit_lines (windowed errors, 7-tap filter, peaks)
 //      flat over all cluster points; k_cluster_peaks: the 10 best peaks of
 //      each cluster;
@@ -645,8 +646,8 @@ __global__ void __launch_bounds__(256) k_scatter_points(const __grid_constant__ 
 }
 
 // ---------------------------------------------------------------------------
-// 4. one cluster per CTA: sort by (theta, point), ClusterPoints, line-fit
-// inputs and their prefix sums
+// 4. one cluster per CTA: sort by (theta, point), ClusterPoints and line-fit
+// inputs; then one warp per run of points: the prefix sums
 // ---------------------------------------------------------------------------
 
 __device__ __forceinline__ uint32_t find_frame(const uint32_t* offsets, uint32_t n_frames, uint32_t item) {
@@ -658,200 +659,322 @@ __device__ __forceinline__ uint32_t find_frame(const uint32_t* offsets, uint32_t
     return lo;
 }
 
-// Inclusive scan of 6 int64 moment lanes within groups of WIDTH lanes
-// (32: the whole warp).  W, Mx and My are scanned in 32 bits: over at most
-// 128 points their sums stay below 2^31 (W <= 361, rx, ry < 2^15), so the
-// result equals the int64 (wrapping) sums.  Callers keep every partial sum
-// within 128 points.
-template <int WIDTH>
-__device__ __forceinline__ Moment scan_moment(const Moment& v) {
-    const int pos = (threadIdx.x & 31) & (WIDTH - 1);
-    uint32_t mx = (uint32_t)v.Mx, my = (uint32_t)v.My, mw = (uint32_t)v.W;
-    long long xx = v.Mxx, yy = v.Myy, xy = v.Mxy;
-#pragma unroll
-    for (int o = 1; o < WIDTH; o <<= 1) {
-        const uint32_t a = __shfl_up_sync(0xffffffffu, mx, o, WIDTH);
-        const uint32_t b = __shfl_up_sync(0xffffffffu, my, o, WIDTH);
-        const uint32_t c = __shfl_up_sync(0xffffffffu, mw, o, WIDTH);
-        const long long d = (long long)__shfl_up_sync(0xffffffffu, (unsigned long long)xx, o, WIDTH);
-        const long long e = (long long)__shfl_up_sync(0xffffffffu, (unsigned long long)yy, o, WIDTH);
-        const long long f = (long long)__shfl_up_sync(0xffffffffu, (unsigned long long)xy, o, WIDTH);
-        if (pos >= o) {
-            mx += a; my += b; mw += c;
-            xx = wadd(xx, d); yy = wadd(yy, e); xy = wadd(xy, f);
-        }
+// Bucket of a sort key's theta half among nb = 4 nq buckets: a monotone
+// function of the key, about uniform over a compact cluster.  calc_theta
+// (boundary_point.h:48-61) is a quadrant's offset plus a ratio r >= 0 of
+// tangent type, which may run into the next quadrant's values, so the four
+// parts are cut by value.  Up to r = 64 a part's first 7/8 of buckets are linear
+// in r / (1 + r) (the angle, nearly); beyond, points close to an axis of the
+// cluster (long thin shapes) take the last 1/8 by the logarithm of r.  Every
+// operation rounds to nearest, so each step and the whole are monotone.
+struct Buckets {
+    uint32_t nq, lin, sh;  // buckets per part, linear ones, log step
+    float scale;
+    __device__ __forceinline__ explicit Buckets(uint32_t nb) {
+        nq = nb >> 2;
+        lin = nq - (nq >> 3);
+        sh = 24u + 6u - (31u - (uint32_t)__clz((int)nq));  // 14 octaves of r fit nq / 8 buckets
+        scale = __fmul_rn((float)lin, 65.0f / 64.0f);
     }
-    return Moment{(long long)mx, (long long)my, xx, yy, xy, (long long)mw};
-}
-__device__ __forceinline__ Moment warp_sum_moment(Moment v) {
-    long long x[6] = {v.Mx, v.My, v.Mxx, v.Myy, v.Mxy, v.W};
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int j = 0; j < 6; j++)
-            x[j] = wadd(x[j], (long long)__shfl_xor_sync(0xffffffffu, (unsigned long long)x[j], o));
-    return Moment{x[0], x[1], x[2], x[3], x[4], x[5]};
-}
-__device__ __forceinline__ Moment shfl_moment(const Moment& v, int src) {
-    auto s = [&](long long x) { return (long long)__shfl_sync(0xffffffffu, (unsigned long long)x, src); };
-    return Moment{s(v.Mx), s(v.My), s(v.Mxx), s(v.Myy), s(v.Mxy), s(v.W)};
-}
+    __device__ __forceinline__ uint32_t operator()(uint32_t theta_key) const {
+        const float th = float_from_order_key(theta_key);
+        const uint32_t part = th < 0.0f ? 0u : th < 65536.0f ? 1u : th < 131072.0f ? 2u : 3u;
+        const float r = __fsub_rn(th, ((float)part - 1.0f) * 65536.0f);
+        uint32_t b;
+        if (r < 64.0f) {
+            const float g = __fsub_rn(1.0f, __frcp_rn(__fadd_rn(1.0f, r)));
+            b = min((uint32_t)max(__float2int_rz(__fmul_rn(g, scale)), 0), lin - 1u);
+        } else {
+            b = lin + min((__float_as_uint(r) - __float_as_uint(64.0f)) >> sh, nq - lin - 1u);
+        }
+        return part * nq + b;
+    }
+};
 
-template <bool LARGE>
+// Sort of one cluster per CTA by (theta, packed point), the reference's
+// (cluster, slope) order (main.cpp:737-750) with ties fixed by the point, as
+// a bucket sort: count the buckets, prefix the counts, place the keys bucket
+// by bucket, then rank each key among its bucket's few keys (rounding of
+// theta leaves up to ~25 equal ones in the largest clusters): O(n), against
+// the log2(threads) merge rounds, and radix passes in global memory above
+// 16,384 keys, that it replaced.  Bound by instruction issue and the latency
+// of one CTA; sort and prefix sums of a lone 1080p frame 82 -> 42 us, of a 4K
+// stress frame 343 -> 100 us, of 64 1080p frames 750 -> 492 us (stage alone).
+// Keys are placed in shared memory, or for clusters over `cap` keys (frames
+// larger than 4K) in their segment of errbuf.  Results: ClusterPoints and, in
+// the segment of sortbuf, each point's line-fit inputs in sorted order; and
+// per run of CE_RUN points the moments of all earlier points, from which
+// k_cluster_lines computes the prefix sums with any number of warps.
+template <uint32_t THREADS, int KEEP, uint32_t MAX_NB, uint32_t MAX_RUNS>
 __device__ __forceinline__ void cluster_sort(const FrameSet& fs, const uint32_t* __restrict__ work_offsets,
-                                             uint32_t n_frames, uint32_t* __restrict__ work_counter,
-                                             uint32_t sort_cap) {
-    constexpr uint32_t THREADS = LARGE ? CF_LARGE_THREADS : CF_SMALL_THREADS;
-    extern __shared__ unsigned long long smem_keys[];
-    __shared__ long long red_m[32][6];
-    __shared__ longlong2 lf_row[THREADS / 32][32][3];  // per warp: one row of LineFitPoints
-    __shared__ uint32_t red32[33];
-    __shared__ uint32_t s_item, s_flag;
-    // radix counters of the global-memory sorts, after the padded key array
-    uint32_t* hist = reinterpret_cast<uint32_t*>(smem_keys + kpad_size(sort_cap));
+                                             uint32_t n_frames, uint32_t* __restrict__ work_counter, uint32_t cap) {
+    constexpr uint32_t W = THREADS / 32;
+    extern __shared__ unsigned long long smem_keys[];  // cap keys, then MAX_NB counters
+    uint32_t* hist = reinterpret_cast<uint32_t*>(smem_keys + cap);
+    __shared__ long long red_m[6][MAX_RUNS];
+    __shared__ uint32_t red32[W];
+    __shared__ uint32_t s_item;
+    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t total = work_offsets[n_frames];
-    for (;;) {
-        __syncthreads();
-        if (threadIdx.x == 0) s_item = atomicAdd(work_counter, 1u);
-        __syncthreads();
-        const uint32_t item = s_item;
-        if (item >= total) return;
+    // a CTA's first cluster is its own index, later ones come from the queue
+    for (uint32_t item = blockIdx.x; item < total;) {
         const uint32_t fidx = find_frame(work_offsets, n_frames, item);
         const FrameDesc& F = fs.get(fidx);
         const uint32_t j = item - work_offsets[fidx];
-        const uint32_t cid = F.cluster_work[LARGE ? F.cluster_cap - 1 - j : j];
+        const uint32_t cid = F.cluster_work[THREADS == CF_LARGE_THREADS ? F.cluster_cap - 1 - j : j];
         const atag_cluster_extents ext = F.cluster_extents[cid];
         const uint32_t n = ext.count, start = ext.start;
-        // sort by (theta, packed point): the reference's (cluster, slope)
-        // order (main.cpp:737-750) with ties fixed by the point.  Up to
-        // sort_cap keys sort in shared memory (padded layout, key i at
-        // kpad(i)): a register bitonic network for up to 4 keys per thread,
-        // a merge sort above; larger clusters (4K frames only) radix-sort
-        // in global memory (plain layout).
-        unsigned long long* X = smem_keys;
-        const unsigned long long* src = F.sortbuf + start;
-        uint32_t pad_mask = ~0u;
-        if (n <= sort_cap) {
-            if (LARGE) {
-                if (n <= THREADS * 8) merge_sort_keys<THREADS, 8>(src, n, X);
-                else if (n <= THREADS * 16) merge_sort_keys<THREADS, 16>(src, n, X);
-                else merge_sort_keys<THREADS, 32>(src, n, X);
-            } else {
-                if (n <= THREADS * 2) sort_keys_regs<THREADS, 2>(src, n, X);
-                else if (n <= THREADS * 4) sort_keys_regs<THREADS, 4>(src, n, X);
-                else if (n <= THREADS * 8) merge_sort_keys<THREADS, 8>(src, n, X);
-                else merge_sort_keys<THREADS, 16>(src, n, X);
-            }
-        } else {
-            X = block_radix_sort_u64<THREADS>(F.sortbuf + start,
-                                              reinterpret_cast<unsigned long long*>(F.errbuf + 2ull * start), n,
-                                              hist, red32, &s_flag);
-            pad_mask = 0u;
+        unsigned long long* src = F.sortbuf + start;
+        unsigned long long* X = n <= cap ? smem_keys : reinterpret_cast<unsigned long long*>(F.errbuf) + start;
+        // about one bucket per key
+        const uint32_t nb = min(max(256u, 1u << (32 - __clz((int)(n - 1u)))), MAX_NB);
+        const Buckets bucket(nb);
+        for (uint32_t i = threadIdx.x; i < nb; i += THREADS) hist[i] = 0u;
+        if (threadIdx.x == 0) s_item = gridDim.x + atomicAdd(work_counter, 1u);
+        __syncthreads();
+        // KEEP keys per thread stay in registers with their buckets (all of a
+        // small cluster's); the rest are read and bucketed twice
+        unsigned long long key[KEEP];
+        uint32_t bkt[KEEP];
+#pragma unroll
+        for (int u = 0; u < KEEP; u++) {
+            const uint32_t i = threadIdx.x + u * THREADS;
+            key[u] = i < n ? __ldcg(src + i) : 0ull;
+        }
+#pragma unroll
+        for (int u = 0; u < KEEP; u++) {
+            const uint32_t i = threadIdx.x + u * THREADS;
+            bkt[u] = bucket((uint32_t)(key[u] >> 32));
+            if (i < n) atomicAdd(&hist[bkt[u]], 1u);
+        }
+        for (uint32_t i = threadIdx.x + KEEP * THREADS; i < n; i += THREADS)
+            atomicAdd(&hist[bucket((uint32_t)(__ldcg(src + i) >> 32))], 1u);
+        __syncthreads();
+        // exclusive prefix: each warp takes a contiguous part, in rows of 32
+        {
+            const uint32_t per = max(nb / W, 32u), h0 = w * per, h1 = min(nb, h0 + per);
+            uint32_t sum = 0;
+            for (uint32_t h = h0 + lane; h < h1; h += 32) sum += hist[h];
+            sum = __reduce_add_sync(0xFFFFFFFFu, sum);
+            if (lane == 0) red32[w] = sum;
             __syncthreads();
-        }
-        auto at = [&](uint32_t i) -> unsigned long long& { return X[i + ((i >> 4) & pad_mask)]; };
-        // The rest runs per warp over contiguous ranges of 128-point chunks
-        // (32 lanes x SEG consecutive points).
-        constexpr uint32_t W = THREADS / 32, SEG = 4, CH = 32 * SEG;
-        const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const uint32_t nch = (n + CH - 1) / CH, ch0 = nch * w / W, ch1 = nch * (w + 1) / W;
-        const uint32_t r0 = ch0 * CH, r1 = min(n, ch1 * CH);
-        // ClusterPoints out; the key slot is reused for the line-fit inputs
-        // (four rows in flight, so their image reads overlap), and the
-        // warp's moment total for the scan below
-        Moment t{0, 0, 0, 0, 0, 0};
-        for (uint32_t i0 = r0 + lane; i0 < r1; i0 += 4 * 32) {
-            unsigned long long k[4];
+            uint32_t carry = __reduce_add_sync(0xFFFFFFFFu, lane < w ? red32[lane] : 0u);
+            for (uint32_t h = h0 + lane; h < h1; h += 32) {
+                const uint32_t v = hist[h];
+                uint32_t x = v;
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const uint32_t i = i0 + u * 32;
-                k[u] = i < r1 ? at(i) : 0ull;
-            }
-            unsigned long long v[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) v[u] = linefit_rxyw((uint32_t)k[u], F.width, F.height, F.grey);
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const uint32_t i = i0 + u * 32;
-                if (i < r1) {
-                    const uint32_t packed = (uint32_t)k[u];
-                    atag_cluster_point cp;
-                    cp.packed_x = (uint16_t)packed;
-                    cp.packed_y = (uint16_t)(packed >> 16);
-                    cp.slope = float_from_order_key((uint32_t)(k[u] >> 32));
-                    F.cluster_points[start + i] = cp;
-                    at(i) = v[u];
-                    t = m_add(t, moment_of(v[u]));
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                    if ((int)lane >= o) x += y;
                 }
-            }
-        }
-        // segmented inclusive scan of the moments (main.cpp:796-801).  The
-        // carry into a warp's range is the sum of the earlier warps' totals;
-        // per chunk, lane l first sums its SEG points (4l .. 4l + 3), one
-        // warp scan of those 32 sums gives each segment's offset, then rows
-        // of 32 consecutive points add a scan within their segment to its
-        // offset, so consecutive lanes store consecutive LineFitPoints.
-        t = warp_sum_moment(t);
-        if (lane == 0) {
-            red_m[w][0] = t.Mx; red_m[w][1] = t.My; red_m[w][2] = t.Mxx;
-            red_m[w][3] = t.Myy; red_m[w][4] = t.Mxy; red_m[w][5] = t.W;
-        }
-        __syncthreads();
-        Moment carry{0, 0, 0, 0, 0, 0};
-        for (uint32_t k = 0; k < w; k++)
-            carry = m_add(carry, Moment{red_m[k][0], red_m[k][1], red_m[k][2], red_m[k][3], red_m[k][4],
-                                        red_m[k][5]});
-        for (uint32_t c = ch0; c < ch1; c++) {
-            const uint32_t c0 = c * CH;
-            Moment seg{0, 0, 0, 0, 0, 0};
-#pragma unroll
-            for (uint32_t q = 0; q < SEG; q++) {
-                const uint32_t i = c0 + lane * SEG + q;
-                if (i < n) seg = m_add(seg, moment_of(at(i)));
-            }
-            const Moment incl = scan_moment<32>(seg);
-            const Moment off = m_add(carry, m_sub(incl, seg));
-            carry = m_add(carry, shfl_moment(incl, 31));
-#pragma unroll
-            for (uint32_t r = 0; r < SEG; r++) {
-                const uint32_t i = c0 + r * 32 + lane;
-                const Moment m = i < n ? moment_of(at(i)) : Moment{0, 0, 0, 0, 0, 0};
-                const Moment in_seg = scan_moment<SEG>(m);
-                const Moment base = shfl_moment(off, (int)(r * (32 / SEG) + lane / SEG));
-                // the row's 32 LineFitPoints go out as 512-byte runs: each
-                // lane parks its 48 bytes in shared memory, then stores 16
-                // consecutive bytes of the row per instruction
-                const Moment lf = m_add(base, in_seg);
-                lf_row[w][lane][0] = make_longlong2(lf.Mx, lf.My);
-                lf_row[w][lane][1] = make_longlong2(lf.Mxx, lf.Myy);
-                lf_row[w][lane][2] = make_longlong2(lf.Mxy, lf.W);
-                __syncwarp();
-                const uint32_t r0 = c0 + r * 32;
-                longlong2* out = reinterpret_cast<longlong2*>(F.line_fit + start + r0);
-#pragma unroll
-                for (uint32_t q = 0; q < 4; q++) {
-                    const uint32_t piece = q * 32 + lane, pt = piece >> 2, f = piece & 3;
-                    if (r0 + pt < n) out[piece] = f < 3 ? lf_row[w][pt][f] : make_longlong2(0, 0);
-                }
-                __syncwarp();
+                hist[h] = carry + x - v;
+                carry += __shfl_sync(0xFFFFFFFFu, x, 31);
             }
         }
         __syncthreads();
+#pragma unroll
+        for (int u = 0; u < KEEP; u++)
+            if (threadIdx.x + u * THREADS < n) X[atomicAdd(&hist[bkt[u]], 1u)] = key[u];
+        for (uint32_t i = threadIdx.x + KEEP * THREADS; i < n; i += THREADS) {
+            const unsigned long long k = __ldcg(src + i);
+            X[atomicAdd(&hist[bucket((uint32_t)(k >> 32))], 1u)] = k;
+        }
+        __syncthreads();
+        // hist[b] is now the end of bucket b.  Two keys per thread and step,
+        // so their image reads overlap.
+        for (uint32_t i0 = threadIdx.x; i0 < n; i0 += 2 * THREADS) {
+            unsigned long long k[2];
+            uint32_t rank[2];
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const uint32_t i = i0 + u * THREADS;
+                k[u] = 0ull;
+                rank[u] = INVALID;
+                if (i >= n) continue;
+                k[u] = X[i];
+                const uint32_t b = bucket((uint32_t)(k[u] >> 32)), lo = b ? hist[b - 1] : 0u, hi = hist[b];
+                uint32_t r = lo;
+                for (uint32_t q = lo; q < i; q++) r += X[q] <= k[u] ? 1u : 0u;
+                for (uint32_t q = i + 1; q < hi; q++) r += X[q] < k[u] ? 1u : 0u;
+                rank[u] = r;
+            }
+            unsigned long long v[2];
+#pragma unroll
+            for (int u = 0; u < 2; u++) v[u] = linefit_rxyw((uint32_t)k[u], F.width, F.height, F.grey);
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                if (rank[u] == INVALID) continue;
+                const uint32_t packed = (uint32_t)k[u];
+                atag_cluster_point cp;
+                cp.packed_x = (uint16_t)packed;
+                cp.packed_y = (uint16_t)(packed >> 16);
+                cp.slope = float_from_order_key((uint32_t)(k[u] >> 32));
+                F.cluster_points[start + rank[u]] = cp;
+                __stcg(src + rank[u], v[u]);
+            }
+        }
+        __syncthreads();
+        // moments of each run of CE_RUN points: W, Mx and My fit 32 bits (W <=
+        // 362, rx, ry <= 8193)
+        const uint32_t nruns = (n + CE_RUN - 1) / CE_RUN;
+        for (uint32_t r = w; r < nruns; r += W) {
+            uint32_t mx = 0, my = 0, mw = 0;
+            long long xx = 0, yy = 0, xy = 0;
+            const uint32_t i1 = min(n, (r + 1) * CE_RUN);
+            for (uint32_t i = r * CE_RUN + lane; i < i1; i += 32) {
+                const Moment m = moment_of(__ldcg(src + i));
+                mx += (uint32_t)m.Mx;
+                my += (uint32_t)m.My;
+                mw += (uint32_t)m.W;
+                xx = wadd(xx, m.Mxx);
+                yy = wadd(yy, m.Myy);
+                xy = wadd(xy, m.Mxy);
+            }
+            mx = __reduce_add_sync(0xFFFFFFFFu, mx);
+            my = __reduce_add_sync(0xFFFFFFFFu, my);
+            mw = __reduce_add_sync(0xFFFFFFFFu, mw);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                xx = wadd(xx, __shfl_xor_sync(0xFFFFFFFFu, xx, o));
+                yy = wadd(yy, __shfl_xor_sync(0xFFFFFFFFu, yy, o));
+                xy = wadd(xy, __shfl_xor_sync(0xFFFFFFFFu, xy, o));
+            }
+            if (lane == 0) {
+                red_m[0][r] = mx; red_m[1][r] = my; red_m[2][r] = xx;
+                red_m[3][r] = yy; red_m[4][r] = xy; red_m[5][r] = mw;
+            }
+        }
+        __syncthreads();
+        // their exclusive prefixes, component c on warp c mod W
+        for (uint32_t c = w; c < 6; c += W) {
+            long long carry = 0;
+            for (uint32_t r0 = 0; r0 < nruns; r0 += 32) {
+                const uint32_t r = r0 + lane;
+                const long long v = r < nruns ? red_m[c][r] : 0ll;
+                long long x = v;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const long long y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                    if ((int)lane >= o) x = wadd(x, y);
+                }
+                if (r < nruns) F.runs[F.cluster_runs[cid] + r].before[c] = wadd(carry, wsub(x, v));
+                carry = wadd(carry, __shfl_sync(0xFFFFFFFFu, x, 31));
+            }
+        }
+        for (uint32_t r = threadIdx.x; r < nruns; r += THREADS) {
+            RunInfo& R = F.runs[F.cluster_runs[cid] + r];
+            R.cluster = cid;
+            R.first = r * CE_RUN;
+        }
+        item = s_item;
+        __syncthreads();  // the shared memory is free for the next cluster
     }
 }
 
-__global__ void __launch_bounds__(CF_SMALL_THREADS, 6) k_cluster_sort_small(const __grid_constant__ FrameSet fs,
+__global__ void __launch_bounds__(CF_SMALL_THREADS, 4) k_cluster_sort_small(const __grid_constant__ FrameSet fs,
                                                                         const uint32_t* __restrict__ work_offsets,
                                                                         uint32_t n_frames,
                                                                         uint32_t* __restrict__ work_counter,
-                                                                        uint32_t sort_cap) {
-    cluster_sort<false>(fs, work_offsets, n_frames, work_counter, sort_cap);
+                                                                        uint32_t cap) {
+    cluster_sort<CF_SMALL_THREADS, CF_SMALL_CAP / CF_SMALL_THREADS, CF_SMALL_NB, CF_SMALL_CAP / CE_RUN>(fs, work_offsets, n_frames, work_counter, cap);
 }
 __global__ void __launch_bounds__(CF_LARGE_THREADS, 1) k_cluster_sort_large(const __grid_constant__ FrameSet fs,
                                                                            const uint32_t* __restrict__ work_offsets,
                                                                            uint32_t n_frames,
-                                                                           uint32_t* __restrict__ work_counter) {
-    cluster_sort<true>(fs, work_offsets, n_frames, work_counter, CF_LARGE_CAP);
+                                                                           uint32_t* __restrict__ work_counter,
+                                                                           uint32_t cap) {
+    cluster_sort<CF_LARGE_THREADS, 4, CF_LARGE_NB, CF_MAX_RUNS>(fs, work_offsets, n_frames, work_counter, cap);
+}
+
+// The segmented inclusive scan of the moments (main.cpp:796-801): one warp per
+// run of CE_RUN points, from the moments of the cluster's earlier runs.  Lane
+// l of a chunk of 128 points has points 4 l .. 4 l + 3: one warp scan of the
+// lanes' sums (W, Mx and My in 32 bits: exact over 128 points), then each
+// lane adds its points one by one and stores their LineFitPoints, a 32-byte
+// sector per store where the array's alignment allows it (the detector's own
+// always does; a caller's array may not).
+__device__ __forceinline__ void store_sector(void* p, long long a, long long b, long long c, long long d) {
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
+}
+
+__global__ void __launch_bounds__(128, 4) k_cluster_lines(const __grid_constant__ FrameSet fs,
+                                                       const uint32_t* __restrict__ run_offsets, uint32_t n_frames) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t total = run_offsets[n_frames], stride = gridDim.x * (blockDim.x >> 5);
+    // items go round the CTAs first, so that a few still use every SM
+    for (uint32_t item = blockIdx.x + gridDim.x * (threadIdx.x >> 5); item < total; item += stride) {
+        const uint32_t fidx = find_frame(run_offsets, n_frames, item);
+        const FrameDesc& F = fs.get(fidx);
+        const RunInfo R = F.runs[item - run_offsets[fidx]];
+        const atag_cluster_extents ext = F.cluster_extents[R.cluster];
+        const unsigned long long* in = F.sortbuf + ext.start;
+        const bool wide = (reinterpret_cast<uintptr_t>(F.line_fit) & 31u) == 0;
+        Moment carry{R.before[0], R.before[1], R.before[2], R.before[3], R.before[4], R.before[5]};
+        const uint32_t end = min(ext.count, R.first + CE_RUN);
+#pragma unroll 1
+        for (uint32_t c0 = R.first; c0 < end; c0 += 128) {
+            const uint32_t i0 = c0 + 4 * lane;
+            uint32_t wt[4], rx[4], ry[4];
+            uint32_t mx = 0, my = 0, mw = 0;
+            unsigned long long xx = 0, yy = 0, xy = 0;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const unsigned long long v = i0 + q < end ? __ldcg(in + i0 + q) : 0ull;
+                rx[q] = (uint32_t)v & 0xFFFFu;
+                ry[q] = (uint32_t)v >> 16;
+                wt[q] = (uint32_t)(v >> 32);
+                const uint32_t ax = wt[q] * rx[q], ay = wt[q] * ry[q];
+                mw += wt[q];
+                mx += ax;
+                my += ay;
+                xx += (unsigned long long)ax * rx[q];
+                yy += (unsigned long long)ay * ry[q];
+                xy += (unsigned long long)ax * ry[q];
+            }
+            const uint32_t lx = mx, ly = my, lw = mw;
+            const unsigned long long lxx = xx, lyy = yy, lxy = xy;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, mx, o), b = __shfl_up_sync(0xFFFFFFFFu, my, o);
+                const uint32_t c = __shfl_up_sync(0xFFFFFFFFu, mw, o);
+                const unsigned long long d = __shfl_up_sync(0xFFFFFFFFu, xx, o), e = __shfl_up_sync(0xFFFFFFFFu, yy, o);
+                const unsigned long long f = __shfl_up_sync(0xFFFFFFFFu, xy, o);
+                if ((int)lane >= o) {
+                    mx += a; my += b; mw += c;
+                    xx += d; yy += e; xy += f;
+                }
+            }
+            // before this lane's points: the carry plus the earlier lanes
+            Moment at = carry;
+            at.Mx = wadd(at.Mx, mx - lx); at.My = wadd(at.My, my - ly); at.W = wadd(at.W, mw - lw);
+            at.Mxx = wadd(at.Mxx, (long long)(xx - lxx)); at.Myy = wadd(at.Myy, (long long)(yy - lyy));
+            at.Mxy = wadd(at.Mxy, (long long)(xy - lxy));
+            carry.Mx = wadd(carry.Mx, __shfl_sync(0xFFFFFFFFu, mx, 31));
+            carry.My = wadd(carry.My, __shfl_sync(0xFFFFFFFFu, my, 31));
+            carry.W = wadd(carry.W, __shfl_sync(0xFFFFFFFFu, mw, 31));
+            carry.Mxx = wadd(carry.Mxx, (long long)__shfl_sync(0xFFFFFFFFu, xx, 31));
+            carry.Myy = wadd(carry.Myy, (long long)__shfl_sync(0xFFFFFFFFu, yy, 31));
+            carry.Mxy = wadd(carry.Mxy, (long long)__shfl_sync(0xFFFFFFFFu, xy, 31));
+            atag_line_fit_point* out = F.line_fit + ext.start + i0;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (i0 + q >= end) break;
+                const uint32_t ax = wt[q] * rx[q], ay = wt[q] * ry[q];
+                at.Mx = wadd(at.Mx, ax);
+                at.My = wadd(at.My, ay);
+                at.W = wadd(at.W, wt[q]);
+                at.Mxx = wadd(at.Mxx, (long long)((unsigned long long)ax * rx[q]));
+                at.Myy = wadd(at.Myy, (long long)((unsigned long long)ay * ry[q]));
+                at.Mxy = wadd(at.Mxy, (long long)((unsigned long long)ax * ry[q]));
+                if (wide) {
+                    store_sector(out + q, at.Mx, at.My, at.Mxx, at.Myy);
+                    store_sector(reinterpret_cast<char*>(out + q) + 32, at.Mxy, at.W, 0ll, 0ll);
+                } else {
+                    store_moment(out + q, at);
+                }
+            }
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -891,18 +1014,12 @@ __global__ void __launch_bounds__(32 * CE_WARPS) k_cluster_errors(const __grid_c
         const uint32_t fidx = find_frame(run_offsets, n_frames, item);
         const FrameDesc& F = fs.get(fidx);
         const uint32_t r = item - run_offsets[fidx];
-        // the cluster whose runs contain r
-        uint32_t lo = 0, hi = F.counters[CNT_CLUSTERS];
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (F.cluster_runs[mid] <= r) lo = mid; else hi = mid;
-        }
-        const uint32_t cid = lo;
+        const uint32_t cid = F.runs[r].cluster;
         const atag_cluster_extents ext = F.cluster_extents[cid];
         const int n = (int)ext.count;
         const uint32_t k = min(20u, ext.count / 12u);
         const atag_line_fit_point* pts = F.line_fit + ext.start;
-        const int li0 = (int)((r - F.cluster_runs[cid]) * CE_RUN);
+        const int li0 = (int)F.runs[r].first;
         const int li1 = min(n, li0 + (int)CE_RUN);
         for (int s = li0; s < li1; s += 32) {
             if (s == li0) {
