@@ -34,6 +34,45 @@ __host__ __device__ __forceinline__ long long wsub(long long a, long long b) {
     return (long long)((unsigned long long)a - (unsigned long long)b);
 }
 
+// Single-precision operations rounded to nearest on both sides: the device
+// spells each one as its _rn intrinsic (never contracted into an FMA), the
+// host build compiles plain operators with -ffp-contract=off.
+__host__ __device__ __forceinline__ float rn_add(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fadd_rn(a, b);
+#else
+    return a + b;
+#endif
+}
+__host__ __device__ __forceinline__ float rn_sub(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fsub_rn(a, b);
+#else
+    return a - b;
+#endif
+}
+__host__ __device__ __forceinline__ float rn_mul(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+__host__ __device__ __forceinline__ float rn_div(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fdiv_rn(a, b);
+#else
+    return a / b;
+#endif
+}
+__host__ __device__ __forceinline__ float rn_fma(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+    return __fmaf_rn(a, b, c);
+#else
+    return __builtin_fmaf(a, b, c);
+#endif
+}
+
 // ---------------------------------------------------------------------------
 // hypotf of the reference's host library: the squares formed exactly in
 // double, summed with one rounding to 53 bits, the square root rounded to 53
@@ -104,27 +143,20 @@ __host__ __device__ __forceinline__ unsigned long long isqrt_2_60(unsigned long 
     while ((u + 1) * (u + 1) <= m) u++;
     return u;
 }
+// The value shifted up to bit 63, its low word folded into a sticky bit far
+// below the rounding position: a 32-bit conversion then rounds it once.
 __host__ __device__ __forceinline__ float u64_to_f32_rn(unsigned long long u) {
-    if (u < (1ull << 24)) return (float)(uint32_t)u;
-    const int L = 64 - clz64(u), sh = L - 24;  // sh >= 1
-    unsigned long long m = u >> sh;
-    const unsigned long long rem = u & ((1ull << sh) - 1ull), half = 1ull << (sh - 1);
-    int e = sh;
-    if (rem > half || (rem == half && (m & 1ull))) {
-        m++;
-        if (m >> 24) {
-            m >>= 1;
-            e++;
-        }
-    }
-    return u2f((uint32_t)(e + 23 + 127) << 23 | ((uint32_t)m & 0x7FFFFFu));
+    const int z = clz64(u) & 63;  // 0 stays 0 whatever the shift
+    const unsigned long long m = u << z;
+    const uint32_t hi = (uint32_t)(m >> 32) | ((uint32_t)m != 0u ? 1u : 0u);
+    return (float)hi * u2f((uint32_t)(127 + 32 - z) << 23);  // exact scaling
 }
 __host__ __device__ __forceinline__ float i64_to_f32_rn(long long v) {
     const unsigned long long u = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
     const float f = u64_to_f32_rn(u);
     return v < 0 ? -f : f;
 }
-__host__ __device__ __forceinline__ float hypot_f(float a, float b) {
+__host__ __device__ __forceinline__ float hypot_f_exact(float a, float b) {
     uint32_t x = f2u(a) & 0x7FFFFFFFu, y = f2u(b) & 0x7FFFFFFFu;
     if (x < y) {
         const uint32_t t = x;
@@ -176,6 +208,45 @@ __host__ __device__ __forceinline__ float hypot_f(float a, float b) {
         k++;
     }
     return u2f((uint32_t)(k + 23 + 127) << 23 | ((uint32_t)q & 0x7FFFFFu));
+}
+
+// The same value, usually without the wide integers.  a^2 + b^2 as a float
+// pair s + t (squares exact as pairs, |error| < 2^-45 s), r close to its
+// root, and T = s + t - r^2 (s - r^2 is exact or off by < 2^-45 s): the root
+// rounds to r while |T| stays below r u (u = ulp of r; the midpoints r +- u/2
+// square to r^2 +- r u + u^2 / 4), and to the next float up or down from
+// there to 3 r u.  r u >= 2^-24 s, so a margin of 2^-18 around both limits
+// covers every error above; inside it (1 call in 10^5, exact ties included),
+// for r next to a power of two and for inputs that could over- or underflow,
+// the exact path decides.
+__host__ __device__ __forceinline__ float hypot_f(float a, float b) {
+    uint32_t xb = f2u(a) & 0x7FFFFFFFu, yb = f2u(b) & 0x7FFFFFFFu;
+    if (xb < yb) {
+        const uint32_t t = xb;
+        xb = yb;
+        yb = t;
+    }
+    if (xb >= 0x30800000u && xb < 0x5D800000u) {  // [2^-30, 2^60)
+        const float x = u2f(xb), y = u2f(yb);
+        const float h = rn_mul(x, x), l = rn_fma(x, x, -h), h2 = rn_mul(y, y), l2 = rn_fma(y, y, -h2);
+        const float s = rn_add(h, h2), t = rn_add(rn_sub(h2, rn_sub(s, h)), rn_add(l, l2));
+#ifdef __CUDA_ARCH__
+        float r;
+        asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(s));
+#else
+        const float r = __builtin_sqrtf(s);
+#endif
+        const uint32_t rb = f2u(r);
+        const float T = rn_add(rn_fma(-r, r, s), t);
+        const float B = rn_mul(r, u2f((rb & 0x7F800000u) - (23u << 23)));
+        const float A = u2f(f2u(T) & 0x7FFFFFFFu);
+        if (rb & 0x007FFFFEu) {
+            if (A < rn_mul(B, 1.0f - 0x1p-18f)) return r;
+            if (A > rn_mul(B, 1.0f + 0x1p-18f) && A < rn_mul(B, 3.0f - 0x1p-16f))
+                return u2f((f2u(T) >> 31) ? rb - 1u : rb + 1u);
+        }
+    }
+    return hypot_f_exact(a, b);
 }
 
 // bytes per pixel of an atag_pixel_format (0 for an unknown format)
@@ -262,38 +333,6 @@ __device__ __forceinline__ bool valid_blob(const FilterParams& f, uint32_t count
 // ---------------------------------------------------------------------------
 // Line-fit moments (line_fit_point.h, fit_quad.cpp:15-105)
 // ---------------------------------------------------------------------------
-// Single-precision operations rounded to nearest on both sides: the device
-// spells each one as its _rn intrinsic (never contracted into an FMA), the
-// host build compiles plain operators with -ffp-contract=off.
-__host__ __device__ __forceinline__ float rn_add(float a, float b) {
-#ifdef __CUDA_ARCH__
-    return __fadd_rn(a, b);
-#else
-    return a + b;
-#endif
-}
-__host__ __device__ __forceinline__ float rn_sub(float a, float b) {
-#ifdef __CUDA_ARCH__
-    return __fsub_rn(a, b);
-#else
-    return a - b;
-#endif
-}
-__host__ __device__ __forceinline__ float rn_mul(float a, float b) {
-#ifdef __CUDA_ARCH__
-    return __fmul_rn(a, b);
-#else
-    return a * b;
-#endif
-}
-__host__ __device__ __forceinline__ float rn_div(float a, float b) {
-#ifdef __CUDA_ARCH__
-    return __fdiv_rn(a, b);
-#else
-    return a / b;
-#endif
-}
-
 struct Moment {
     long long Mx, My, Mxx, Myy, Mxy, W;
 };
@@ -445,20 +484,6 @@ __device__ __forceinline__ float window_error(const atag_line_fit_point* points,
     Moment m = get_moment(points + start, count, i0, i1, &n);
     float e;
     fit_line(m, n, nullptr, &e, nullptr);
-    return e;
-}
-
-// window_error for a point at cluster-local index i of a cluster of n > 2k
-// points whose prefix sums start at `points` (same arithmetic, no modulo).
-__device__ __forceinline__ float window_error_local(const atag_line_fit_point* points, uint32_t n, uint32_t k,
-                                                    uint32_t i) {
-    if (k < 2) return __int_as_float(0x7fc00000);
-    uint32_t i0 = i >= k ? i - k : i + n - k;
-    uint32_t i1 = i + k < n ? i + k : i + k - n;
-    unsigned long long cnt;
-    Moment m = get_moment(points, n, i0, i1, &cnt);
-    float e;
-    fit_line(m, cnt, nullptr, &e, nullptr);
     return e;
 }
 

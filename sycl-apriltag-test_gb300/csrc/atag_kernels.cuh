@@ -53,11 +53,11 @@ struct FrameDesc {
     uint32_t* quad_ok;                 // per rank q
     // cluster points
     uint32_t cpoint_cap;
-    unsigned long long* sortbuf;       // (theta key << 32) | packed; then the sorted points' line-fit inputs;
-                                       // then the corner candidates
+    unsigned long long* sortbuf;       // (theta key << 32) | packed; then the sorted points' line-fit inputs
     atag_cluster_point* cluster_points;
     atag_line_fit_point* line_fit;
-    float* errbuf;                     // 2 floats per point (sort scratch of clusters past the shared memory)
+    float* errbuf;                     // 8 bytes per point: sort scratch of clusters past the shared memory,
+                                       // then the corner candidates
     uint32_t* cluster_work;            // small clusters from the front, large from the back
     uint32_t* cluster_runs;            // first run (CE_RUN points) of each cluster
     struct RunInfo* runs;              // per run
@@ -203,8 +203,8 @@ __global__ void k_cluster_sort_small(const __grid_constant__ FrameSet fs, const 
 __global__ void k_cluster_sort_large(const __grid_constant__ FrameSet fs, const uint32_t* work_offsets,
                                      uint32_t n_frames, uint32_t* work_counter, uint32_t cap);
 __global__ void k_cluster_lines(const __grid_constant__ FrameSet fs, const uint32_t* run_offsets, uint32_t n_frames);
-__global__ void k_cluster_errors(const __grid_constant__ FrameSet fs, const uint32_t* run_offsets,
-                                 uint32_t n_frames, uint32_t* work_counter);
+constexpr uint32_t CE_LINES_SMEM = 4 * 12432;  // four warps' RunSums
+__global__ void k_cluster_prefix(const __grid_constant__ FrameSet fs, const uint32_t* run_offsets);
 __global__ void k_cluster_peaks(const __grid_constant__ FrameSet fs, const uint32_t* cluster_offsets,
                                 uint32_t n_frames);
 __global__ void k_peaks_scan(const __grid_constant__ FrameSet fs, PipelineParams p);

@@ -69,6 +69,7 @@ atag_status ensure_device(DeviceInfo** out) {
         e = cudaFuncGetAttributes(&fa, k_threshold);
         if (e != cudaSuccess) return fail(ATAG_ERR_NO_DEVICE, "kernels do not load: %s", cudaGetErrorString(e));
         CK(cudaFuncSetAttribute(k_cluster_sort_large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF_LARGE_SMEM));
+        CK(cudaFuncSetAttribute(k_cluster_lines, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CE_LINES_SMEM));
         CK(cudaFuncSetAttribute(k_peaks_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PK_SMEM));
         d.num_sms = prop.multiProcessorCount;
         d.smem_optin = prop.sharedMemPerBlockOptin;
@@ -619,7 +620,7 @@ atag_status atag_cluster(const atag_boundary_point* points, const uint64_t* keys
     k_cluster_sort_small<<<sms * 8, CF_SMALL_THREADS, cf_smem(CF_SMALL_CAP, CF_SMALL_NB), s>>>(fs, off_small, 1, wc,
                                                                                               CF_SMALL_CAP);
     LAUNCHED();
-    k_cluster_lines<<<sms * 8, 128, 0, s>>>(fs, off_runs, 1);
+    k_cluster_prefix<<<sms * 4, 128, 0, s>>>(fs, off_runs);
     LAUNCHED();
     k_stage_cluster_out<<<sms * 4, 256, 0, s>>>(fs, o->cluster_indices, (unsigned long long*)o->filtered_keys);
     LAUNCHED();
@@ -987,10 +988,8 @@ static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, con
     LAUNCHED();
     CK(cudaEventRecord(det->join[lane], side));
     CK(cudaStreamWaitEvent(s, det->join[lane], 0));
-    k_cluster_lines<<<sms * 8, 128, 0, s>>>(fs, off_runs, (uint32_t)n);
-    LAUNCHED();
     STAGE(10);
-    k_cluster_errors<<<sms * 8, 256, 0, s>>>(fs, off_runs, (uint32_t)n, wc + 2);
+    k_cluster_lines<<<sms * 4, 128, CE_LINES_SMEM, s>>>(fs, off_runs, (uint32_t)n);
     LAUNCHED();
     STAGE(11);
     k_cluster_peaks<<<sms * 4, 256, 0, s>>>(fs, off_clusters, (uint32_t)n);

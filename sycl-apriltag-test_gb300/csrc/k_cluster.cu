@@ -20,10 +20,9 @@
 //      cluster's segment with their theta key; the rest are dropped;
 //   4. k_cluster_sort: one CTA per cluster sorts by (theta, point) in
 //      shared memory and writes ClusterPoints and the line-fit inputs;
-//      k_cluster_lines: line-fit prefix sums, a warp per run of points;
-//      k_cluster_errors: fit_lines (windowed errors, 7-tap filter, peaks)
-//      flat over all cluster points; k_cluster_peaks: the 10 best peaks of
-//      each cluster;
+//      k_cluster_lines: line-fit prefix sums and fit_lines (windowed errors,
+//      7-tap filter, peaks), a warp per run of points; k_cluster_peaks: the
+//      10 best peaks of each cluster;
 //   5. k_peaks_scan / k_index_quads / k_compact_quads: peak extents,
 //      do_indexing and the corner intersection, quads in reference order.
 #include "atag_kernels.cuh"
@@ -886,107 +885,26 @@ __global__ void __launch_bounds__(CF_LARGE_THREADS, 1) k_cluster_sort_large(cons
     cluster_sort<CF_LARGE_THREADS, 4, CF_LARGE_NB, CF_MAX_RUNS>(fs, work_offsets, n_frames, work_counter, cap);
 }
 
-// The segmented inclusive scan of the moments (main.cpp:796-801): one warp per
-// run of CE_RUN points, from the moments of the cluster's earlier runs.  Lane
-// l of a chunk of 128 points has points 4 l .. 4 l + 3: one warp scan of the
-// lanes' sums (W, Mx and My in 32 bits: exact over 128 points), then each
-// lane adds its points one by one and stores their LineFitPoints, a 32-byte
-// sector per store where the array's alignment allows it (the detector's own
-// always does; a caller's array may not).
-__device__ __forceinline__ void store_sector(void* p, long long a, long long b, long long c, long long d) {
-    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
-}
-
-__global__ void __launch_bounds__(128, 4) k_cluster_lines(const __grid_constant__ FrameSet fs,
-                                                       const uint32_t* __restrict__ run_offsets, uint32_t n_frames) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t total = run_offsets[n_frames], stride = gridDim.x * (blockDim.x >> 5);
-    // items go round the CTAs first, so that a few still use every SM
-    for (uint32_t item = blockIdx.x + gridDim.x * (threadIdx.x >> 5); item < total; item += stride) {
-        const uint32_t fidx = find_frame(run_offsets, n_frames, item);
-        const FrameDesc& F = fs.get(fidx);
-        const RunInfo R = F.runs[item - run_offsets[fidx]];
-        const atag_cluster_extents ext = F.cluster_extents[R.cluster];
-        const unsigned long long* in = F.sortbuf + ext.start;
-        const bool wide = (reinterpret_cast<uintptr_t>(F.line_fit) & 31u) == 0;
-        Moment carry{R.before[0], R.before[1], R.before[2], R.before[3], R.before[4], R.before[5]};
-        const uint32_t end = min(ext.count, R.first + CE_RUN);
-#pragma unroll 1
-        for (uint32_t c0 = R.first; c0 < end; c0 += 128) {
-            const uint32_t i0 = c0 + 4 * lane;
-            uint32_t wt[4], rx[4], ry[4];
-            uint32_t mx = 0, my = 0, mw = 0;
-            unsigned long long xx = 0, yy = 0, xy = 0;
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const unsigned long long v = i0 + q < end ? __ldcg(in + i0 + q) : 0ull;
-                rx[q] = (uint32_t)v & 0xFFFFu;
-                ry[q] = (uint32_t)v >> 16;
-                wt[q] = (uint32_t)(v >> 32);
-                const uint32_t ax = wt[q] * rx[q], ay = wt[q] * ry[q];
-                mw += wt[q];
-                mx += ax;
-                my += ay;
-                xx += (unsigned long long)ax * rx[q];
-                yy += (unsigned long long)ay * ry[q];
-                xy += (unsigned long long)ax * ry[q];
-            }
-            const uint32_t lx = mx, ly = my, lw = mw;
-            const unsigned long long lxx = xx, lyy = yy, lxy = xy;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, mx, o), b = __shfl_up_sync(0xFFFFFFFFu, my, o);
-                const uint32_t c = __shfl_up_sync(0xFFFFFFFFu, mw, o);
-                const unsigned long long d = __shfl_up_sync(0xFFFFFFFFu, xx, o), e = __shfl_up_sync(0xFFFFFFFFu, yy, o);
-                const unsigned long long f = __shfl_up_sync(0xFFFFFFFFu, xy, o);
-                if ((int)lane >= o) {
-                    mx += a; my += b; mw += c;
-                    xx += d; yy += e; xy += f;
-                }
-            }
-            // before this lane's points: the carry plus the earlier lanes
-            Moment at = carry;
-            at.Mx = wadd(at.Mx, mx - lx); at.My = wadd(at.My, my - ly); at.W = wadd(at.W, mw - lw);
-            at.Mxx = wadd(at.Mxx, (long long)(xx - lxx)); at.Myy = wadd(at.Myy, (long long)(yy - lyy));
-            at.Mxy = wadd(at.Mxy, (long long)(xy - lxy));
-            carry.Mx = wadd(carry.Mx, __shfl_sync(0xFFFFFFFFu, mx, 31));
-            carry.My = wadd(carry.My, __shfl_sync(0xFFFFFFFFu, my, 31));
-            carry.W = wadd(carry.W, __shfl_sync(0xFFFFFFFFu, mw, 31));
-            carry.Mxx = wadd(carry.Mxx, (long long)__shfl_sync(0xFFFFFFFFu, xx, 31));
-            carry.Myy = wadd(carry.Myy, (long long)__shfl_sync(0xFFFFFFFFu, yy, 31));
-            carry.Mxy = wadd(carry.Mxy, (long long)__shfl_sync(0xFFFFFFFFu, xy, 31));
-            atag_line_fit_point* out = F.line_fit + ext.start + i0;
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                if (i0 + q >= end) break;
-                const uint32_t ax = wt[q] * rx[q], ay = wt[q] * ry[q];
-                at.Mx = wadd(at.Mx, ax);
-                at.My = wadd(at.My, ay);
-                at.W = wadd(at.W, wt[q]);
-                at.Mxx = wadd(at.Mxx, (long long)((unsigned long long)ax * rx[q]));
-                at.Myy = wadd(at.Myy, (long long)((unsigned long long)ay * ry[q]));
-                at.Mxy = wadd(at.Mxy, (long long)((unsigned long long)ax * ry[q]));
-                if (wide) {
-                    store_sector(out + q, at.Mx, at.My, at.Mxx, at.Myy);
-                    store_sector(reinterpret_cast<char*>(out + q) + 32, at.Mxy, at.W, 0ll, 0ll);
-                } else {
-                    store_moment(out + q, at);
-                }
-            }
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
-// 4b. fit_lines (fit_quad.cpp:153-375) in its cyclic form: the error of the
-// window around each point, the 7-tap filter and the strict local maxima.
-// One warp per run of up to CE_RUN consecutive points of one cluster, 32
-// points per step: the warp keeps the errors of positions [s-4, s+36) and
-// the filtered errors of [s-1, s+33) in shared memory (cluster-local,
-// cyclic indices), carrying the last 8 errors into the next step.  Maxima
-// are appended to their cluster's candidate list, which reuses the
-// cluster's segment of the sort-key buffer (a cyclic sequence of n values
-// has at most n/2 strict maxima).
+// 4b. the segmented inclusive scan of the moments (main.cpp:796-801) and
+// fit_lines (fit_quad.cpp:153-375) in its cyclic form: the error of the window
+// around each point, the 7-tap filter and the strict local maxima.
+// One warp per run of up to CE_RUN consecutive points of one cluster.  It
+// reads the line-fit inputs of the run and, for the errors, of 24 points on
+// either side (cyclic), and scans them in chunks of 128: lane l has points 4 l
+// .. 4 l + 3, one warp scan of the lanes' sums, then each lane adds its points
+// one by one.  With the moments of the cluster's earlier runs that gives the
+// run's LineFitPoints, and the scan itself, kept in shared memory, every
+// window's moment: integer sums, so the same whatever they start from, and no
+// prefix sum is read back from memory.  W, Mx and My stay below 2^32 over a run
+// and its margins (W <= 362, coordinates <= 2^15).  Then lane l filters
+// positions 8 l .. 8 l + 7 from 14 errors and compares with its neighbour
+// lanes'.  Maxima are appended to their cluster's candidate list in the
+// cluster's segment of errbuf (a cyclic sequence of n values has at most n/2
+// strict maxima).  Bound by latency (128 registers and 50 KB of shared memory
+// leave 16 warps per SM); as two kernels, the errors reading prefix sums back,
+// 64 frames of 1080p took 125 + 197 us and a lone frame 10 + 30 us, now 277 and
+// 20 us (with the cheaper hypotf and conversions in both: 125 + 235 and 10 + 16).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cyclic(int i, int n) {  // i in [-n, 3n)
     if (i < 0) i += n;
@@ -994,73 +912,213 @@ __device__ __forceinline__ uint32_t cyclic(int i, int n) {  // i in [-n, 3n)
     return (uint32_t)i;
 }
 
-constexpr int CE_WARPS = 8;
+__device__ __forceinline__ void store_sector(void* p, long long a, long long b, long long c, long long d) {
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
+}
 
-__global__ void __launch_bounds__(32 * CE_WARPS) k_cluster_errors(const __grid_constant__ FrameSet fs,
-                                                                  const uint32_t* __restrict__ run_offsets,
-                                                                  uint32_t n_frames,
-                                                                  uint32_t* __restrict__ work_counter) {
-    __shared__ float s_err[CE_WARPS][40];
-    __shared__ float s_flt[CE_WARPS][34];
-    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    float* e = s_err[wid];
-    float* f = s_flt[wid];
-    const uint32_t total = run_offsets[n_frames];
-    for (;;) {
-        uint32_t item = 0;
-        if (lane == 0) item = atomicAdd(work_counter, 1u);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= total) return;
-        const uint32_t fidx = find_frame(run_offsets, n_frames, item);
-        const FrameDesc& F = fs.get(fidx);
-        const uint32_t r = item - run_offsets[fidx];
-        const uint32_t cid = F.runs[r].cluster;
-        const atag_cluster_extents ext = F.cluster_extents[cid];
-        const int n = (int)ext.count;
-        const uint32_t k = min(20u, ext.count / 12u);
-        const atag_line_fit_point* pts = F.line_fit + ext.start;
-        const int li0 = (int)F.runs[r].first;
-        const int li1 = min(n, li0 + (int)CE_RUN);
-        for (int s = li0; s < li1; s += 32) {
-            if (s == li0) {
-                e[lane] = window_error_local(pts, n, k, cyclic(s - 4 + (int)lane, n));
-                if (lane < 8) e[32 + lane] = window_error_local(pts, n, k, cyclic(s + 28 + (int)lane, n));
+struct ShortMoment {  // of at most a run and its margins
+    uint32_t w, mx, my;
+    unsigned long long xx, yy, xy;
+};
+__device__ __forceinline__ ShortMoment s_add(const ShortMoment& a, const ShortMoment& b) {
+    return ShortMoment{a.w + b.w, a.mx + b.mx, a.my + b.my, a.xx + b.xx, a.yy + b.yy, a.xy + b.xy};
+}
+__device__ __forceinline__ ShortMoment s_sub(const ShortMoment& a, const ShortMoment& b) {
+    return ShortMoment{a.w - b.w, a.mx - b.mx, a.my - b.my, a.xx - b.xx, a.yy - b.yy, a.xy - b.xy};
+}
+__device__ __forceinline__ ShortMoment s_shfl(const ShortMoment& a, int src) {
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    return ShortMoment{__shfl_sync(FULL, a.w, src), __shfl_sync(FULL, a.mx, src), __shfl_sync(FULL, a.my, src),
+                       __shfl_sync(FULL, a.xx, src), __shfl_sync(FULL, a.yy, src), __shfl_sync(FULL, a.xy, src)};
+}
+// of one point's line-fit inputs (linefit_rxyw)
+__device__ __forceinline__ ShortMoment s_of(unsigned long long v) {
+    const uint32_t rx = (uint32_t)v & 0xFFFFu, ry = (uint32_t)v >> 16, w = (uint32_t)(v >> 32);
+    const uint32_t ax = w * rx, ay = w * ry;
+    return ShortMoment{w, ax, ay, (unsigned long long)ax * rx, (unsigned long long)ay * ry, (unsigned long long)ax * ry};
+}
+
+// fit_line's error (fit_quad.cpp:37-105) of a window of `count` <= 41 points:
+// the same integers, in the widths they need
+__device__ __forceinline__ float window_fit_error(const ShortMoment& m, uint32_t count) {
+    const unsigned long long cxx = m.xx * m.w - (unsigned long long)m.mx * m.mx;
+    const unsigned long long cyy = m.yy * m.w - (unsigned long long)m.my * m.my;
+    const unsigned long long cxy = m.xy * m.w - (unsigned long long)m.mx * m.my;
+    const float sdist = hypot_f(i64_to_f32_rn((long long)(cxx - cyy)), i64_to_f32_rn((long long)(2 * cxy)));
+    const float num = __fsub_rn(i64_to_f32_rn((long long)(cxx + cyy)), sdist);
+    const float eig = __fdiv_rn(num, (float)(8u * m.w * m.w));
+    return __fmul_rn((float)count, eig);
+}
+
+constexpr uint32_t CE_MARGIN = 24;                           // window (20) and filter (3) reach, and a neighbour
+constexpr uint32_t CE_SPAN = CE_RUN + 2 * CE_MARGIN;         // points a warp scans
+constexpr uint32_t CE_ERRS = CE_RUN + 8;                     // errors of positions -4 .. CE_RUN + 3
+// Sums of the points before local index j at [CE_BASE + j]: the base keeps a
+// lane's four sums (j = i + 1 .. i + 4, i a multiple of 4) 16-byte aligned.
+constexpr uint32_t CE_BASE = 3;
+struct RunSums {
+    unsigned long long xx[CE_BASE + CE_SPAN + 5], yy[CE_BASE + CE_SPAN + 5], xy[CE_BASE + CE_SPAN + 5];
+    uint32_t w[CE_BASE + CE_SPAN + 5], mx[CE_BASE + CE_SPAN + 5], my[CE_BASE + CE_SPAN + 5];
+    float err[CE_ERRS + CE_ERRS / 8];  // error i at i + i / 8: lanes eight apart read distinct banks
+    uint32_t pad_[3];
+};
+static_assert((CE_BASE + CE_SPAN + 5) % 4 == 0 && sizeof(RunSums) % 16 == 0, "16-byte aligned sums");
+
+template <bool ERRORS>
+__device__ __forceinline__ void cluster_run(const FrameDesc& F, const RunInfo& R, RunSums* S) {
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31, cid = R.cluster, first = R.first;
+    const atag_cluster_extents ext = F.cluster_extents[cid];
+    const uint32_t n = ext.count, len = min(CE_RUN, n - first);
+    constexpr uint32_t M = ERRORS ? CE_MARGIN : 0u;
+    const uint32_t span = len + 2 * M;  // local index i: point first - M + i (cyclic)
+    const unsigned long long* in = F.sortbuf + ext.start;
+    // a 32-byte sector per store where the array's alignment allows it (the
+    // detector's own always does; a caller's array may not)
+    const bool wide = (reinterpret_cast<uintptr_t>(F.line_fit) & 31u) == 0;
+    atag_line_fit_point* out = F.line_fit + ext.start + first;
+    ShortMoment carry{0, 0, 0, 0ull, 0ull, 0ull}, start{0, 0, 0, 0ull, 0ull, 0ull};
+    if (ERRORS && lane == 0) {
+        S->w[CE_BASE] = S->mx[CE_BASE] = S->my[CE_BASE] = 0u;
+        S->xx[CE_BASE] = S->yy[CE_BASE] = S->xy[CE_BASE] = 0ull;
+    }
+#pragma unroll 1
+    for (uint32_t c0 = 0; c0 < span; c0 += 128) {
+        const uint32_t i0 = c0 + 4 * lane;
+        unsigned long long v[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint32_t i = i0 + q;
+            v[q] = i < span ? __ldcg(in + (ERRORS ? cyclic((int)(first + i) - (int)M, (int)n) : first + i)) : 0ull;
+        }
+        ShortMoment sum = s_of(v[0]);
+#pragma unroll
+        for (int q = 1; q < 4; q++) sum = s_add(sum, s_of(v[q]));
+        ShortMoment incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const ShortMoment t{__shfl_up_sync(FULL, incl.w, o),  __shfl_up_sync(FULL, incl.mx, o),
+                                __shfl_up_sync(FULL, incl.my, o), __shfl_up_sync(FULL, incl.xx, o),
+                                __shfl_up_sync(FULL, incl.yy, o), __shfl_up_sync(FULL, incl.xy, o)};
+            if ((int)lane >= o) incl = s_add(incl, t);
+        }
+        ShortMoment at = s_add(carry, s_sub(incl, sum));  // of the points before this lane's
+        carry = s_add(carry, s_shfl(incl, 31));
+        // the sums before the run itself: after the last margin point
+        if (ERRORS && c0 == 0) start = s_shfl(s_add(at, sum), (int)(M / 4 - 1));
+        ShortMoment p[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            at = s_add(at, s_of(v[q]));
+            p[q] = at;
+            const uint32_t i = i0 + q;
+            if ((int)i < (int)M || i - M >= len) continue;
+            const ShortMoment d = s_sub(at, start);
+            const long long Mx = wadd(R.before[0], d.mx), My = wadd(R.before[1], d.my), W = wadd(R.before[5], d.w);
+            const long long Mxx = wadd(R.before[2], (long long)d.xx), Myy = wadd(R.before[3], (long long)d.yy);
+            const long long Mxy = wadd(R.before[4], (long long)d.xy);
+            atag_line_fit_point* o = out + (i - M);
+            if (wide) {
+                store_sector(o, Mx, My, Mxx, Myy);
+                store_sector(reinterpret_cast<char*>(o) + 32, Mxy, W, 0ll, 0ll);
             } else {
-                const float carry = lane < 8 ? e[32 + lane] : 0.0f;
-                __syncwarp();
-                if (lane < 8) e[lane] = carry;
-                e[8 + lane] = window_error_local(pts, n, k, cyclic(s + 4 + (int)lane, n));
+                store_moment(o, Moment{Mx, My, Mxx, Myy, Mxy, W});
             }
-            __syncwarp();
-            // cyclic 7-tap filter (fit_quad.cpp:296-324): f[j] is position s - 1 + j
-            {
-                float acc = 0.0f;
+        }
+        if (ERRORS && i0 < span) {
+            const uint32_t j = CE_BASE + i0 + 1;
+            *reinterpret_cast<uint4*>(S->w + j) = make_uint4(p[0].w, p[1].w, p[2].w, p[3].w);
+            *reinterpret_cast<uint4*>(S->mx + j) = make_uint4(p[0].mx, p[1].mx, p[2].mx, p[3].mx);
+            *reinterpret_cast<uint4*>(S->my + j) = make_uint4(p[0].my, p[1].my, p[2].my, p[3].my);
 #pragma unroll
-                for (int j = 0; j < 7; j++) acc = __fadd_rn(acc, __fmul_rn(e[lane + j], filter_tap(j)));
-                f[lane] = acc;
-                if (lane < 2) {
-                    float a2 = 0.0f;
-#pragma unroll
-                    for (int j = 0; j < 7; j++) a2 = __fadd_rn(a2, __fmul_rn(e[32 + lane + j], filter_tap(j)));
-                    f[32 + lane] = a2;
-                }
+            for (int q = 0; q < 4; q += 2) {
+                *reinterpret_cast<ulonglong2*>(S->xx + j + q) = make_ulonglong2(p[q].xx, p[q + 1].xx);
+                *reinterpret_cast<ulonglong2*>(S->yy + j + q) = make_ulonglong2(p[q].yy, p[q + 1].yy);
+                *reinterpret_cast<ulonglong2*>(S->xy + j + q) = make_ulonglong2(p[q].xy, p[q + 1].xy);
             }
-            __syncwarp();
-            // strict local maxima (fit_quad.cpp:341-371) with error != 0
-            // (main.cpp:832-835); global point 0 is never a corner (the
-            // first work-group's first output is x = 1, fit_quad.cpp:182-190)
-            const int li = s + (int)lane;
-            if (li < li1) {
-                const float cur = f[lane + 1];
-                if (cur > f[lane] && cur > f[lane + 2] && cur != 0.0f && !(cid == 0 && li == 0)) {
-                    const uint32_t at = atomicAdd(F.peak_count + cid, 1u);
-                    F.sortbuf[ext.start + at] =
-                        ((unsigned long long)float_order_key(cur) << 32) | (uint32_t)(~(uint32_t)li);
-                }
-            }
-            __syncwarp();
         }
     }
+    if (!ERRORS) return;
+    __syncwarp();
+    // error i: position first - 4 + i, the window of k points on either side
+    const uint32_t k = min(20u, n / 12u);
+    constexpr uint32_t ILP = 3;
+    for (uint32_t i0 = lane; i0 < len + 8; i0 += 32 * ILP) {
+#pragma unroll
+        for (uint32_t u = 0; u < ILP; u++) {
+            const uint32_t i = i0 + 32 * u;
+            if (i >= len + 8) break;
+            const uint32_t lo = CE_BASE + (M - 4) + i - k, hi = lo + 2 * k + 1;
+            const ShortMoment m{S->w[hi] - S->w[lo],   S->mx[hi] - S->mx[lo], S->my[hi] - S->my[lo],
+                                S->xx[hi] - S->xx[lo], S->yy[hi] - S->yy[lo], S->xy[hi] - S->xy[lo]};
+            S->err[i + (i >> 3)] = window_fit_error(m, 2 * k + 1);
+        }
+    }
+    __syncwarp();
+    // cyclic 7-tap filter (fit_quad.cpp:296-324): output o is position
+    // first + o, from errors o + 1 .. o + 7
+    auto filter = [&](const float* e) {
+        float acc = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 7; j++) acc = __fadd_rn(acc, __fmul_rn(e[j], filter_tap(j)));
+        return acc;
+    };
+    auto err_at = [&](uint32_t i) { return S->err[i + (i >> 3)]; };
+    float f[10];  // outputs 8 l - 1 .. 8 l + 8
+    {
+        float e[14];
+#pragma unroll
+        for (int j = 0; j < 14; j++) e[j] = err_at(min(8 * lane + 1 + j, CE_ERRS - 1));
+#pragma unroll
+        for (int o = 0; o < 8; o++) f[1 + o] = filter(e + o);
+        // the outputs before the run (lane 0) and past a full one (lane 31)
+        const uint32_t b = lane == 0 ? 0u : CE_RUN + 1u;
+#pragma unroll
+        for (int j = 0; j < 7; j++) e[j] = err_at(b + j);
+        const float edge = filter(e);
+        f[0] = __shfl_up_sync(FULL, f[8], 1);
+        f[9] = __shfl_down_sync(FULL, f[1], 1);
+        if (lane == 0) f[0] = edge;
+        if (lane == 31) f[9] = edge;
+    }
+    // strict local maxima (fit_quad.cpp:341-371) with error != 0
+    // (main.cpp:832-835); global point 0 is never a corner (the first
+    // work-group's first output is x = 1, fit_quad.cpp:182-190)
+    unsigned long long* cand = reinterpret_cast<unsigned long long*>(F.errbuf) + ext.start;
+#pragma unroll
+    for (int o = 0; o < 8; o++) {
+        const uint32_t li = first + 8 * lane + o;
+        const float cur = f[1 + o];
+        if (8 * lane + o < len && cur > f[o] && cur > f[o + 2] && cur != 0.0f && !(cid == 0 && li == 0)) {
+            const uint32_t at = atomicAdd(F.peak_count + cid, 1u);
+            cand[at] = ((unsigned long long)float_order_key(cur) << 32) | (uint32_t)(~li);
+        }
+    }
+    __syncwarp();
+}
+
+// Items go round the CTAs first, so that a few still use every SM.
+constexpr int CE_WARPS = 4;
+static_assert(CE_LINES_SMEM == CE_WARPS * sizeof(RunSums), "dynamic shared memory of k_cluster_lines");
+__global__ void __launch_bounds__(32 * CE_WARPS, 4) k_cluster_lines(const __grid_constant__ FrameSet fs,
+                                                                    const uint32_t* __restrict__ run_offsets,
+                                                                    uint32_t n_frames) {
+    extern __shared__ __align__(16) unsigned char smem_runs[];
+    const uint32_t wid = threadIdx.x >> 5, total = run_offsets[n_frames];
+    RunSums* S = reinterpret_cast<RunSums*>(smem_runs) + wid;
+    for (uint32_t item = blockIdx.x + gridDim.x * wid; item < total; item += gridDim.x * CE_WARPS) {
+        const uint32_t fidx = find_frame(run_offsets, n_frames, item);
+        const FrameDesc& F = fs.get(fidx);
+        cluster_run<true>(F, F.runs[item - run_offsets[fidx]], S);
+    }
+}
+// the stage entry point: prefix sums only
+__global__ void __launch_bounds__(32 * CE_WARPS, 4) k_cluster_prefix(const __grid_constant__ FrameSet fs,
+                                                                     const uint32_t* __restrict__ run_offsets) {
+    const FrameDesc& F = fs.get(0);
+    const uint32_t total = run_offsets[1];
+    for (uint32_t item = blockIdx.x + gridDim.x * (threadIdx.x >> 5); item < total; item += gridDim.x * CE_WARPS)
+        cluster_run<false>(F, F.runs[item], nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -1078,7 +1136,8 @@ __global__ void __launch_bounds__(256) k_cluster_peaks(const __grid_constant__ F
         const FrameDesc& F = fs.get(fidx);
         const uint32_t cid = item - cluster_offsets[fidx];
         const uint32_t npeaks = F.peak_count[cid];
-        const unsigned long long* cand = F.sortbuf + F.cluster_extents[cid].start;
+        const unsigned long long* cand =
+            reinterpret_cast<const unsigned long long*>(F.errbuf) + F.cluster_extents[cid].start;
         const uint32_t take = npeaks < 10u ? npeaks : 10u;
         unsigned long long last = ~0ull;
         for (uint32_t j = 0; j < take; j++) {
