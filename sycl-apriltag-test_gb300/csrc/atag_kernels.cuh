@@ -169,10 +169,9 @@ __global__ void k_threshold(const __grid_constant__ FrameSet fs, int min_diff, i
 // CCL tiles of 32 x 8 or 32 x 16 blocks (2x2 pixels)
 __global__ void k_ccl_local_r8(const __grid_constant__ FrameSet fs);
 __global__ void k_ccl_local_r16(const __grid_constant__ FrameSet fs);
-__global__ void k_ccl_border_r8(const __grid_constant__ FrameSet fs);
+__global__ void k_ccl_local_stage(const __grid_constant__ FrameSet fs);  // r16 over a caller's image: any byte values
 __global__ void k_ccl_local_r32(const __grid_constant__ FrameSet fs);
 __global__ void k_ccl_border_r16(const __grid_constant__ FrameSet fs);
-__global__ void k_ccl_border_r32(const __grid_constant__ FrameSet fs);
 __global__ void k_ccl_border_edges_r8(const __grid_constant__ FrameSet fs);
 __global__ void k_ccl_border_edges_r16(const __grid_constant__ FrameSet fs);
 __global__ void k_ccl_border_edges_r32(const __grid_constant__ FrameSet fs);

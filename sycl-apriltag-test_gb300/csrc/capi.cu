@@ -446,22 +446,13 @@ atag_status atag_threshold_image(const uint8_t* grey, uint8_t* extrema, uint8_t*
     return ATAG_OK;
 }
 
-static atag_status launch_segmentation(const FrameSet& fs, size_t max_w, size_t max_h, size_t nf, cudaStream_t s,
-                                       int rows = 16) {
-    size_t tiles = cdiv(max_w / 2, 32) * cdiv(max_h / 2, (size_t)rows);
-    size_t border = tiles * (32 + 2 * (rows - 1));
-    if (rows == 8) {
-        k_ccl_local_r8<<<ccl_grid(max_w, max_h, 8, nf), 32 * 8, 0, s>>>(fs);
-        LAUNCHED();
-        k_ccl_border_r8<<<grid2(cdiv(border, 256), nf), 256, 0, s>>>(fs);
-        LAUNCHED();
-    } else {
-        k_ccl_local_r16<<<ccl_grid(max_w, max_h, 16, nf), 32 * 16, 0, s>>>(fs);
-        LAUNCHED();
-        k_ccl_border_r16<<<grid2(cdiv(border, 256), nf), 256, 0, s>>>(fs);
-        LAUNCHED();
-    }
-    k_ccl_final<<<final_grid(max_w, max_h, nf), CCL_FINAL_THREADS, 0, s>>>(fs);
+static atag_status launch_segmentation(const FrameSet& fs, size_t w, size_t h, cudaStream_t s) {
+    const size_t border = cdiv(w / 2, 32) * cdiv(h / 2, 16) * (32 + 2 * (16 - 1));
+    k_ccl_local_stage<<<ccl_grid(w, h, 16, 1), 32 * 16, 0, s>>>(fs);
+    LAUNCHED();
+    k_ccl_border_r16<<<grid2(cdiv(border, 256), 1), 256, 0, s>>>(fs);
+    LAUNCHED();
+    k_ccl_final<<<final_grid(w, h, 1), CCL_FINAL_THREADS, 0, s>>>(fs);
     LAUNCHED();
     return ATAG_OK;
 }
@@ -478,7 +469,7 @@ atag_status atag_image_segmentation(const uint8_t* thr, uint32_t* scratch, uint3
     d.width = (uint32_t)w; d.height = (uint32_t)h; d.factor = 1;
     d.thr = const_cast<uint8_t*>(thr); d.scratch = scratch; d.labels = labels; d.sizes = sizes;
     d.stage_outputs = 1;
-    return launch_segmentation(single(d), w, h, 1, (cudaStream_t)stream);
+    return launch_segmentation(single(d), w, h, (cudaStream_t)stream);
 }
 
 atag_status atag_find_boundaries(const uint32_t* labels, const uint32_t* sizes, atag_boundary_point* points,

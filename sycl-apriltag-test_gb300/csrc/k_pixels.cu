@@ -133,6 +133,13 @@ __global__ void __launch_bounds__(256, 8) k_threshold(const __grid_constant__ Fr
 // root (global index) and each tile root holds its tile-local pixel count;
 // (2) links that cross tile borders are merged in global memory;
 // (3) final labels, and tile counts folded into the component root.
+//
+// The tile pass is bound by instruction issue (~0.83 per scheduler and clock,
+// 95% occupancy).  A warp takes a block row; with links computed per lane on
+// byte masks, one walk after the other and full edge records it executed 696
+// instructions per row (64 frames of 1080p 703 us); links as words for the
+// whole row, walks of both forests in lock step and edge bits only where they
+// are read make it 670 (676 us).  About 170 of them are the unions.
 // ---------------------------------------------------------------------------
 constexpr int CCL_BX = 32;  // blocks per tile row; CCL_BY (8, 16 or 32) rows is a tuning choice
 
@@ -230,11 +237,37 @@ __device__ __forceinline__ bool uf_union(Ptr par, uint32_t a, uint32_t b, uint32
     return false;
 }
 
+// The same within a tile's shared-memory forest: both walks in lock step, so
+// their loads overlap and the warp runs the longer walk once, and no halving
+// (a run's slots point at its head, which keeps chains short).
+__device__ __forceinline__ void tile_union(volatile uint32_t* par, uint32_t a, uint32_t b, uint32_t cap) {
+    for (uint32_t it = 0; it < cap; it++) {
+        const uint32_t pa = par[a], pb = par[b];
+        if (pa != a || pb != b) {
+            a = pa;
+            b = pb;
+            continue;
+        }
+        if (a == b) return;
+        const uint32_t hi = max(a, b), lo = min(a, b);
+        const uint32_t old = atomicMin((uint32_t*)&par[hi], lo);
+        if (old == hi) return;
+        a = lo;
+        b = old;
+    }
+}
+
 __device__ __forceinline__ uint32_t ccl_tiles_x(uint32_t w) { return (w / 2 + CCL_BX - 1) / CCL_BX; }
 template <int CCL_BY>
 __device__ __forceinline__ uint32_t ccl_tiles_y(uint32_t h) { return (h / 2 + CCL_BY - 1) / CCL_BY; }
 
-template <int CCL_BY>
+// The pixels of a 64-pixel row segment as bit words, bit i = block i of the
+// tile row: 255 (w) and 0 (k) at even (e) and odd (o) columns.
+struct RowBits {
+    uint32_t we, wo, ke, ko;
+};
+
+template <int CCL_BY, bool EXACT>
 __device__ __forceinline__ void ccl_local_impl(const FrameSet& fs) {
     constexpr int CCL_THREADS = CCL_BX * CCL_BY;
     constexpr unsigned FULL = 0xFFFFFFFFu;
@@ -248,86 +281,76 @@ __device__ __forceinline__ void ccl_local_impl(const FrameSet& fs) {
     const int x0 = bx0 * 2, y0 = by0 * 2;
     const uint32_t tile = blockIdx.y * (uint32_t)ntx + blockIdx.x;  // row-major within the frame
 
-    // words of pixels x0 - 4 .. x0 + 2 CCL_BX + 3 of a row (x0 and w are
-    // multiples of 4): pixel x is byte x - x0 + 4
-    constexpr int WPR = (2 * CCL_BX + 8) / 4;
-    static_assert(WPR <= 32, "one word per lane");
-    __shared__ uint32_t par[2 * CCL_THREADS];
-    __shared__ uint32_t cnt[2 * CCL_THREADS];
-    __shared__ uint32_t row_runs[CCL_BY][2];  // S-link ballots of each tile row (255, 0 forest)
+    __shared__ __align__(8) uint32_t par[2 * CCL_THREADS];
+    __shared__ __align__(8) uint32_t cnt[2 * CCL_THREADS];
+    __shared__ uint32_t row_runs[CCL_BY][2];  // S-link words of each tile row (255, 0 forest)
     __shared__ uint32_t ulist[CCL_BY][192];   // per row: unions with the row above (slot << 16 | slot)
-    __shared__ uint8_t s_links[CCL_THREADS];  // the blocks' links (edge records)
 
     const int tx = threadIdx.x % CCL_BX, ty = threadIdx.x / CCL_BX;  // lane, warp
-    // the warp's pixel rows y - 1, y, y + 1 (y = y0 + 2 ty) with a one-pixel
-    // halo as aligned 32-bit words, one per lane (WPR lanes), that the lanes
-    // share by shuffles: no shared-memory staging and no barrier before the
-    // links (the rows between two warps are read by both, from L1)
-    const int o = 2 * tx + 3, wq = o >> 2, sh = (o & 3) * 8;
-    uint32_t vm, v0, v1;
-    {
-        const uint32_t* thr32 = reinterpret_cast<const uint32_t*>(F.thr);
-        const int xw = x0 - 4 + 4 * tx;
-        const bool colok = tx < WPR && xw >= 0 && xw < w;
-        uint32_t v[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const int y = y0 - 1 + 2 * ty + k;
-            v[k] = (colok && y >= 0 && y < h) ? __ldg(thr32 + (size_t)y * (uint32_t)(w >> 2) + (xw >> 2)) : 0x7F7F7F7Fu;
-        }
-        // pixels x - 1 .. x + 2 of a row as one word (x = 2 bx)
-        auto win = [&](uint32_t r) { return __funnelshift_r(__shfl_sync(FULL, r, wq), __shfl_sync(FULL, r, wq + 1), sh); };
-        vm = win(v[0]);
-        v0 = win(v[1]);
-        v1 = win(v[2]);
-    }
     const int bx = bx0 + tx, by = by0 + ty;
     const bool live = bx < w / 2 && by < h / 2;
-    const uint32_t l = threadIdx.x;
-    cnt[2 * l] = 0;
-    cnt[2 * l + 1] = 0;
-
-    // The block's links, computed on bytes: p(x - 1) .. p(x + 2) of pixel
-    // rows y - 1, y and y + 1 (x = 2 bx, y = 2 by) as one word each, and
-    // per byte "is 255" / "is 0" masks.  The neighbour test pixels and
-    // block_links' check masks become: P (up-left) tests p(x-1, y-1) when
-    // TL is valid, Q (up) p(x, y-1) or p(x+1, y-1) when TL or TR is, R
-    // (up-right) p(x+2, y-1) when TR is, S (left) p(x-1, y) or p(x-1, y+1)
-    // when TL or BL is; image edges drop P and S (x = 0), R (x + 2 >= w)
-    // and P, Q, R (y = 0).
-    const uint32_t Wm = __vcmpeq4(vm, FULL), Km = __vcmpeq4(vm, 0u);
-    const uint32_t W0 = __vcmpeq4(v0, FULL), K0 = __vcmpeq4(v0, 0u);
-    const uint32_t W1 = __vcmpeq4(v1, FULL), K1 = __vcmpeq4(v1, 0u);
-    const uint32_t V0 = W0 | K0, V1 = W1 | K1;
-    const bool tl = V0 & 0xFF00u, tr = V0 & 0xFF0000u, bl = V1 & 0xFF00u;
-    const bool gx = bx > 0, gy = by > 0, gr = 2 * bx + 2 < w;
-    const bool cP = live && tl && gx && gy, cQ = live && (tl || tr) && gy, cR = live && tr && gr && gy;
-    const bool cS = live && (tl || bl) && gx;
-    // bit 0 P, 1 Q, 2 R, 3 S
-    auto links = [&](uint32_t M, uint32_t X0, uint32_t X1) {
-        return (cP && (M & 0xFFu) ? 1u : 0u) | (cQ && (M & 0xFFFF00u) ? 2u : 0u) | (cR && (M & 0xFF000000u) ? 4u : 0u) |
-               (cS && ((X0 | X1) & 0xFFu) ? 8u : 0u);
+    const uint32_t l = threadIdx.x, lane = (uint32_t)tx;
+    *reinterpret_cast<uint2*>(cnt + 2 * l) = make_uint2(0u, 0u);
+    // The warp's pixel rows y - 1, y, y + 1 (y = y0 + 2 ty): lane i loads the
+    // two pixels of block i, and ballots of "is 255" and "is 0" make the rows'
+    // bit words (the rows between two warps are read by both, from L1).
+    // Lanes 0 .. 3 also load the pixels left of the tile row and the one right
+    // of row y - 1.  Pixels outside the image read 127.  The detector's own
+    // thresholded pixels are 0, 127 or 255, told apart by one bit; a caller's
+    // image is compared in full.
+    RowBits row[3];
+    unsigned hw_, hk_;  // halo pixels that are 255, 0: bits 0-2 left of rows y - 1, y, y + 1, bit 3 right of y - 1
+    {
+        const int y = y0 + 2 * ty;
+        const uint8_t* base = F.thr + (ptrdiff_t)y * w + x0;
+        uint32_t v[3], hv = 127u;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const bool in = bx < w / 2 && y - 1 + k >= 0 && y - 1 + k < h;
+            v[k] = in ? (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(base + (k - 1) * w) + tx) : 0x7F7Fu;
+        }
+        const int hx = tx == 3 ? 2 * CCL_BX : -1, hy = tx == 3 ? -1 : tx - 1;
+        if (tx < 4 && x0 + hx >= 0 && x0 + hx < w && y + hy >= 0 && y + hy < h) hv = __ldg(base + hy * w + hx);
+        auto white = [](uint32_t p, int sh) { return EXACT ? ((p >> sh) & 255u) == 255u : (p & (0x80u << sh)) != 0u; };
+        auto black = [](uint32_t p, int sh) { return EXACT ? ((p >> sh) & 255u) == 0u : (p & (1u << sh)) == 0u; };
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            row[k].we = __ballot_sync(FULL, white(v[k], 0));
+            row[k].wo = __ballot_sync(FULL, white(v[k], 8));
+            row[k].ke = __ballot_sync(FULL, black(v[k], 0));
+            row[k].ko = __ballot_sync(FULL, black(v[k], 8));
+        }
+        hw_ = __ballot_sync(FULL, white(hv, 0));
+        hk_ = __ballot_sync(FULL, black(hv, 0));
+    }
+    // The links of all 32 blocks of the row at once, in words: with TL, TR and
+    // BL the blocks' valid (0 or 255) pixels, P (up-left) needs TL and p(x-1,
+    // y-1), Q (up) TL or TR and p(x, y-1) or p(x+1, y-1), R (up-right) TR and
+    // p(x+2, y-1), S (left) TL or BL and p(x-1, y) or p(x-1, y+1)
+    // (block_links' check masks; image edges read 127, which links nothing).
+    const uint32_t TL = row[1].we | row[1].ke, TR = row[1].wo | row[1].ko, BL = row[2].we | row[2].ke;
+    auto up_left = [&](uint32_t o0, unsigned hb) { return TL & ((o0 << 1) | (hb & 1u)); };
+    auto up = [&](uint32_t e0, uint32_t o0) { return (TL | TR) & (e0 | o0); };
+    auto up_right = [&](uint32_t e0, unsigned hb) { return TR & ((e0 >> 1) | ((hb & 8u) << 28)); };
+    auto left = [&](uint32_t o1, uint32_t o2, unsigned hb) {
+        return (TL | BL) & (((o1 | o2) << 1) | (((hb >> 1) | (hb >> 2)) & 1u));
     };
-    const uint32_t lw = links(Wm, W0, W1), lb = links(Km, K0, K1);
-    s_links[threadIdx.x] = (uint8_t)(lw | (lb << 4));
-    // the block's 255 and 0 pixel counts
-    const uint32_t cw = live ? (uint32_t)(__popc(W0 & 0x00FFFF00u) + __popc(W1 & 0x00FFFF00u)) >> 3 : 0u;
-    const uint32_t cb = live ? (uint32_t)(__popc(K0 & 0x00FFFF00u) + __popc(K1 & 0x00FFFF00u)) >> 3 : 0u;
+    const uint32_t Pw = up_left(row[0].wo, hw_), Pk = up_left(row[0].ko, hk_);
+    const uint32_t Qw = up(row[0].we, row[0].wo), Qk = up(row[0].ke, row[0].ko);
+    const uint32_t Rw = up_right(row[0].we, hw_), Rk = up_right(row[0].ke, hk_);
+    const uint32_t Sw = left(row[1].wo, row[2].wo, hw_), Sk = left(row[1].ko, row[2].ko, hk_);
 
     // S links (left neighbour) inside the tile row, which is this warp: a run
     // of blocks that each link to their left neighbour points at its first
     // block, a smaller slot, so the root of a set stays its minimum
-    const uint32_t lane = (uint32_t)tx;
-    const unsigned sw = __ballot_sync(FULL, tx > 0 && (lw & 8u));
-    const unsigned sb = __ballot_sync(FULL, tx > 0 && (lb & 8u));
+    const unsigned sw = Sw & ~1u, sb = Sk & ~1u;
     const unsigned le = (2u << lane) - 1u;  // lanes 0 .. lane (2 << 31 wraps to 0)
     const uint32_t hw = 31 - __clz(~sw & le), hb = 31 - __clz(~sb & le);  // run heads (lanes)
     const unsigned mw = le & ~((1u << hw) - 1u), mb = le & ~((1u << hb) - 1u);  // the run up to this lane
     const uint32_t row0 = (uint32_t)ty * CCL_BX;
     const bool last_w = lane == 31 || !((sw >> (lane + 1)) & 1u);  // last block of its run
     const bool last_b = lane == 31 || !((sb >> (lane + 1)) & 1u);
-    par[2 * l] = 2 * (row0 + hw);
-    par[2 * l + 1] = 2 * (row0 + hb) + 1;
+    *reinterpret_cast<uint2*>(par + 2 * l) = make_uint2(2 * (row0 + hw), 2 * (row0 + hb) + 1);
     if (lane == 0) {
         row_runs[ty][0] = sw;
         row_runs[ty][1] = sb;
@@ -340,12 +363,9 @@ __device__ __forceinline__ void ccl_local_impl(const FrameSet& fs) {
     // to, keeps the first linked block of each above run and makes those
     // unions.
     if (ty > 0) {
-        const unsigned PW = __ballot_sync(FULL, tx > 0 && (lw & 1u)), QW = __ballot_sync(FULL, lw & 2u);
-        const unsigned RW = __ballot_sync(FULL, tx < CCL_BX - 1 && (lw & 4u));
-        const unsigned PB = __ballot_sync(FULL, tx > 0 && (lb & 1u)), QB = __ballot_sync(FULL, lb & 2u);
-        const unsigned RB = __ballot_sync(FULL, tx < CCL_BX - 1 && (lb & 4u));
-        const uint32_t aw = ((PW & mw) >> 1) | (QW & mw) | ((RW & mw) << 1);
-        const uint32_t ab = ((PB & mb) >> 1) | (QB & mb) | ((RB & mb) << 1);
+        // the bits that leave the tile (P of block 0, R of block 31) shift out
+        const uint32_t aw = ((Pw & mw) >> 1) | (Qw & mw) | ((Rw & mw) << 1);
+        const uint32_t ab = ((Pk & mb) >> 1) | (Qk & mb) | ((Rk & mb) << 1);
         const uint32_t up0 = row0 - CCL_BX;
         uint32_t ew = last_w ? (aw & ~((aw << 1) & row_runs[ty - 1][0])) : 0u;
         uint32_t eb = last_b ? (ab & ~((ab << 1) & row_runs[ty - 1][1])) : 0u;
@@ -366,25 +386,28 @@ __device__ __forceinline__ void ccl_local_impl(const FrameSet& fs) {
         const uint32_t total = __shfl_sync(FULL, incl, 31);
         for (uint32_t k = lane; k < total; k += 32) {
             const uint32_t e = ulist[ty][k];
-            uf_union((volatile uint32_t*)par, e >> 16, e & 0xFFFFu, 2u * CCL_THREADS);
+            tile_union((volatile uint32_t*)par, e >> 16, e & 0xFFFFu, 8u * CCL_THREADS);
         }
     }
     __syncthreads();
-    // roots: a run's head finds it, its other blocks take it from the head
-    bool local_capped = false;  // cannot happen: a tile chain visits at most its 2 CCL_THREADS slots
-    uint32_t rw = lane == hw ? find_root_volatile((volatile uint32_t*)par, 2 * l, 2u * CCL_THREADS, &local_capped) : 0u;
-    uint32_t rb = lane == hb ? find_root_volatile((volatile uint32_t*)par, 2 * l + 1, 2u * CCL_THREADS, &local_capped) : 0u;
-    rw = __shfl_sync(FULL, rw, hw);
-    rb = __shfl_sync(FULL, rb, hb);
-    // pixel counts per root: the run's last lane adds the run's count, the
-    // sum over the run's lanes of the ballots of each count bit
-    {
-        const unsigned w1 = __ballot_sync(FULL, cw & 1u), w2 = __ballot_sync(FULL, cw & 2u), w4 = __ballot_sync(FULL, cw & 4u);
-        const unsigned b1 = __ballot_sync(FULL, cb & 1u), b2 = __ballot_sync(FULL, cb & 2u), b4 = __ballot_sync(FULL, cb & 4u);
-        const uint32_t sw_ = (uint32_t)(__popc(w1 & mw) + 2 * __popc(w2 & mw) + 4 * __popc(w4 & mw));
-        const uint32_t sb_ = (uint32_t)(__popc(b1 & mb) + 2 * __popc(b2 & mb) + 4 * __popc(b4 & mb));
-        if (last_w && sw_) atomicAdd(&cnt[rw], sw_);
-        if (last_b && sb_) atomicAdd(&cnt[rb], sb_);
+    // roots of both of the block's slots, from its runs' heads (the lanes of a
+    // run read the same words); a chain visits each slot at most once
+    uint32_t rw = 2 * (row0 + hw), rb = 2 * (row0 + hb) + 1;
+    for (uint32_t it = 0; it < 2u * CCL_THREADS; it++) {
+        const uint32_t pw = par[rw], pb = par[rb];
+        if (pw == rw && pb == rb) break;
+        rw = pw;
+        rb = pb;
+    }
+    // pixel counts per root: the run's last lane adds the run's count, its
+    // bits in the words of rows y and y + 1
+    if (last_w) {
+        const uint32_t c = (uint32_t)(__popc(row[1].we & mw) + __popc(row[1].wo & mw) + __popc(row[2].we & mw) + __popc(row[2].wo & mw));
+        if (c) atomicAdd(&cnt[rw], c);
+    }
+    if (last_b) {
+        const uint32_t c = (uint32_t)(__popc(row[1].ke & mb) + __popc(row[1].ko & mb) + __popc(row[2].ke & mb) + __popc(row[2].ko & mb));
+        if (c) atomicAdd(&cnt[rb], c);
     }
     __syncthreads();
     // tile slot s = 2 (row CCL_BX + col) + forest -> frame slot: the tile's
@@ -398,26 +421,34 @@ __device__ __forceinline__ void ccl_local_impl(const FrameSet& fs) {
         // links of that forest in bits 24-27 (slots are below 2^24); links
         // that leave the tile are the border pass's work
         uint2* rec = reinterpret_cast<uint2*>(F.edges + (size_t)tile * ccl_edge_words(CCL_BY));
-        const uint32_t lk = s_links[threadIdx.x];
-        const uint2 e = make_uint2(parents.x | ((lk & 15u) << 24), parents.y | ((lk >> 4) << 24));
-        if (ty == 0) rec[tx] = e;
-        if (ty == CCL_BY - 1) rec[32 + tx] = e;
-        if (tx == 0) rec[64 + ty] = e;
-        if (tx == CCL_BX - 1) rec[64 + CCL_BY + ty] = e;
+        if (ty == 0 || ty == CCL_BY - 1) {
+            auto bits = [&](uint32_t P, uint32_t Q, uint32_t R, uint32_t S) {
+                return (((P >> lane) & 1u) | (((Q >> lane) & 1u) << 1) | (((R >> lane) & 1u) << 2) | (((S >> lane) & 1u) << 3)) << 24;
+            };
+            rec[(ty ? 32 : 0) + tx] = make_uint2(parents.x | bits(Pw, Qw, Rw, Sw), parents.y | bits(Pk, Qk, Rk, Sk));
+        }
+        if (lane == 0 || lane == 31) {  // P and S leave to the left, R to the right
+            const uint32_t ew = lane ? (Rw >> 31) << 26 : ((Pw & 1u) << 24) | ((Sw & 1u) << 27);
+            const uint32_t ek = lane ? (Rk >> 31) << 26 : ((Pk & 1u) << 24) | ((Sk & 1u) << 27);
+            rec[64 + (lane ? CCL_BY : 0) + ty] = make_uint2(parents.x | ew, parents.y | ek);
+        }
     }
     if (live) {
-        size_t id = (size_t)(by * 2) * w + bx * 2;
+        const uint32_t id = tslot0 + (uint32_t)ty * 2u * (uint32_t)w + 2u * lane;
         *reinterpret_cast<uint2*>(F.scratch + id) = parents;
-        uint2 sz = make_uint2(rw == 2 * l ? cnt[2 * l] : 0u, rb == 2 * l + 1 ? cnt[2 * l + 1] : 0u);
+        const uint2 c = *reinterpret_cast<const uint2*>(cnt + 2 * l);
+        const uint2 sz = make_uint2(rw == 2 * l ? c.x : 0u, rb == 2 * l + 1 ? c.y : 0u);
         *reinterpret_cast<uint2*>(F.sizes + id) = sz;
         if (F.stage_outputs) {
             *reinterpret_cast<uint2*>(F.sizes + id + w) = make_uint2(0u, 0u);
             // the reference keeps the block's information word at scratch[id + w]:
             // bits 0-3 the pixels (TL, TR, BL, BR) that are 255, bits 8-11 those that are 0
-            auto bits = [](uint32_t X0, uint32_t X1) {
-                return ((X0 >> 8) & 1u) | ((X0 >> 15) & 2u) | ((X1 >> 6) & 4u) | ((X1 >> 13) & 8u);
+            auto bits = [&](uint32_t tl, uint32_t tr, uint32_t bl, uint32_t br) {
+                return ((tl >> lane) & 1u) | (((tr >> lane) & 1u) << 1) | (((bl >> lane) & 1u) << 2) | (((br >> lane) & 1u) << 3);
             };
-            *reinterpret_cast<uint2*>(F.scratch + id + w) = make_uint2(bits(W0, W1) | (bits(K0, K1) << 8), 0u);
+            *reinterpret_cast<uint2*>(F.scratch + id + w) =
+                make_uint2(bits(row[1].we, row[1].wo, row[2].we, row[2].wo) |
+                               (bits(row[1].ke, row[1].ko, row[2].ke, row[2].ko) << 8), 0u);
         }
     }
 }
@@ -716,12 +747,11 @@ __global__ void __launch_bounds__(256) k_boundaries_dense(const __grid_constant_
     }
 }
 
-__global__ void __launch_bounds__(CCL_BX * 8, 8) k_ccl_local_r8(const __grid_constant__ FrameSet fs) { ccl_local_impl<8>(fs); }
-__global__ void __launch_bounds__(CCL_BX * 16, 4) k_ccl_local_r16(const __grid_constant__ FrameSet fs) { ccl_local_impl<16>(fs); }
-__global__ void __launch_bounds__(CCL_BX * 32, 2) k_ccl_local_r32(const __grid_constant__ FrameSet fs) { ccl_local_impl<32>(fs); }
-__global__ void __launch_bounds__(256) k_ccl_border_r8(const __grid_constant__ FrameSet fs) { ccl_border_impl<8>(fs); }
+__global__ void __launch_bounds__(CCL_BX * 8, 8) k_ccl_local_r8(const __grid_constant__ FrameSet fs) { ccl_local_impl<8, false>(fs); }
+__global__ void __launch_bounds__(CCL_BX * 16, 4) k_ccl_local_r16(const __grid_constant__ FrameSet fs) { ccl_local_impl<16, false>(fs); }
+__global__ void __launch_bounds__(CCL_BX * 32, 2) k_ccl_local_r32(const __grid_constant__ FrameSet fs) { ccl_local_impl<32, false>(fs); }
+__global__ void __launch_bounds__(CCL_BX * 16, 4) k_ccl_local_stage(const __grid_constant__ FrameSet fs) { ccl_local_impl<16, true>(fs); }
 __global__ void __launch_bounds__(256) k_ccl_border_r16(const __grid_constant__ FrameSet fs) { ccl_border_impl<16>(fs); }
-__global__ void __launch_bounds__(256) k_ccl_border_r32(const __grid_constant__ FrameSet fs) { ccl_border_impl<32>(fs); }
 __global__ void __launch_bounds__(256) k_ccl_border_edges_r8(const __grid_constant__ FrameSet fs) { ccl_border_edges_impl<8>(fs); }
 __global__ void __launch_bounds__(256) k_ccl_border_edges_r16(const __grid_constant__ FrameSet fs) { ccl_border_edges_impl<16>(fs); }
 __global__ void __launch_bounds__(256) k_ccl_border_edges_r32(const __grid_constant__ FrameSet fs) { ccl_border_edges_impl<32>(fs); }
