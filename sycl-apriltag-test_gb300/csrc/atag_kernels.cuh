@@ -66,8 +66,9 @@ struct FrameDesc {
     uint32_t quad_cap;
     atag_frame_stats* stats;
     uint32_t* counters;                // per-frame work counters (see Counter)
-    // DEAD_PAIRS keys (EMPTY = ~0) of pairs whose running point count is
-    // already above the cluster size limit; null when not tracked
+    // DEAD_PAIRS label word pairs (white << 32 | black, EMPTY = ~0) of pairs
+    // whose running point count is already above the cluster size limit; null
+    // when not tracked
     unsigned long long* dead_pairs;
     // iteration cap of the frame-wide union-find loops (0: the bound the
     // tile count gives, see k_pixels.cu)

@@ -56,13 +56,16 @@ constexpr int BP_SW = BP_W + 8;  // label row: x0 - 4 .. x0 + BP_W + 3 (16-byte 
 constexpr int BP_LC = 64;                      // CTA hash-table entries (a tile has a few dozen pairs; more go straight to the frame's table)
 constexpr uint32_t BP_VALUE = 0x3FFFFFFFu;  // label value without the colour bit
 
-struct PairTableSmem {
+// The CTA's pair table.  Fields that start at all ones come first, then the
+// zeroed ones: both halves are filled with 16-byte stores.
+struct __align__(16) PairTableSmem {
     unsigned long long key[BP_LC];
-    uint32_t cnt[BP_LC], xmin[BP_LC], xmax[BP_LC], ymin[BP_LC], ymax[BP_LC];
-    int gx[BP_LC], gy[BP_LC];
+    uint32_t xmin[BP_LC], ymin[BP_LC], gslot[BP_LC];
+    uint32_t cnt[BP_LC], xmax[BP_LC], ymax[BP_LC];
+    int gx[BP_LC];
     int pxgx[BP_LC];  // a tile's sum fits 32 bits: at most 4096 points, |x| < 2^13
-    uint32_t gslot[BP_LC];
 };
+constexpr int BP_TABLE_ONES = BP_LC * (8 + 3 * 4) / 16, BP_TABLE_QUADS = sizeof(PairTableSmem) / 16;
 
 // Insert-or-find in the CTA's pair table; a plain read first avoids the
 // atomic for keys that are already present (the common case).  *fresh is
@@ -96,9 +99,28 @@ __device__ __forceinline__ uint32_t stage_packed(uint32_t e, uint32_t x0, uint32
     const uint32_t xy = (x0 | (y0 << 16)) + (e & 63) + (((e >> 6) & 15) << 16);
     return xy | (((e >> 10) & 3) << 14) | (((e >> 12) & 1) << 31);
 }
+// The two label words of a pair: it joins a white label (colour bit | an even
+// root slot) and a black one (an odd root slot, or label 0 of pixels that are
+// neither 0 nor 255).  White in the high word.
+__device__ __forceinline__ unsigned long long pair_labels(unsigned long long key) {
+    const uint32_t kA = (uint32_t)(key >> 32), kB = (uint32_t)key;
+    if ((kA ^ kB) & 1u) {
+        const uint32_t white = (kA & 1u) ? kB : kA, black = (kA & 1u) ? kA : kB;
+        return (unsigned long long)(LABEL_PIXEL_MASK | white) << 32 | black;
+    }
+    return kA == 0u ? (unsigned long long)(LABEL_PIXEL_MASK | kB) << 32 : EMPTY_KEY;
+}
 
 // find_boundaries (find_boundaries.cpp:10-155) fused with the per-pair
 // ClusterBounds reduction (main.cpp:571-585) and the compaction of points.
+//
+// Bound by instruction issue (~0.8 per scheduler and clock at 90% occupancy),
+// a third of it the tile load, and before this form half of it the rounds
+// over staged points: match_any per round and seven reductions over every
+// key's lanes were ~480 instructions per 32 points.  A strip's points belong
+// to 1.4 pairs on average, so a warp keeps one pair's sums in registers across
+// its rounds and reduces them when the pair changes.  64 frames of 1080p 926
+// -> 877 us.
 template <int BP_H>
 __device__ __forceinline__ void boundaries_pairs_impl(const FrameSet& fs, uint32_t min_size) {
     constexpr int BP_SH = BP_H + 1;
@@ -116,52 +138,34 @@ __device__ __forceinline__ void boundaries_pairs_impl(const FrameSet& fs, uint32
     const int ntx = (w + BP_W - 1) / BP_W, nty = (h + BP_H - 1) / BP_H;
     if ((int)blockIdx.y >= ntx || (int)blockIdx.z >= nty) return;
     const int x0 = blockIdx.y * BP_W, y0 = blockIdx.z * BP_H;
-    uint32_t* status = F.counters + CNT_STATUS;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
     // labels of the tile and its halo (column c = pixel x0 + c - 4: 3 = x0 -
     // 1, BP_W + 4 = x0 + BP_W; row BP_H is the row below the tile), and four
     // bit planes of them: per row four words, [0] bit 31 = x0 - 1, [1] and
-    // [2] = x0 .. x0 + 63, [3] bit 0 = x0 + 64.  Plane 0: the colour bit
-    // (255 pixel), 1: the component has at least min_size pixels, 2 and 3:
+    // [2] = x0 .. x0 + 63, [3] bit 0 = x0 + 64.  Plane x: the colour bit
+    // (255 pixel), y: the component has at least min_size pixels, z and w:
     // the label is one of the two labels of the frame's first / second pair
     // known to be over the cluster size limit.
     __shared__ __align__(16) uint32_t lab[BP_SH][BP_SW];
-    __shared__ __align__(16) uint32_t planes[4][BP_SH][4];
+    __shared__ uint4 planes[BP_SH][4];
     __shared__ PairTableSmem T;
     __shared__ uint32_t stage[BP_STAGE];
     __shared__ uint32_t s_nall;
     const bool track_dead = !F.stage_outputs && F.dead_pairs;
 
-    // pairs that earlier tiles already pushed over the cluster size limit
-    // (snapshots: a pair published later is simply processed in full;
-    // points of a published pair can never survive, so steps and warps that
-    // see different snapshots still agree on the result).  Both filter
-    // points at emission.
+    // label words of the pairs that earlier tiles already pushed over the
+    // cluster size limit (snapshots: a pair published later is simply
+    // processed in full; points of a published pair can never survive).  Both
+    // filter points at emission; all ones, for none, equals no label.
     static_assert(DEAD_PAIRS == 2, "two over-limit pair planes");
-    // a pair joins a white label (colour bit | an even root slot) and a
-    // black one (an odd root slot, or label 0 of pixels that are neither 0
-    // nor 255): its two label words
-    auto pair_labels = [&](unsigned long long key, uint32_t& lw, uint32_t& lk) {
-        lw = FULL;
-        lk = FULL;
-        const uint32_t kA = (uint32_t)(key >> 32), kB = (uint32_t)key;
-        if ((kA ^ kB) & 1u) {
-            lw = LABEL_PIXEL_MASK | ((kA & 1u) ? kB : kA);
-            lk = (kA & 1u) ? kA : kB;
-        } else if (kA == 0u) {
-            lw = LABEL_PIXEL_MASK | kB;
-            lk = 0u;
-        }
-    };
-    uint32_t dW, dK, eW, eK;
-    pair_labels(track_dead ? __ldcg(F.dead_pairs) : EMPTY_KEY, dW, dK);
-    pair_labels(track_dead ? __ldcg(F.dead_pairs + 1) : EMPTY_KEY, eW, eK);
+    const unsigned long long dead0 = track_dead ? __ldcg(F.dead_pairs) : EMPTY_KEY;
+    const unsigned long long dead1 = track_dead ? __ldcg(F.dead_pairs + 1) : EMPTY_KEY;
+    const uint32_t dW = (uint32_t)(dead0 >> 32), dK = (uint32_t)dead0, eW = (uint32_t)(dead1 >> 32), eK = (uint32_t)dead1;
     if (threadIdx.x == 0) s_nall = 0;
-    for (int i = threadIdx.x; i < BP_LC; i += blockDim.x) {
-        T.key[i] = EMPTY_KEY;
-        T.cnt[i] = 0; T.xmin[i] = 0xFFFFFFFFu; T.xmax[i] = 0; T.ymin[i] = 0xFFFFFFFFu; T.ymax[i] = 0;
-        T.gx[i] = 0; T.gy[i] = 0; T.pxgx[i] = 0; T.gslot[i] = INVALID;
+    for (int i = threadIdx.x; i < BP_TABLE_QUADS; i += blockDim.x) {
+        const uint32_t v = i < BP_TABLE_ONES ? FULL : 0u;
+        reinterpret_cast<uint4*>(&T)[i] = make_uint4(v, v, v, v);
     }
     // Loads.  Row-word unit u = 2 r + k (row r of the tile and its halo row,
     // 32-pixel word k) belongs to warp u % NW: lane i loads the label of
@@ -180,6 +184,7 @@ __device__ __forceinline__ void boundaries_pairs_impl(const FrameSet& fs, uint32
         const int kk = warp & 1, r0 = warp >> 1;
         const bool xin = x0 + 32 * kk + lane < w;
         const uint32_t* lrow = F.labels + (size_t)(y0 + r0) * w + (x0 + 32 * kk + lane);
+        const uint32_t* sizes = F.sizes;
         uint32_t lv[PER], sz[PER];
 #pragma unroll
         for (int j = 0; j < PER; j++) {
@@ -187,36 +192,34 @@ __device__ __forceinline__ void boundaries_pairs_impl(const FrameSet& fs, uint32
             lv[j] = in ? __ldg(lrow + (size_t)j * (NW / 2) * w) : 0u;
         }
         const bool halo = warp >= NW - 2, right = warp == NW - 1;
-        const int hx = right ? x0 + BP_W : x0 - 1, hy = y0 + lane;
-        const uint32_t hl = (halo && lane < BP_SH && hx >= 0 && hx < w && hy < h) ? __ldg(F.labels + (size_t)hy * w + hx) : 0u;
+        uint32_t hl = 0u, hs = 0u;
+        if (halo) {
+            const int hx = right ? x0 + BP_W : x0 - 1, hy = y0 + lane;
+            if (lane < BP_SH && hx >= 0 && hx < w && hy < h) hl = __ldg(F.labels + (size_t)hy * w + hx);
+        }
 #pragma unroll
         for (int j = 0; j < PER; j++)
-            if (warp + NW * j < NUNIT) sz[j] = __ldg(F.sizes + (lv[j] & LABEL_VALUE_MASK));
-        const uint32_t hs = halo ? __ldg(F.sizes + (hl & LABEL_VALUE_MASK)) : 0u;
+            if (warp + NW * j < NUNIT) sz[j] = __ldg(sizes + (lv[j] & LABEL_VALUE_MASK));
+        if (halo) hs = __ldg(sizes + (hl & LABEL_VALUE_MASK));
 #pragma unroll
         for (int j = 0; j < PER; j++) {
-            const int r = r0 + (NW / 2) * j, k = kk;
+            const int r = r0 + (NW / 2) * j;
             if (warp + NW * j >= NUNIT) break;
             const uint32_t l = lv[j];
-            lab[r][4 + 32 * k + lane] = l;
-            const unsigned bc = __ballot_sync(FULL, (int)l < 0);
-            const unsigned bb = __ballot_sync(FULL, sz[j] >= min_size);
-            const unsigned bd = __ballot_sync(FULL, l == dW || l == dK);
-            const unsigned be = __ballot_sync(FULL, l == eW || l == eK);
-            if (lane == 0) {
-                planes[0][r][1 + k] = bc;
-                planes[1][r][1 + k] = bb;
-                planes[2][r][1 + k] = bd;
-                planes[3][r][1 + k] = be;
-            }
+            lab[r][4 + 32 * kk + lane] = l;
+            uint4 pl;
+            pl.x = __ballot_sync(FULL, (int)l < 0);
+            pl.y = __ballot_sync(FULL, sz[j] >= min_size);
+            pl.z = __ballot_sync(FULL, l == dW || l == dK);
+            pl.w = __ballot_sync(FULL, l == eW || l == eK);
+            if (lane == 0) planes[r][1 + kk] = pl;
         }
         if (halo && lane < BP_SH) {
             lab[lane][right ? BP_W + 4 : 3] = hl;
-            const int wq = right ? 3 : 0, sh = right ? 0 : 31;
-            planes[0][lane][wq] = (hl >> 31) << sh;
-            planes[1][lane][wq] = (hs >= min_size ? 1u : 0u) << sh;
-            planes[2][lane][wq] = (hl == dW || hl == dK ? 1u : 0u) << sh;
-            planes[3][lane][wq] = (hl == eW || hl == eK ? 1u : 0u) << sh;
+            const int sh = right ? 0 : 31;
+            planes[lane][right ? 3 : 0] =
+                make_uint4((hl >> 31) << sh, (hs >= min_size ? 1u : 0u) << sh, (hl == dW || hl == dK ? 1u : 0u) << sh,
+                           (hl == eW || hl == eK ? 1u : 0u) << sh);
         }
     }
     __syncthreads();
@@ -227,132 +230,145 @@ __device__ __forceinline__ void boundaries_pairs_impl(const FrameSet& fs, uint32
     // 2 w + rl and test t: a pixel emits test t when it is in the image and
     // big and the tested neighbour is big and of the other colour (BL also
     // not when it duplicates the left pixel's BR), computed for the word at
-    // once on the bit planes.  Points of the frame's first over-limit pair
-    // are counted but not staged.
-    const int rl = lane >> 4, k = (lane >> 3) & 1, t = (lane >> 1) & 3, half = lane & 1;
-    const int r = 2 * warp + rl;
+    // once on the bit planes.  Points of the over-limit pairs are counted but
+    // not staged.
     uint32_t mt, st;
+    const int k = (lane >> 3) & 1, t = (lane >> 1) & 3, r = 2 * warp + (lane >> 4);
     {
         const int xb = x0 + 32 * k;
         // The lane's tested neighbour: the same row for R (t = 0), the row
         // below for BL, B and BR.  Bit i of its plane word is pixel
         // xb + i + dx (dx = +1 for R and BR, -1 for BL, 0 for B): a funnel
         // shift of words lo, lo + 1 of that plane row.
-        const int nrow = r + (t != 0 ? 1 : 0), lo = t == 1 ? k : k + 1, amt = t == 1 ? 31 : (t == 2 ? 0 : 1);
-        auto nb = [&](int p) { return __funnelshift_r(planes[p][nrow][lo], planes[p][nrow][lo + 1], amt); };
-        auto own = [&](int p) { return planes[p][r][k + 1]; };
-        const uint32_t c0 = own(0), b0 = own(1);
+        const int lo = t == 1 ? k : k + 1, amt = t == 1 ? 31 : (t == 2 ? 0 : 1);
+        const uint4 own = planes[r][k + 1];
+        const uint4* nrow = planes[r + (t != 0 ? 1 : 0)];
+        const uint4 a = nrow[lo], b = nrow[lo + 1];
+        const uint2 lf = *reinterpret_cast<const uint2*>(&planes[r][k]);  // colour and size of the word to the left
         uint32_t live = (y0 + r < h) ? (xb + 32 <= w ? FULL : (xb < w ? ((1u << (w - xb)) - 1u) : 0u)) : 0u;
         if (xb == 0) live &= ~1u;  // column 0 is never processed
-        live &= b0 & (half ? 0xFFFF0000u : 0x0000FFFFu);
+        live &= own.y & ((lane & 1) ? 0xFFFF0000u : 0x0000FFFFu);
         // BL is not emitted where the left pixel's BR covers the same pair
-        uint32_t keep = FULL;
-        if (t == 1) {
-            const uint32_t c0L = __funnelshift_l(planes[0][r][k], c0, 1), b0L = __funnelshift_l(planes[1][r][k], b0, 1);
-            keep = ~((c0L ^ planes[0][r + 1][k + 1]) & b0L & planes[1][r + 1][k + 1]);
-        }
-        mt = (nb(0) ^ c0) & nb(1) & live & keep;
+        // (for BL, word b is the one below the lane's own)
+        if (t == 1) live &= ~((__funnelshift_l(lf.x, own.x, 1) ^ b.x) & __funnelshift_l(lf.y, own.y, 1) & b.y);
+        mt = (__funnelshift_r(a.x, b.x, amt) ^ own.x) & __funnelshift_r(a.y, b.y, amt) & live;
         // points whose two pixels are both labels of one published pair
-        st = mt & ~((own(2) & nb(2)) | (own(3) & nb(3)));
+        st = mt & ~((own.z & __funnelshift_r(a.z, b.z, amt)) | (own.w & __funnelshift_r(a.w, b.w, amt)));
     }
     // Each warp lists its staged points in its own part of the staging
     // array (warp scan) and aggregates them itself, so no CTA barrier
     // separates the masks from the rounds.
     uint32_t* wst = stage + warp * BP_WSTAGE;
-    const uint32_t ns = (uint32_t)__popc(st);
-    uint32_t incl = ns;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(FULL, incl, o);
-        if (lane >= o) incl += v;
-    }
-    const uint32_t nst = __shfl_sync(FULL, incl, 31);
+    uint32_t nst = 0;
     {
-        uint32_t pos = incl - ns;
-        const uint32_t base = stage_entry(0, 32 * k, r, t, 0) - 1u;  // + ffs: pixel 32 k + ffs - 1 (mod 2^32)
-        for (uint32_t mm = st; mm; mm &= mm - 1) wst[pos++] = base + (uint32_t)__ffs(mm);
         const uint32_t nall_w = __reduce_add_sync(FULL, (uint32_t)__popc(mt));
         if (lane == 0 && nall_w) atomicAdd(&s_nall, nall_w);
     }
-    __syncwarp();
-    // the over-limit pairs again, for the rounds (a later snapshot)
-    unsigned long long dead0 = EMPTY_KEY, dead1 = EMPTY_KEY;
-    if (track_dead) {
-        dead0 = __ldcg(F.dead_pairs);
-        dead1 = __ldcg(F.dead_pairs + 1);
-    }
-    // The warp takes its staged points 32 at a time: pair key, CTA table
-    // slot (one insert per distinct key of the round) and the per-pair sums
-    // of the round's points, merged into the table by one lane per key.
-    for (uint32_t b0 = 0; b0 < nst; b0 += 32) {
-        const uint32_t i = b0 + (uint32_t)lane;
-        const bool v = i < nst;
-        uint32_t e = v ? wst[i] : 0u;
-        const int xo = (int)(e & 63), ro = (int)((e >> 6) & 15), t = (int)((e >> 10) & 3);
-        // the point's pixel and its tested neighbour in the label tile: R is
-        // the next word, BL, B and BR the row below (BP_SW - 1, BP_SW, BP_SW + 1)
-        static_assert(BP_SW == 72, "neighbour offsets 1, 71, 72, 73");
-        const uint32_t* pl = &lab[0][4] + ro * BP_SW + xo;
-        const uint32_t p = pl[0], q = pl[(0x49484701u >> (8 * t)) & 0xFFu];
-        const uint32_t lp = p & BP_VALUE, lq = q & BP_VALUE;
-        const int dir = (q & LABEL_PIXEL_MASK) > (p & LABEL_PIXEL_MASK) ? 1 : 0;
-        const unsigned long long key = v ? (((unsigned long long)min(lp, lq) << 32) | max(lp, lq)) : EMPTY_KEY;
-        // a round whose points all belong to pairs already over the limit
-        // contributes nothing: its points are neither aggregated nor listed
-        static_assert(DEAD_PAIRS == 2, "the test below reads both entries");
-        const bool dead = v && (key == dead0 || key == dead1);
-        if (__all_sync(0xFFFFFFFFu, dead || !v)) {
-            if (v) wst[i] = e | STAGE_DIRECT;
-            continue;
+    if (__any_sync(FULL, st != 0u)) {
+        const uint32_t ns = (uint32_t)__popc(st);
+        uint32_t incl = ns;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += v;
         }
-        const unsigned m = __match_any_sync(0xFFFFFFFFu, key);
-        const int leader = __ffs(m) - 1;
-        int ls = 0;
-        if (v && lane == leader) {
-            // a key new to the tile also takes its slot in the frame's
-            // table now, so the merge below needs one round trip less
-            bool fresh = false;
-            ls = local_insert(T, key, &fresh);
-            if (fresh) {
-                const uint32_t gs = global_insert(F, key);
-                if (gs == INVALID) atomicOr(status, ATAG_DEVFLAG_PAIR_OVERFLOW);
-                T.gslot[ls] = gs;
+        nst = __shfl_sync(FULL, incl, 31);
+        uint32_t pos = incl - ns;
+        const uint32_t base = stage_entry(0, 32 * k, r, t, 0) - 1u;  // + ffs: pixel 32 k + ffs - 1 (mod 2^32)
+        for (uint32_t mm = st; mm; mm &= mm - 1) wst[pos++] = base + (uint32_t)__ffs(mm);
+        __syncwarp();
+
+        // The warp takes its staged points 32 at a time.  The points of one
+        // pair at a time add to the warp's sums of its current pair: counts
+        // from ballots, extents and the weighted sum per lane.  When the
+        // pair changes the sums are reduced into the CTA table's slot.
+        unsigned long long cur = EMPTY_KEY;
+        int ls = -1, gx = 0, px = 0;
+        uint32_t cnt = 0, rows = 0, xmn = FULL, xmx = 0u;  // rows: bit 0 / 1, a point in the warp's first / second row
+        auto flush = [&]() {
+            if (ls < 0) return;
+            const uint32_t a = __reduce_min_sync(FULL, xmn), b = __reduce_max_sync(FULL, xmx);
+            const int s = __reduce_add_sync(FULL, px);
+            if (lane == 0) {
+                const uint32_t yd = 2u * (uint32_t)(y0 + 2 * warp);
+                atomicAdd(&T.cnt[ls], cnt);
+                atomicMin(&T.xmin[ls], a);
+                atomicMax(&T.xmax[ls], b);
+                atomicMin(&T.ymin[ls], (rows & 1u) ? yd : yd + 2u);
+                atomicMax(&T.ymax[ls], (rows & 2u) ? yd + 2u : yd);
+                atomicAdd(&T.gx[ls], gx);
+                atomicAdd(&T.pxgx[ls], s);
             }
-        }
-        ls = __shfl_sync(0xFFFFFFFFu, ls, leader);
-        const uint32_t xd = 2u * (uint32_t)(x0 + xo) + 1u, yd = 2u * (uint32_t)(y0 + ro);
-        const int gx = dir ? 1 : -1;
-        e |= (uint32_t)dir << 12;
-        if (v && ls < 0) {  // CTA table full: account for and list the point directly
-            e |= STAGE_DIRECT;
-            const uint32_t gs = global_insert(F, key);
-            if (gs == INVALID) {
-                atomicOr(status, ATAG_DEVFLAG_PAIR_OVERFLOW);
-            } else {
-                global_flush(F, gs, 1, xd, xd, yd, yd, gx, 0, (unsigned long long)(long long)((int)xd * gx));
-                const uint32_t at = atomicAdd(F.counters + CNT_POINTS, 1u);
-                if (at < F.point_cap) F.points[at] = ((unsigned long long)gs << 32) | stage_packed(e, x0, y0);
-                else atomicOr(status, ATAG_DEVFLAG_POINT_OVERFLOW);
+        };
+        for (uint32_t b0 = 0; b0 < nst; b0 += 32) {
+            const uint32_t i = b0 + (uint32_t)lane;
+            const bool v = i < nst;
+            uint32_t e = v ? wst[i] : 0u;
+            // the point's pixel and its tested neighbour in the label tile: R is
+            // the next word, BL, B and BR the row below (BP_SW - 1, BP_SW, BP_SW + 1)
+            static_assert(BP_SW == 72, "neighbour offsets 1, 71, 72, 73");
+            const uint32_t* pl = &lab[0][4] + ((e >> 6) & 15u) * BP_SW + (e & 63u);
+            const uint32_t p = pl[0], q = pl[(0x49484701u >> (8 * ((e >> 10) & 3u))) & 0xFFu];
+            const uint32_t lp = p & BP_VALUE, lq = q & BP_VALUE;
+            const uint32_t kA = min(lp, lq), kB = max(lp, lq);
+            const bool dir = q > p;  // the colours differ: q is the 255 pixel
+            const uint32_t xd = 2u * ((uint32_t)x0 + (e & 63u)) + 1u;
+            const unsigned second = __ballot_sync(FULL, (e >> 6) & 1u), up = __ballot_sync(FULL, dir);
+            e |= (dir ? 1u : 0u) << 12;
+            for (unsigned pend = __ballot_sync(FULL, v); pend;) {
+                const int leader = __ffs(pend) - 1;
+                const uint32_t gA = __shfl_sync(FULL, kA, leader), gB = __shfl_sync(FULL, kB, leader);
+                const bool in = v && kA == gA && kB == gB;
+                const unsigned m = __ballot_sync(FULL, in);
+                pend &= ~m;
+                const unsigned long long key = (unsigned long long)gA << 32 | gB;
+                if (key != cur) {
+                    flush();
+                    cur = key;
+                    if (lane == 0) {
+                        // a key new to the tile also takes its slot in the frame's
+                        // table now, so the merge below needs one round trip less
+                        bool fresh = false;
+                        ls = local_insert(T, key, &fresh);
+                        if (fresh) {
+                            const uint32_t gs = global_insert(F, key);
+                            if (gs == INVALID) atomicOr(F.counters + CNT_STATUS, ATAG_DEVFLAG_PAIR_OVERFLOW);
+                            T.gslot[ls] = gs;
+                        }
+                    }
+                    ls = __shfl_sync(FULL, ls, 0);
+                    cnt = rows = xmx = 0u;
+                    xmn = FULL;
+                    gx = px = 0;
+                }
+                if (ls >= 0) {
+                    cnt += (uint32_t)__popc(m);
+                    gx += 2 * __popc(m & up) - __popc(m);
+                    rows |= ((m & ~second) ? 1u : 0u) | ((m & second) ? 2u : 0u);
+                    if (in) {
+                        xmn = min(xmn, xd);
+                        xmx = max(xmx, xd);
+                        px += dir ? (int)xd : -(int)xd;
+                        e |= (uint32_t)ls << 13;
+                    }
+                } else if (in) {  // CTA table full: account for and list the point directly
+                    e |= STAGE_DIRECT;
+                    uint32_t* status = F.counters + CNT_STATUS;
+                    const uint32_t gs = global_insert(F, key), yd = 2u * (uint32_t)(y0 + (int)((e >> 6) & 15u));
+                    if (gs == INVALID) {
+                        atomicOr(status, ATAG_DEVFLAG_PAIR_OVERFLOW);
+                    } else {
+                        const int g = dir ? 1 : -1;
+                        global_flush(F, gs, 1, xd, xd, yd, yd, g, 0, (unsigned long long)(long long)((int)xd * g));
+                        const uint32_t at = atomicAdd(F.counters + CNT_POINTS, 1u);
+                        if (at < F.point_cap) F.points[at] = ((unsigned long long)gs << 32) | stage_packed(e, x0, y0);
+                        else atomicOr(status, ATAG_DEVFLAG_POINT_OVERFLOW);
+                    }
+                }
             }
-        } else {
-            e |= (uint32_t)ls << 13;
+            if (v) wst[i] = e;
         }
-        if (v) wst[i] = e;
-        const bool a = v && ls >= 0;
-        const uint32_t cnt = __reduce_add_sync(m, a ? 1u : 0u);
-        const uint32_t xmn = __reduce_min_sync(m, xd), xmx = __reduce_max_sync(m, xd);
-        const uint32_t ymn = __reduce_min_sync(m, yd), ymx = __reduce_max_sync(m, yd);
-        const int sgx = __reduce_add_sync(m, a ? gx : 0);
-        const int spx = __reduce_add_sync(m, a ? (int)xd * gx : 0);
-        if (a && lane == leader) {
-            atomicAdd(&T.cnt[ls], cnt);
-            atomicMin(&T.xmin[ls], xmn);
-            atomicMax(&T.xmax[ls], xmx);
-            atomicMin(&T.ymin[ls], ymn);
-            atomicMax(&T.ymax[ls], ymx);
-            atomicAdd(&T.gx[ls], sgx);
-            atomicAdd(&T.pxgx[ls], spx);
-        }
+        flush();
     }
     __syncthreads();
 
@@ -367,16 +383,19 @@ __device__ __forceinline__ void boundaries_pairs_impl(const FrameSet& fs, uint32
         if (key == EMPTY_KEY) continue;
         const uint32_t gs = T.gslot[i];  // INVALID: the frame's table was full (flagged)
         if (gs == INVALID) continue;
-        uint32_t old = global_flush(F, gs, T.cnt[i], T.xmin[i], T.xmax[i], T.ymin[i], T.ymax[i], T.gx[i], T.gy[i],
+        uint32_t old = global_flush(F, gs, T.cnt[i], T.xmin[i], T.xmax[i], T.ymin[i], T.ymax[i], T.gx[i], 0,
                                     (unsigned long long)(long long)T.pxgx[i]);
         T.gslot[i] = (old + T.cnt[i] > max_pixels) ? INVALID : gs;
         // the flush that crosses the limit publishes the pair, so that later
         // tiles skip its points (its count only grows: it stays rejected)
-        if (track_dead && old <= max_pixels && old + T.cnt[i] > max_pixels)
+        if (track_dead && old <= max_pixels && old + T.cnt[i] > max_pixels) {
+            const unsigned long long labels = pair_labels(key);
             for (uint32_t d = 0; d < DEAD_PAIRS; d++)
-                if (atomicCAS(F.dead_pairs + d, EMPTY_KEY, key) == EMPTY_KEY) break;
+                if (atomicCAS(F.dead_pairs + d, EMPTY_KEY, labels) == EMPTY_KEY) break;
+        }
     }
     __syncthreads();
+    if (nst == 0) return;
 
     // D: each warp lists the points of live pairs from its own staging
     // part: a count pass, one atomic for the warp's place in the list, then
@@ -394,17 +413,19 @@ __device__ __forceinline__ void boundaries_pairs_impl(const FrameSet& fs, uint32
     uint32_t at = 0;
     if (lane == 0) {
         at = atomicAdd(F.counters + CNT_POINTS, nlive);
-        if ((unsigned long long)at + nlive > F.point_cap) atomicOr(status, ATAG_DEVFLAG_POINT_OVERFLOW);
+        if ((unsigned long long)at + nlive > F.point_cap) atomicOr(F.counters + CNT_STATUS, ATAG_DEVFLAG_POINT_OVERFLOW);
     }
     at = __shfl_sync(0xFFFFFFFFu, at, 0);
     const unsigned lt = (1u << lane) - 1u;
+    const uint32_t point_cap = F.point_cap;
+    unsigned long long* points = F.points;
     for (uint32_t b0 = 0; b0 < nst; b0 += 32) {
         const uint32_t i = b0 + (uint32_t)lane;
         const unsigned m = b0 == 0 ? m_first : __ballot_sync(0xFFFFFFFFu, live_at(i));
         const bool lv = (m >> lane) & 1u;
         if (lv) {
             const uint32_t e = wst[i], dst = at + (uint32_t)__popc(m & lt);
-            if (dst < F.point_cap) F.points[dst] = ((unsigned long long)T.gslot[(e >> 13) & 255] << 32) | stage_packed(e, x0, y0);
+            if (dst < point_cap) points[dst] = ((unsigned long long)T.gslot[(e >> 13) & 255] << 32) | stage_packed(e, x0, y0);
         }
         at += (uint32_t)__popc(m);
     }
