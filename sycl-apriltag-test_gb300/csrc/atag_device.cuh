@@ -497,27 +497,6 @@ __device__ __forceinline__ float filter_tap(int i) {
     }
 }
 
-// Combinatorial number system decode of n < 210 into 4 descending indices
-// below 10 (combinadics.h:36-53 with Combinadics<uint8_t,15,4,16>).
-__device__ __forceinline__ void combination_decode(uint32_t num, uint32_t out[4]) {
-    // C(c, k) for c = 0..9, k = 4..1
-    const uint32_t c4[10] = {0, 0, 0, 0, 1, 5, 15, 35, 70, 126};
-    const uint32_t c3[10] = {0, 0, 0, 1, 4, 10, 20, 35, 56, 84};
-    const uint32_t c2[10] = {0, 0, 1, 3, 6, 10, 15, 21, 28, 36};
-    int c = 9;
-    while (c > 0 && c4[c] > num) c--;
-    num -= c4[c];
-    out[0] = c;
-    c = 9;
-    while (c > 0 && c3[c] > num) c--;
-    num -= c3[c];
-    out[1] = c;
-    c = 9;
-    while (c > 0 && c2[c] > num) c--;
-    num -= c2[c];
-    out[2] = c;
-    out[3] = num;
-}
 __host__ __device__ __forceinline__ uint32_t n_choose_4(uint32_t n) {
     return n < 4 ? 0 : n * (n - 1) * (n - 2) * (n - 3) / 24;
 }

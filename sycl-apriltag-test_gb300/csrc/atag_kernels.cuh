@@ -205,8 +205,6 @@ __global__ void k_cluster_sort_large(const __grid_constant__ FrameSet fs, const 
 __global__ void k_cluster_lines(const __grid_constant__ FrameSet fs, const uint32_t* run_offsets, uint32_t n_frames);
 constexpr uint32_t CE_LINES_SMEM = 4 * 12432;  // four warps' RunSums
 __global__ void k_cluster_prefix(const __grid_constant__ FrameSet fs, const uint32_t* run_offsets);
-__global__ void k_cluster_peaks(const __grid_constant__ FrameSet fs, const uint32_t* cluster_offsets,
-                                uint32_t n_frames);
 __global__ void k_peaks_scan(const __grid_constant__ FrameSet fs, PipelineParams p);
 __global__ void k_batch_offsets(const __grid_constant__ FrameSet fs, uint32_t n_frames, BatchOffsets a);
 __global__ void k_index_quads(const __grid_constant__ FrameSet fs, const uint32_t* work_offsets, uint32_t n_frames,

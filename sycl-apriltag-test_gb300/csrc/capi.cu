@@ -214,7 +214,7 @@ size_t layout_frame(char* base, uint32_t w, uint32_t h, uint32_t factor, bool ow
 
 constexpr int RING = 16;
 constexpr int CAPTURE_SLOTS = 16;  // distinct frame tables that captured graphs may hold
-constexpr size_t WORK_LISTS = 5;  // batch-wide work lists of the per-cluster kernels
+constexpr size_t WORK_LISTS = 4;  // batch-wide work lists of the per-cluster kernels
 constexpr int MAX_LANES = 4;      // sub-batches of one call that run concurrently
 
 // Workspace of atag_cluster: the pair table and the cluster scratch of one
@@ -511,7 +511,7 @@ atag_status atag_do_indexing(const atag_peak_extents* extents, size_t count, con
     if (!extents || !corners || !points || !cluster_extents || !fitted)
         return fail(ATAG_ERR_INVALID_ARGUMENT, "do_indexing: null pointer");
     float cosc = (float)std::cos(10 * M_PI / 180);
-    k_do_indexing<<<grid2(std::min<size_t>(count, 65535), 1), 256, 0, (cudaStream_t)stream>>>(
+    k_do_indexing<<<grid2(std::min<size_t>(count, 65535), 1), 128, 0, (cudaStream_t)stream>>>(
         extents, count, corners, points, cluster_extents, 10.0f, cosc, fitted);
     LAUNCHED();
     return ATAG_OK;
@@ -527,7 +527,7 @@ atag_status atag_process_fitted_quads(const atag_fitted_quad* fitted, size_t cou
     if (!d_count || (count && (!fitted || !quads))) return fail(ATAG_ERR_INVALID_ARGUMENT, "process_fitted_quads: null pointer");
     atag_config c;
     if (cfg) c = *cfg; else atag_config_default(&c);
-    k_process_quads<<<1, 256, 0, (cudaStream_t)stream>>>(fitted, count, make_params(c), quads, cap, d_count);
+    k_process_quads<<<1, 1024, 0, (cudaStream_t)stream>>>(fitted, count, make_params(c), quads, cap, d_count);
     LAUNCHED();
     return ATAG_OK;
 }
@@ -899,13 +899,12 @@ static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, con
     const PipelineParams& p = det->pp;
     const int sms = det->dev->num_sms;
     // batch-wide work lists of this lane: small clusters, large clusters,
-    // point runs, all clusters, clusters with peaks; one queue cursor each
+    // point runs, clusters with peaks; one queue cursor each
     uint32_t* work = det->d_work + (size_t)lane * (WORK_LISTS * (det->max_frames + 1) + WORK_LISTS);
     uint32_t* off_small = work;
     uint32_t* off_large = work + (n + 1);
     uint32_t* off_runs = work + 2 * (n + 1);
-    uint32_t* off_clusters = work + 3 * (n + 1);
-    uint32_t* off_peaks = work + 4 * (n + 1);
+    uint32_t* off_peaks = work + 3 * (n + 1);
     uint32_t* wc = work + WORK_LISTS * (det->max_frames + 1);
     cudaStream_t side = det->side[lane];
     auto mark = [&](int i) -> atag_status {
@@ -956,8 +955,7 @@ static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, con
     k_pairs_finalize<<<(unsigned)n, 1024, 0, s>>>(fs, p, (uint32_t)tu.small_cluster_max);
     LAUNCHED();
     {
-        BatchOffsets bo{{CNT_SMALL, CNT_LARGE, CNT_RUNS, CNT_CLUSTERS},
-                        {off_small, off_large, off_runs, off_clusters}, wc};
+        BatchOffsets bo{{CNT_SMALL, CNT_LARGE, CNT_RUNS, 0}, {off_small, off_large, off_runs, nullptr}, wc};
         k_batch_offsets<<<1, 1024, 0, s>>>(fs, (uint32_t)n, bo);
     }
     LAUNCHED();
@@ -983,13 +981,11 @@ static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, con
     k_cluster_lines<<<sms * 4, 128, CE_LINES_SMEM, s>>>(fs, off_runs, (uint32_t)n);
     LAUNCHED();
     STAGE(11);
-    k_cluster_peaks<<<sms * 4, 256, 0, s>>>(fs, off_clusters, (uint32_t)n);
-    LAUNCHED();
     STAGE(12);
     k_peaks_scan<<<(unsigned)n, 1024, 0, s>>>(fs, p);
     LAUNCHED();
     {
-        BatchOffsets bo{{CNT_PEAKCLU, 0, 0, 0}, {off_peaks, nullptr, nullptr, nullptr}, wc + 4};
+        BatchOffsets bo{{CNT_PEAKCLU, 0, 0, 0}, {off_peaks, nullptr, nullptr, nullptr}, wc + 3};
         k_batch_offsets<<<1, 1024, 0, s>>>(fs, (uint32_t)n, bo);
     }
     LAUNCHED();

@@ -21,10 +21,10 @@
 //   4. k_cluster_sort: one CTA per cluster sorts by (theta, point) in
 //      shared memory and writes ClusterPoints and the line-fit inputs;
 //      k_cluster_lines: line-fit prefix sums and fit_lines (windowed errors,
-//      7-tap filter, peaks), a warp per run of points; k_cluster_peaks: the
-//      10 best peaks of each cluster;
-//   5. k_peaks_scan / k_index_quads / k_compact_quads: peak extents,
-//      do_indexing and the corner intersection, quads in reference order.
+//      7-tap filter, peaks), a warp per run of points;
+//   5. k_peaks_scan / k_index_quads / k_compact_quads: peak extents, the 10
+//      best peaks, do_indexing and the corner intersection, quads in reference
+//      order.
 #include "atag_kernels.cuh"
 #include "atag_pairs.cuh"
 #include "atag_quads.cuh"
@@ -1143,48 +1143,6 @@ __global__ void __launch_bounds__(32 * CE_WARPS, 4) k_cluster_prefix(const __gri
 }
 
 // ---------------------------------------------------------------------------
-// 4c. the 10 best peaks of each cluster by (error desc, index asc): the
-// corner sort of main.cpp:856-863 restricted to what do_indexing reads
-// (fit_quad.cpp:411-414 uses at most 10 corners).  One warp per cluster.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_cluster_peaks(const __grid_constant__ FrameSet fs,
-                                                       const uint32_t* __restrict__ cluster_offsets,
-                                                       uint32_t n_frames) {
-    const uint32_t lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    const uint32_t total = cluster_offsets[n_frames];
-    for (uint32_t item = blockIdx.x * wpb + (threadIdx.x >> 5); item < total; item += gridDim.x * wpb) {
-        const uint32_t fidx = find_frame(cluster_offsets, n_frames, item);
-        const FrameDesc& F = fs.get(fidx);
-        const uint32_t cid = item - cluster_offsets[fidx];
-        const uint32_t npeaks = F.peak_count[cid];
-        const unsigned long long* cand =
-            reinterpret_cast<const unsigned long long*>(F.errbuf) + F.cluster_extents[cid].start;
-        const uint32_t take = npeaks < 10u ? npeaks : 10u;
-        unsigned long long last = ~0ull;
-        for (uint32_t j = 0; j < take; j++) {
-            unsigned long long best = 0;
-            for (uint32_t c = lane; c < npeaks; c += 32) {
-                const unsigned long long key = cand[c];
-                if (key < last && key > best) best = key;
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const unsigned long long v = __shfl_xor_sync(0xffffffffu, best, o);
-                best = v > best ? v : best;
-            }
-            if (lane == 0) {
-                atag_corner c;
-                c.line_fit_point_index = ~(uint32_t)best;
-                c.cluster_index = (uint16_t)cid;
-                c.error = float_from_order_key((uint32_t)(best >> 32));
-                F.peaks[(size_t)cid * 10 + j] = c;
-            }
-            last = best;
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
 // 5. peak extents (D10-D12), do_indexing + corners, ordered quads
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) k_peaks_scan(const __grid_constant__ FrameSet fs, PipelineParams p) {
@@ -1212,30 +1170,84 @@ __global__ void __launch_bounds__(1024) k_peaks_scan(const __grid_constant__ Fra
     }
 }
 
+// The 10 best corner candidates of a cluster by (error desc, index asc), one
+// per lane from lane 0 (0 past the last): the corner sort of main.cpp:856-863
+// restricted to what do_indexing reads (fit_quad.cpp:411-414 uses at most 10
+// corners).
+__device__ __forceinline__ unsigned long long best_candidates(const unsigned long long* cand, uint32_t n) {
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    constexpr int KEEP = 4;  // per lane in registers; clusters with more candidates than fit read the rest each time
+    const uint32_t lane = threadIdx.x & 31, take = n < 10u ? n : 10u;
+    unsigned long long c[KEEP], mine = 0, last = ~0ull;
+#pragma unroll
+    for (int u = 0; u < KEEP; u++) c[u] = lane + 32u * u < n ? cand[lane + 32u * u] : 0ull;
+    for (uint32_t j = 0; j < take; j++) {
+        unsigned long long best = 0;
+#pragma unroll
+        for (int u = 0; u < KEEP; u++)
+            if (c[u] < last && c[u] > best) best = c[u];
+        for (uint32_t i = lane + 32u * KEEP; i < n; i += 32) {
+            const unsigned long long key = cand[i];
+            if (key < last && key > best) best = key;
+        }
+        const uint32_t hi = __reduce_max_sync(FULL, (uint32_t)(best >> 32));
+        const uint32_t lo = __reduce_max_sync(FULL, (uint32_t)(best >> 32) == hi ? (uint32_t)best : 0u);
+        last = (unsigned long long)hi << 32 | lo;
+        if (lane == j) mine = last;
+    }
+    return mine;
+}
+
+// One warp per cluster with peaks: its 10 best corners, the combination
+// search, and the corners of the chosen four on lanes of their own.  Bound by
+// the latency of one warp: the clusters go round the CTAs first, so that a
+// lone frame's ~100 use every SM.  A lone 1080p frame's selection and search
+// took 12 + 29 us as a kernel each with serial corners (25 now), 64 frames
+// 30 + 133 us (82 now).
 __global__ void __launch_bounds__(256) k_index_quads(const __grid_constant__ FrameSet fs,
                                                      const uint32_t* __restrict__ work_offsets, uint32_t n_frames,
                                                      PipelineParams p) {
     __shared__ SegmentTable T[8];  // one per warp
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t total = work_offsets[n_frames];
-    for (uint32_t item = blockIdx.x * 8 + wid; item < total; item += gridDim.x * 8) {
+    for (uint32_t item = blockIdx.x + gridDim.x * wid; item < total; item += gridDim.x * 8) {
         const uint32_t fidx = find_frame(work_offsets, n_frames, item);
         const FrameDesc& F = fs.get(fidx);
         const uint32_t q = item - work_offsets[fidx];
-        const uint32_t cid = F.peak_clusters[q];
+        const uint32_t cid = F.peak_clusters[q], count = F.peak_count[cid];
         const atag_cluster_extents ce = F.cluster_extents[p.compat_peak_index ? q : cid];
+        const unsigned long long key = best_candidates(
+            reinterpret_cast<const unsigned long long*>(F.errbuf) + F.cluster_extents[cid].start, count);
+        if (lane < min(count, 10u)) {
+            atag_corner c;
+            c.line_fit_point_index = ~(uint32_t)key;
+            c.cluster_index = (uint16_t)cid;
+            c.error = float_from_order_key((uint32_t)(key >> 32));
+            F.peaks[(size_t)cid * 10 + lane] = c;
+        }
         atag_fitted_quad* fq = F.fitted + q;
-        const int chosen = index_one_cluster(F.peak_count[cid], F.peaks + (size_t)cid * 10, F.line_fit + ce.start,
-                                             ce.count, p.max_line_fit_mse, p.cos_critical_f, T[wid], fq);
+        QuadSide side;
+        const int chosen = index_one_cluster(count, ~(uint32_t)key, F.line_fit + ce.start, ce.count, p.max_line_fit_mse,
+                                             p.cos_critical_f, T[wid], fq, side);
         if (chosen < 0) {
             // no combination: the quad stays zero (main.cpp:318-319)
             for (uint32_t k = lane; k < sizeof(atag_fitted_quad) / 4; k += 32) reinterpret_cast<uint32_t*>(fq)[k] = 0u;
             if (lane == 0) F.quad_ok[q] = 0;
-        } else if (lane == ((uint32_t)chosen & 31u)) {
-            atag_quad_corners qc;
-            const bool ok = quad_corners(*fq, p, q, &qc);
-            F.quad_tmp[q] = qc;
-            F.quad_ok[q] = ok ? 1u : 0u;
+        } else {
+            float line[4] = {0.0f, 0.0f, 0.0f, 0.0f}, cx, cy, e, mse;
+            if (lane < 4) fit_line(side.m, side.points, line, &e, &mse);
+            const bool any = __any_sync(0xFFFFFFFFu, lane < 4 && side.index != 0);
+            const bool ok = __shfl_sync(0xFFFFFFFFu, (int)quad_corners8(line, p, cx, cy), 0) && any;
+            atag_quad_corners& qc = F.quad_tmp[q];
+            if (lane < 4) {
+                qc.corners[lane][0] = cx;
+                qc.corners[lane][1] = cy;
+            } else if (lane == 4) {
+                qc.reversed_border = (uint8_t)p.reversed_border;
+                qc.pad_[0] = qc.pad_[1] = qc.pad_[2] = 0;
+                qc.blob_index = q;
+                F.quad_ok[q] = ok ? 1u : 0u;
+            }
         }
         __syncwarp();
     }

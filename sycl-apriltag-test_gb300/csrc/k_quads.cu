@@ -73,44 +73,63 @@ __global__ void __launch_bounds__(128) k_fit_lines_windowed(const atag_line_fit_
 }
 
 // ---------------------------------------------------------------------------
-// do_indexing (fit_quad.cpp:392-535): one 256-thread CTA per peak extent,
-// one thread per combination number; cluster_extents is indexed by the
-// extent's position, exactly as the reference does.
+// do_indexing (fit_quad.cpp:392-535): one warp per peak extent;
+// cluster_extents is indexed by the extent's position, exactly as the
+// reference does.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_do_indexing(const atag_peak_extents* __restrict__ extents, size_t count,
+__global__ void __launch_bounds__(128) k_do_indexing(const atag_peak_extents* __restrict__ extents, size_t count,
                                                      const atag_corner* __restrict__ corners,
                                                      const atag_line_fit_point* __restrict__ points,
                                                      const atag_cluster_extents* __restrict__ cluster_extents,
                                                      float max_mse, float cos_critical,
                                                      atag_fitted_quad* __restrict__ fitted) {
-    __shared__ SegmentTable T[8];  // one per warp
-    const uint32_t wid = threadIdx.x >> 5;
-    for (size_t q = (size_t)blockIdx.x * 8 + wid; q < count; q += (size_t)gridDim.x * 8) {
+    __shared__ SegmentTable T[4];  // one per warp
+    const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (size_t q = blockIdx.x + (size_t)gridDim.x * wid; q < count; q += (size_t)gridDim.x * 4) {
         const atag_peak_extents pe = extents[q];
         const atag_cluster_extents ce = cluster_extents[q];
-        index_one_cluster(pe.count, corners + pe.start, points + ce.start, ce.count, max_mse, cos_critical, T[wid],
-                          fitted + q);
+        const uint32_t idx = lane < min(pe.count, 10u) ? corners[pe.start + lane].line_fit_point_index : 0u;
+        QuadSide side;
+        index_one_cluster(pe.count, idx, points + ce.start, ce.count, max_mse, cos_critical, T[wid], fitted + q, side);
         __syncwarp();
     }
 }
 
 // ---------------------------------------------------------------------------
 // process_fitted_quads (main.cpp:1035-1162) up to tag decoding, on one CTA
-// with an ordered compaction.
+// with an ordered compaction: eight lanes per quad, for the latency of one
+// quad's FP64 chain is what it takes.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_process_quads(const atag_fitted_quad* __restrict__ fitted, size_t count,
-                                                       PipelineParams p, atag_quad_corners* __restrict__ out,
-                                                       size_t cap, uint32_t* __restrict__ count_out) {
+__global__ void __launch_bounds__(1024) k_process_quads(const atag_fitted_quad* __restrict__ fitted, size_t count,
+                                                        PipelineParams p, atag_quad_corners* __restrict__ out,
+                                                        size_t cap, uint32_t* __restrict__ count_out) {
     __shared__ uint32_t red[33];
+    const uint32_t g = threadIdx.x & 7;
     uint32_t base = 0;
-    for (size_t c0 = 0; c0 < count; c0 += blockDim.x) {
-        size_t i = c0 + threadIdx.x;
-        atag_quad_corners qc;
-        bool ok = false;
-        if (i < count) ok = quad_corners(fitted[i], p, (uint32_t)i, &qc);
+    for (size_t c0 = 0; c0 < count; c0 += 128) {
+        const size_t i = c0 + (threadIdx.x >> 3);
+        float line[4] = {0.0f, 0.0f, 0.0f, 0.0f}, cx, cy, e, mse;
+        bool any = false;
+        if (i < count) {
+            const atag_fitted_quad& fq = fitted[i];
+            any = (fq.indices[0] | fq.indices[1] | fq.indices[2] | fq.indices[3]) != 0;
+            if (any && g < 4) fit_line(load_moment(&fq.moments[g]), fq.num_in_moments[g], line, &e, &mse);
+        }
+        const bool ok = quad_corners8(line, p, cx, cy) && any;
         uint32_t total;
-        uint32_t pos = block_exclusive_scan_u32(ok ? 1u : 0u, red, &total);
-        if (ok && base + pos < cap) out[base + pos] = qc;
+        const uint32_t pos = block_exclusive_scan_u32(ok && g == 0 ? 1u : 0u, red, &total);
+        const uint32_t at = base + __shfl_sync(0xFFFFFFFFu, pos, (int)(threadIdx.x & 31) & ~7);
+        if (ok && at < cap) {
+            atag_quad_corners& qc = out[at];
+            if (g < 4) {
+                qc.corners[g][0] = cx;
+                qc.corners[g][1] = cy;
+            } else if (g == 4) {
+                qc.reversed_border = (uint8_t)p.reversed_border;
+                qc.pad_[0] = qc.pad_[1] = qc.pad_[2] = 0;
+                qc.blob_index = (uint32_t)i;
+            }
+        }
         base += total;
     }
     if (threadIdx.x == 0) *count_out = base < cap ? base : (uint32_t)cap;
