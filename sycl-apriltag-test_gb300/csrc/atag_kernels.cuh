@@ -103,8 +103,24 @@ __host__ __device__ constexpr uint32_t ccl_edge_words(uint32_t rows) { return 2 
 struct FrameSet {
     const FrameDesc* table;
     FrameDesc one;
+    uint32_t overlap;  // launched to overlap the previous kernel's end (await_previous_kernel)
     __device__ __forceinline__ const FrameDesc& get(uint32_t i) const { return table ? table[i] : one; }
 };
+
+// First in every kernel of the detector's path when it is launched with
+// fs.overlap: its CTAs may then be placed on the SMs while the kernel before
+// it still runs (programmatic dependent launch).  The first call returns when
+// that kernel, and with it everything before it, has finished; the second lets
+// the next kernel's CTAs be placed once all of this kernel's have started.
+// The compiler may move a read-only load (__ldg, const __restrict__) up across
+// the wait, so one of data that an earlier kernel wrote goes through a
+// descriptor's pointer that is itself read, by a plain load, after it.
+// Large lanes run without: the calls alone made their pixel kernels, of up to
+// half a million short CTAs, 1-4% slower, so those are compiled both ways.
+__device__ __forceinline__ void await_previous_kernel() {
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+}
 
 // per-frame counters (FrameDesc::counters[...])
 enum Counter : uint32_t {
@@ -167,19 +183,27 @@ struct PipelineParams {
 // k_pixels.cu
 __global__ void k_decimate(const __grid_constant__ FrameSet fs);
 __global__ void k_threshold(const __grid_constant__ FrameSet fs, int min_diff, int write_extrema);
+__global__ void k_threshold_overlapped(const __grid_constant__ FrameSet fs, int min_diff, int write_extrema);
 // CCL tiles of 32 x 8 or 32 x 16 blocks (2x2 pixels)
 __global__ void k_ccl_local_r8(const __grid_constant__ FrameSet fs);
+__global__ void k_ccl_local_r8_overlapped(const __grid_constant__ FrameSet fs);
 __global__ void k_ccl_local_r16(const __grid_constant__ FrameSet fs);
+__global__ void k_ccl_local_r16_overlapped(const __grid_constant__ FrameSet fs);
 __global__ void k_ccl_local_stage(const __grid_constant__ FrameSet fs);  // r16 over a caller's image: any byte values
 __global__ void k_ccl_local_r32(const __grid_constant__ FrameSet fs);
+__global__ void k_ccl_local_r32_overlapped(const __grid_constant__ FrameSet fs);
 __global__ void k_ccl_border_r16(const __grid_constant__ FrameSet fs);
 __global__ void k_ccl_border_edges_r8(const __grid_constant__ FrameSet fs);
+__global__ void k_ccl_border_edges_r8_overlapped(const __grid_constant__ FrameSet fs);
 __global__ void k_ccl_border_edges_r16(const __grid_constant__ FrameSet fs);
+__global__ void k_ccl_border_edges_r16_overlapped(const __grid_constant__ FrameSet fs);
 __global__ void k_ccl_border_edges_r32(const __grid_constant__ FrameSet fs);
+__global__ void k_ccl_border_edges_r32_overlapped(const __grid_constant__ FrameSet fs);
 // final labelling: grid (cdiv(w / 4, CCL_FINAL_THREADS), h / 2, frames) of
 // CCL_FINAL_THREADS threads, one pair of 2x2 blocks per thread
 constexpr int CCL_FINAL_THREADS = 128;
 __global__ void k_ccl_final(const __grid_constant__ FrameSet fs);
+__global__ void k_ccl_final_overlapped(const __grid_constant__ FrameSet fs);
 __global__ void k_boundaries_dense(const __grid_constant__ FrameSet fs, uint32_t min_size);
 
 // k_quads.cu (drop-in stage kernels)
@@ -195,7 +219,9 @@ __global__ void k_process_quads(const atag_fitted_quad* fitted, size_t count, Pi
 __global__ void k_reset_frames(const __grid_constant__ FrameSet fs);
 // boundary tiles of 64 x 8 or 64 x 16 pixels
 __global__ void k_boundaries_pairs_r8(const __grid_constant__ FrameSet fs, uint32_t min_size);
+__global__ void k_boundaries_pairs_r8_overlapped(const __grid_constant__ FrameSet fs, uint32_t min_size);
 __global__ void k_boundaries_pairs_r16(const __grid_constant__ FrameSet fs, uint32_t min_size);
+__global__ void k_boundaries_pairs_r16_overlapped(const __grid_constant__ FrameSet fs, uint32_t min_size);
 __global__ void k_pairs_finalize(const __grid_constant__ FrameSet fs, PipelineParams p, uint32_t small_max);
 __global__ void k_scatter_points(const __grid_constant__ FrameSet fs);
 __global__ void k_cluster_sort_small(const __grid_constant__ FrameSet fs, const uint32_t* work_offsets,

@@ -42,6 +42,24 @@ atag_status fail(atag_status s, const char* fmt, ...) {
         if (e_ != cudaSuccess) return fail(ATAG_ERR_CUDA, "launch: %s", cudaGetErrorString(e_));   \
     } while (0)
 
+// Launch a kernel of the detector's path.  `overlap`: its CTAs may be placed
+// while the stream's previous kernel still runs (see await_previous_kernel).
+template <typename... P, typename... A>
+cudaError_t launch(bool overlap, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s,
+                   A&&... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 struct DeviceInfo {
     int device = -1;
     int num_sms = 0;
@@ -214,6 +232,7 @@ size_t layout_frame(char* base, uint32_t w, uint32_t h, uint32_t factor, bool ow
 
 constexpr int RING = 16;
 constexpr int CAPTURE_SLOTS = 16;  // distinct frame tables that captured graphs may hold
+constexpr size_t OVERLAP_LANE_PIXELS = 6u << 20;  // see launch_lane
 constexpr size_t WORK_LISTS = 4;  // batch-wide work lists of the per-cluster kernels
 constexpr int MAX_LANES = 4;      // sub-batches of one call that run concurrently
 
@@ -878,14 +897,15 @@ static atag_status upload_table(atag_detector* det, const std::vector<FrameDesc>
 }
 
 // The whole path for frames [first, last) of the uploaded table, on stream
-// s, with lane `lane`'s work lists and side stream.  Stage events are
+// s, with lane `lane` of `lanes`' work lists and side stream.  Stage events are
 // recorded when `timed`.
 static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, const std::vector<FrameDesc>& t,
-                               size_t first, size_t last, cudaStream_t s, int lane, bool timed) {
+                               size_t first, size_t last, cudaStream_t s, int lane, int lanes, bool timed) {
     const size_t n = last - first;
-    size_t mw = 0, mh = 0, max_pair = 0, max_points = 0, max_cluster = 0;
+    size_t mw = 0, mh = 0, max_pair = 0, max_points = 0, max_cluster = 0, pixels = 0;
     bool any_decim = false;
     for (size_t i = first; i < last; i++) {
+        pixels += (size_t)t[i].width * t[i].height;
         mw = std::max<size_t>(mw, t[i].width);
         mh = std::max<size_t>(mh, t[i].height);
         max_pair = std::max<size_t>(max_pair, t[i].pair_cap);
@@ -916,51 +936,65 @@ static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, con
     const int ccl_rows = tu.ccl_tile_rows == 8 || tu.ccl_tile_rows == 32 ? tu.ccl_tile_rows : 16;
     const int bp_rows = tu.boundary_tile_rows == 8 ? 8 : 16;
     const size_t tiles_ccl = cdiv(mw / 2, 32) * cdiv(mh / 2, (size_t)ccl_rows);
+    // Placing a kernel's CTAs early hides its launch and its start when the
+    // kernels are launched one by one: 1920x1080 214 -> 187 us, 640x480 145 ->
+    // 127, 3840x2160 383 -> 367, 8 of 1280x720 291 -> 270.  Not in a captured
+    // graph, whose kernels already follow each other closely (1920x1080 187 ->
+    // 185, but 960x540 128 -> 135 and 3840x2160 348 -> 358).  The waiting CTAs
+    // also keep another lane's off the SMs: with two lanes of 8 megapixels and
+    // more, batches of unequal frames lost up to 4% (64 frames 2907 -> 3036
+    // us), while lanes below 6 gained.
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s, &cs));
+    const bool overlap =
+        !timed && cs == cudaStreamCaptureStatusNone && (lanes == 1 || pixels <= OVERLAP_LANE_PIXELS);
+    fs.overlap = overlap ? 1u : 0u;
+#define PIXEL(k) (overlap ? k##_overlapped : k)
     STAGE(0);
     k_reset_frames<<<grid2(cdiv(max_pair, 256), n), 256, 0, s>>>(fs);
     LAUNCHED();
     STAGE(1);
     if (any_decim) {
-        k_decimate<<<grid2(std::min<size_t>(cdiv(mw / 4 * mh, 256), 2048), n), 256, 0, s>>>(fs);
+        launch(overlap, k_decimate, grid2(std::min<size_t>(cdiv(mw / 4 * mh, 256), 2048), n), 256, 0, s, fs);
         LAUNCHED();
     }
     STAGE(2);
-    k_threshold<<<grid2(cdiv(mw / 4, 32) * cdiv(mh / 4, 16), n), 256, 0, s>>>(fs, p.min_white_black_diff, 0);
+    launch(overlap, PIXEL(k_threshold), grid2(cdiv(mw / 4, 32) * cdiv(mh / 4, 16), n), 256, 0, s, fs, p.min_white_black_diff, 0);
     LAUNCHED();
     STAGE(3);
-    if (ccl_rows == 8) k_ccl_local_r8<<<ccl_grid(mw, mh, 8, n), 32 * 8, 0, s>>>(fs);
-    else if (ccl_rows == 32) k_ccl_local_r32<<<ccl_grid(mw, mh, 32, n), 32 * 32, 0, s>>>(fs);
-    else k_ccl_local_r16<<<ccl_grid(mw, mh, 16, n), 32 * 16, 0, s>>>(fs);
+    if (ccl_rows == 8) launch(overlap, PIXEL(k_ccl_local_r8), ccl_grid(mw, mh, 8, n), 32 * 8, 0, s, fs);
+    else if (ccl_rows == 32) launch(overlap, PIXEL(k_ccl_local_r32), ccl_grid(mw, mh, 32, n), 32 * 32, 0, s, fs);
+    else launch(overlap, PIXEL(k_ccl_local_r16), ccl_grid(mw, mh, 16, n), 32 * 16, 0, s, fs);
     LAUNCHED();
     STAGE(4);
     {
         const size_t border = tiles_ccl * (32 + 2 * (ccl_rows - 1));
-        if (ccl_rows == 8) k_ccl_border_edges_r8<<<grid2(cdiv(border, 256), n), 256, 0, s>>>(fs);
-        else if (ccl_rows == 32) k_ccl_border_edges_r32<<<grid2(cdiv(border, 256), n), 256, 0, s>>>(fs);
-        else k_ccl_border_edges_r16<<<grid2(cdiv(border, 256), n), 256, 0, s>>>(fs);
+        if (ccl_rows == 8) launch(overlap, PIXEL(k_ccl_border_edges_r8), grid2(cdiv(border, 256), n), 256, 0, s, fs);
+        else if (ccl_rows == 32) launch(overlap, PIXEL(k_ccl_border_edges_r32), grid2(cdiv(border, 256), n), 256, 0, s, fs);
+        else launch(overlap, PIXEL(k_ccl_border_edges_r16), grid2(cdiv(border, 256), n), 256, 0, s, fs);
         LAUNCHED();
     }
     STAGE(5);
-    k_ccl_final<<<final_grid(mw, mh, n), CCL_FINAL_THREADS, 0, s>>>(fs);
+    launch(overlap, PIXEL(k_ccl_final), final_grid(mw, mh, n), CCL_FINAL_THREADS, 0, s, fs);
     LAUNCHED();
     STAGE(6);
     // grid (frames, tile columns, tile rows): at most 64 x 512 tiles of a
     // 4096 x 4096 frame
     if (bp_rows == 8)
-        k_boundaries_pairs_r8<<<dim3((unsigned)n, (unsigned)cdiv(mw, 64), (unsigned)cdiv(mh, 8)), 16 * 8, 0, s>>>(fs, p.min_component_size);
+        launch(overlap, PIXEL(k_boundaries_pairs_r8), dim3((unsigned)n, (unsigned)cdiv(mw, 64), (unsigned)cdiv(mh, 8)), 16 * 8, 0, s, fs, p.min_component_size);
     else
-        k_boundaries_pairs_r16<<<dim3((unsigned)n, (unsigned)cdiv(mw, 64), (unsigned)cdiv(mh, 16)), 16 * 16, 0, s>>>(fs, p.min_component_size);
+        launch(overlap, PIXEL(k_boundaries_pairs_r16), dim3((unsigned)n, (unsigned)cdiv(mw, 64), (unsigned)cdiv(mh, 16)), 16 * 16, 0, s, fs, p.min_component_size);
     LAUNCHED();
     STAGE(7);
-    k_pairs_finalize<<<(unsigned)n, 1024, 0, s>>>(fs, p, (uint32_t)tu.small_cluster_max);
+    launch(overlap, k_pairs_finalize, (unsigned)n, 1024, 0, s, fs, p, (uint32_t)tu.small_cluster_max);
     LAUNCHED();
     {
         BatchOffsets bo{{CNT_SMALL, CNT_LARGE, CNT_RUNS, 0}, {off_small, off_large, off_runs, nullptr}, wc};
-        k_batch_offsets<<<1, 1024, 0, s>>>(fs, (uint32_t)n, bo);
+        launch(overlap, k_batch_offsets, 1, 1024, 0, s, fs, (uint32_t)n, bo);
     }
     LAUNCHED();
     STAGE(8);
-    k_scatter_points<<<grid2(std::min<size_t>(cdiv(max_points, 256), 1024), n), 256, 0, s>>>(fs);
+    launch(overlap, k_scatter_points, grid2(std::min<size_t>(cdiv(max_points, 256), 1024), n), 256, 0, s, fs);
     LAUNCHED();
     STAGE(9);
     // large clusters on the side stream, concurrently with the small ones
@@ -982,26 +1016,27 @@ static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, con
     LAUNCHED();
     STAGE(11);
     STAGE(12);
-    k_peaks_scan<<<(unsigned)n, 1024, 0, s>>>(fs, p);
+    launch(overlap, k_peaks_scan, (unsigned)n, 1024, 0, s, fs, p);
     LAUNCHED();
     {
         BatchOffsets bo{{CNT_PEAKCLU, 0, 0, 0}, {off_peaks, nullptr, nullptr, nullptr}, wc + 3};
-        k_batch_offsets<<<1, 1024, 0, s>>>(fs, (uint32_t)n, bo);
+        launch(overlap, k_batch_offsets, 1, 1024, 0, s, fs, (uint32_t)n, bo);
     }
     LAUNCHED();
     STAGE(13);
-    k_index_quads<<<sms * std::max(1, tu.index_ctas_per_sm), 256, 0, s>>>(fs, off_peaks, (uint32_t)n, p);
+    launch(overlap, k_index_quads, sms * std::max(1, tu.index_ctas_per_sm), 256, 0, s, fs, off_peaks, (uint32_t)n, p);
     LAUNCHED();
     STAGE(14);
-    k_compact_quads<<<(unsigned)n, 1024, 0, s>>>(fs);
+    launch(overlap, k_compact_quads, (unsigned)n, 1024, 0, s, fs);
     LAUNCHED();
     STAGE(15);
     if (det->refine) {
-        k_refine_detected<<<dim3((unsigned)n, 64), 128, 0, s>>>(fs);
+        launch(overlap, k_refine_detected, dim3((unsigned)n, 64), 128, 0, s, fs);
         LAUNCHED();
     }
     STAGE(16);
 #undef STAGE
+#undef PIXEL
     return ATAG_OK;
 }
 
@@ -1053,7 +1088,7 @@ atag_status atag_detect_batch(atag_detector* det, const atag_frame* frames, size
     // stream, so it runs one lane.
     const bool timed = det->stage_events.size() == ATAG_STAGE_COUNT + 1;
     const int lanes = timed ? 1 : (int)std::min<size_t>((size_t)std::min(det->tuning.batch_lanes, MAX_LANES), n);
-    if (lanes == 1) return launch_lane(det, d_table, t, 0, n, s, 0, timed);
+    if (lanes == 1) return launch_lane(det, d_table, t, 0, n, s, 0, 1, timed);
     size_t cut[MAX_LANES + 1];
     cut[0] = 0;
     cut[lanes] = n;
@@ -1075,7 +1110,7 @@ atag_status atag_detect_batch(atag_detector* det, const atag_frame* frames, size
     CK(cudaEventRecord(det->lane_fork, s));
     for (int k = 1; k < lanes; k++) CK(cudaStreamWaitEvent(det->lane_stream[k], det->lane_fork, 0));
     for (int k = 0; k < lanes; k++) {
-        st = launch_lane(det, d_table, t, cut[k], cut[k + 1], k ? det->lane_stream[k] : s, k, false);
+        st = launch_lane(det, d_table, t, cut[k], cut[k + 1], k ? det->lane_stream[k] : s, k, lanes, false);
         if (st) return st;
     }
     for (int k = 1; k < lanes; k++) {

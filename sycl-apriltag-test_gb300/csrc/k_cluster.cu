@@ -35,6 +35,7 @@ namespace atag {
 // reset
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_reset_frames(const __grid_constant__ FrameSet fs) {
+    if (fs.overlap) await_previous_kernel();
     const FrameDesc& F = fs.get(blockIdx.y);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < F.pair_cap; i += gridDim.x * blockDim.x) {
         F.pair_keys[i] = EMPTY_KEY;
@@ -482,6 +483,7 @@ __device__ __forceinline__ void block_exclusive_scan_multi(uint32_t (&v)[K], uin
 
 __global__ void __launch_bounds__(PF_THREADS) k_pairs_finalize(const __grid_constant__ FrameSet fs,
                                                                PipelineParams p, uint32_t small_max) {
+    if (fs.overlap) await_previous_kernel();
     const FrameDesc& F = fs.get(blockIdx.x);
     uint32_t* status = F.counters + CNT_STATUS;
     __shared__ unsigned long long s_keys[PF_SMEM_KEYS];
@@ -610,6 +612,7 @@ __global__ void __launch_bounds__(PF_THREADS) k_pairs_finalize(const __grid_cons
 // Prefix offsets of per-frame counts over the batch (the flattened work
 // spaces of the per-cluster kernels) and reset of their queue cursors.
 __global__ void k_batch_offsets(const __grid_constant__ FrameSet fs, uint32_t n_frames, BatchOffsets a) {
+    if (fs.overlap) await_previous_kernel();
     __shared__ uint32_t red[33];
     for (int k = 0; k < 4; k++) {
         const uint32_t which = a.which[k];
@@ -636,6 +639,7 @@ __global__ void k_batch_offsets(const __grid_constant__ FrameSet fs, uint32_t n_
 // 3. scatter points of surviving pairs into their cluster segments
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_scatter_points(const __grid_constant__ FrameSet fs) {
+    if (fs.overlap) await_previous_kernel();
     const FrameDesc& F = fs.get(blockIdx.y);
     uint32_t n = F.counters[CNT_POINTS];
     if (n > F.point_cap) n = F.point_cap;
@@ -1146,6 +1150,7 @@ __global__ void __launch_bounds__(32 * CE_WARPS, 4) k_cluster_prefix(const __gri
 // 5. peak extents (D10-D12), do_indexing + corners, ordered quads
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) k_peaks_scan(const __grid_constant__ FrameSet fs, PipelineParams p) {
+    if (fs.overlap) await_previous_kernel();
     const FrameDesc& F = fs.get(blockIdx.x);
     __shared__ uint32_t red[33];
     const uint32_t C = F.counters[CNT_CLUSTERS];
@@ -1205,8 +1210,9 @@ __device__ __forceinline__ unsigned long long best_candidates(const unsigned lon
 // took 12 + 29 us as a kernel each with serial corners (25 now), 64 frames
 // 30 + 133 us (82 now).
 __global__ void __launch_bounds__(256) k_index_quads(const __grid_constant__ FrameSet fs,
-                                                     const uint32_t* __restrict__ work_offsets, uint32_t n_frames,
+                                                     const uint32_t* work_offsets, uint32_t n_frames,
                                                      PipelineParams p) {
+    if (fs.overlap) await_previous_kernel();
     __shared__ SegmentTable T[8];  // one per warp
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t total = work_offsets[n_frames];
@@ -1254,6 +1260,7 @@ __global__ void __launch_bounds__(256) k_index_quads(const __grid_constant__ Fra
 }
 
 __global__ void __launch_bounds__(1024) k_compact_quads(const __grid_constant__ FrameSet fs) {
+    if (fs.overlap) await_previous_kernel();
     const FrameDesc& F = fs.get(blockIdx.x);
     __shared__ uint32_t red[33];
     const uint32_t Cp = F.counters[CNT_PEAKCLU];
@@ -1283,13 +1290,19 @@ __global__ void __launch_bounds__(1024) k_compact_quads(const __grid_constant__ 
     }
 }
 
-__global__ void __launch_bounds__(BP_W / 4 * 8, 16) k_boundaries_pairs_r8(const __grid_constant__ FrameSet fs,
-                                                                       uint32_t min_size) {
-    boundaries_pairs_impl<8>(fs, min_size);
-}
-__global__ void __launch_bounds__(BP_W / 4 * 16, 8) k_boundaries_pairs_r16(const __grid_constant__ FrameSet fs,
-                                                                        uint32_t min_size) {
-    boundaries_pairs_impl<16>(fs, min_size);
-}
+#define BOUNDARY_KERNELS(SUFFIX, BEFORE)                                                                        \
+    __global__ void __launch_bounds__(BP_W / 4 * 8, 16)                                                         \
+        k_boundaries_pairs_r8##SUFFIX(const __grid_constant__ FrameSet fs, uint32_t min_size) {                 \
+        BEFORE;                                                                                                 \
+        boundaries_pairs_impl<8>(fs, min_size);                                                                 \
+    }                                                                                                           \
+    __global__ void __launch_bounds__(BP_W / 4 * 16, 8)                                                         \
+        k_boundaries_pairs_r16##SUFFIX(const __grid_constant__ FrameSet fs, uint32_t min_size) {                \
+        BEFORE;                                                                                                 \
+        boundaries_pairs_impl<16>(fs, min_size);                                                                \
+    }
+BOUNDARY_KERNELS(, )
+BOUNDARY_KERNELS(_overlapped, await_previous_kernel())
+#undef BOUNDARY_KERNELS
 
 }  // namespace atag

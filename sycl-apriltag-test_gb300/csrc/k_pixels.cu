@@ -25,6 +25,7 @@ __device__ __forceinline__ uint32_t pixel_grey(const uint8_t* p, uint32_t format
 }
 
 __global__ void k_decimate(const __grid_constant__ FrameSet fs) {
+    if (fs.overlap) await_previous_kernel();
     const FrameDesc& F = fs.get(blockIdx.y);
     if (F.factor <= 1 && F.src_format == ATAG_PIX_GREY8) return;
     const uint32_t w = F.width, h = F.height, f = F.factor, fmt = F.src_format;
@@ -51,8 +52,7 @@ __global__ void k_decimate(const __grid_constant__ FrameSet fs) {
 constexpr int TH_TX = 32, TH_TY = 16;
 constexpr int TH_EX = TH_TX + 2, TH_EY = TH_TY + 2;
 
-__global__ void __launch_bounds__(256, 8) k_threshold(const __grid_constant__ FrameSet fs,
-                                                   int min_diff, int write_extrema) {
+__device__ __forceinline__ void threshold_impl(const FrameSet& fs, int min_diff, int write_extrema) {
     const FrameDesc& F = fs.get(blockIdx.y);
     const int tw = F.width / 4, th = F.height / 4;
     const int ntx = (tw + TH_TX - 1) / TH_TX, nty = (th + TH_TY - 1) / TH_TY;
@@ -639,7 +639,7 @@ __device__ __forceinline__ void ccl_border_edges_impl(const FrameSet& fs) {
 // step, so four dependent loads are in flight at once.  The forest is final
 // here; the only concurrent writes replace a parent by its root, so any
 // value read is an ancestor.
-__global__ void __launch_bounds__(CCL_FINAL_THREADS, 2048 / CCL_FINAL_THREADS) k_ccl_final(const __grid_constant__ FrameSet fs) {
+__device__ __forceinline__ void ccl_final_impl(const FrameSet& fs) {
     // grid (block pairs of a row / CCL_FINAL_THREADS, block rows, frames):
     // the block pair from the block indices, no division
     const FrameDesc& F = fs.get(blockIdx.z);
@@ -747,13 +747,48 @@ __global__ void __launch_bounds__(256) k_boundaries_dense(const __grid_constant_
     }
 }
 
-__global__ void __launch_bounds__(CCL_BX * 8, 8) k_ccl_local_r8(const __grid_constant__ FrameSet fs) { ccl_local_impl<8, false>(fs); }
-__global__ void __launch_bounds__(CCL_BX * 16, 4) k_ccl_local_r16(const __grid_constant__ FrameSet fs) { ccl_local_impl<16, false>(fs); }
-__global__ void __launch_bounds__(CCL_BX * 32, 2) k_ccl_local_r32(const __grid_constant__ FrameSet fs) { ccl_local_impl<32, false>(fs); }
+// Each kernel of the detector's path twice: as it is, and for launches that
+// overlap the previous kernel's end (await_previous_kernel).
+#define PIXEL_KERNELS(SUFFIX, BEFORE)                                                                           \
+    __global__ void __launch_bounds__(256, 8)                                                                   \
+        k_threshold##SUFFIX(const __grid_constant__ FrameSet fs, int min_diff, int write_extrema) {             \
+        BEFORE;                                                                                                 \
+        threshold_impl(fs, min_diff, write_extrema);                                                            \
+    }                                                                                                           \
+    __global__ void __launch_bounds__(CCL_BX * 8, 8) k_ccl_local_r8##SUFFIX(const __grid_constant__ FrameSet fs) { \
+        BEFORE;                                                                                                 \
+        ccl_local_impl<8, false>(fs);                                                                           \
+    }                                                                                                           \
+    __global__ void __launch_bounds__(CCL_BX * 16, 4) k_ccl_local_r16##SUFFIX(const __grid_constant__ FrameSet fs) { \
+        BEFORE;                                                                                                 \
+        ccl_local_impl<16, false>(fs);                                                                          \
+    }                                                                                                           \
+    __global__ void __launch_bounds__(CCL_BX * 32, 2) k_ccl_local_r32##SUFFIX(const __grid_constant__ FrameSet fs) { \
+        BEFORE;                                                                                                 \
+        ccl_local_impl<32, false>(fs);                                                                          \
+    }                                                                                                           \
+    __global__ void __launch_bounds__(256) k_ccl_border_edges_r8##SUFFIX(const __grid_constant__ FrameSet fs) { \
+        BEFORE;                                                                                                 \
+        ccl_border_edges_impl<8>(fs);                                                                           \
+    }                                                                                                           \
+    __global__ void __launch_bounds__(256) k_ccl_border_edges_r16##SUFFIX(const __grid_constant__ FrameSet fs) { \
+        BEFORE;                                                                                                 \
+        ccl_border_edges_impl<16>(fs);                                                                          \
+    }                                                                                                           \
+    __global__ void __launch_bounds__(256) k_ccl_border_edges_r32##SUFFIX(const __grid_constant__ FrameSet fs) { \
+        BEFORE;                                                                                                 \
+        ccl_border_edges_impl<32>(fs);                                                                          \
+    }                                                                                                           \
+    __global__ void __launch_bounds__(CCL_FINAL_THREADS, 2048 / CCL_FINAL_THREADS)                              \
+        k_ccl_final##SUFFIX(const __grid_constant__ FrameSet fs) {                                              \
+        BEFORE;                                                                                                 \
+        ccl_final_impl(fs);                                                                                     \
+    }
+PIXEL_KERNELS(, )
+PIXEL_KERNELS(_overlapped, await_previous_kernel())
+#undef PIXEL_KERNELS
+
 __global__ void __launch_bounds__(CCL_BX * 16, 4) k_ccl_local_stage(const __grid_constant__ FrameSet fs) { ccl_local_impl<16, true>(fs); }
 __global__ void __launch_bounds__(256) k_ccl_border_r16(const __grid_constant__ FrameSet fs) { ccl_border_impl<16>(fs); }
-__global__ void __launch_bounds__(256) k_ccl_border_edges_r8(const __grid_constant__ FrameSet fs) { ccl_border_edges_impl<8>(fs); }
-__global__ void __launch_bounds__(256) k_ccl_border_edges_r16(const __grid_constant__ FrameSet fs) { ccl_border_edges_impl<16>(fs); }
-__global__ void __launch_bounds__(256) k_ccl_border_edges_r32(const __grid_constant__ FrameSet fs) { ccl_border_edges_impl<32>(fs); }
 
 }  // namespace atag

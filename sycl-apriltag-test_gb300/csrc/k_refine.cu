@@ -299,6 +299,7 @@ __global__ void __launch_bounds__(32 * RF_WARPS) k_refine_forward(const float* _
 // at most 1e-3) keeps its unrefined position.  Frame blockIdx.x; its quads
 // blockIdx.y, blockIdx.y + gridDim.y, ...
 __global__ void __launch_bounds__(32 * RF_WARPS) k_refine_detected(const __grid_constant__ FrameSet fs) {
+    if (fs.overlap) await_previous_kernel();
     __shared__ EdgeSums sums[4];
     const FrameDesc& F = fs.get(blockIdx.x);
     const uint32_t nq = min(F.stats->n_quads, F.quad_cap);
