@@ -134,7 +134,8 @@ enum Counter : uint32_t {
     CNT_SMALL = 6,       // clusters of at most CF_SMALL_CAP points
     CNT_LARGE = 7,       // larger clusters
     CNT_RUNS = 8,        // runs of up to CE_RUN points of one cluster
-    CNT_COUNT = 9
+    CNT_PAIRS = 9,       // distinct pairs (entries of the frame's key list)
+    CNT_COUNT = 10
 };
 
 constexpr uint32_t DEAD_PAIRS = 2;
@@ -160,11 +161,12 @@ struct RunInfo {
 };
 __host__ __device__ constexpr size_t max_runs(size_t points, size_t clusters) { return points / CE_RUN + clusters; }
 
-// Batch-wide prefix offsets of up to four per-frame counters.
+// Batch-wide prefix offsets of up to three per-frame counters, made by the last
+// CTA of the kernel that writes the counters.
 struct BatchOffsets {
-    uint32_t which[4];
-    uint32_t* offsets[4];      // n_frames + 1 entries each, or null
-    uint32_t* work_counters;   // one queue cursor per used entry, reset to 0
+    uint32_t which[3];
+    uint32_t* offsets[3];  // n_frames + 1 entries each, or null
+    uint32_t* ticket;      // CTAs that have finished; zero before the kernel
 };
 
 struct PipelineParams {
@@ -216,13 +218,13 @@ __global__ void k_process_quads(const atag_fitted_quad* fitted, size_t count, Pi
                                 atag_quad_corners* out, size_t cap, uint32_t* count_out);
 
 // k_cluster.cu (fused path)
-__global__ void k_reset_frames(const __grid_constant__ FrameSet fs);
+__global__ void k_reset_frames(const __grid_constant__ FrameSet fs, uint32_t* cursors, uint32_t n_cursors);
 // boundary tiles of 64 x 8 or 64 x 16 pixels
 __global__ void k_boundaries_pairs_r8(const __grid_constant__ FrameSet fs, uint32_t min_size);
 __global__ void k_boundaries_pairs_r8_overlapped(const __grid_constant__ FrameSet fs, uint32_t min_size);
 __global__ void k_boundaries_pairs_r16(const __grid_constant__ FrameSet fs, uint32_t min_size);
 __global__ void k_boundaries_pairs_r16_overlapped(const __grid_constant__ FrameSet fs, uint32_t min_size);
-__global__ void k_pairs_finalize(const __grid_constant__ FrameSet fs, PipelineParams p, uint32_t small_max);
+__global__ void k_pairs_finalize(const __grid_constant__ FrameSet fs, PipelineParams p, uint32_t small_max, BatchOffsets a);
 __global__ void k_scatter_points(const __grid_constant__ FrameSet fs);
 __global__ void k_cluster_sort_small(const __grid_constant__ FrameSet fs, const uint32_t* work_offsets,
                                      uint32_t n_frames, uint32_t* work_counter, uint32_t cap);
@@ -231,8 +233,7 @@ __global__ void k_cluster_sort_large(const __grid_constant__ FrameSet fs, const 
 __global__ void k_cluster_lines(const __grid_constant__ FrameSet fs, const uint32_t* run_offsets, uint32_t n_frames);
 constexpr uint32_t CE_LINES_SMEM = 4 * 12432;  // four warps' RunSums
 __global__ void k_cluster_prefix(const __grid_constant__ FrameSet fs, const uint32_t* run_offsets);
-__global__ void k_peaks_scan(const __grid_constant__ FrameSet fs, PipelineParams p);
-__global__ void k_batch_offsets(const __grid_constant__ FrameSet fs, uint32_t n_frames, BatchOffsets a);
+__global__ void k_peaks_scan(const __grid_constant__ FrameSet fs, BatchOffsets a);
 __global__ void k_index_quads(const __grid_constant__ FrameSet fs, const uint32_t* work_offsets, uint32_t n_frames,
                               PipelineParams p);
 __global__ void k_compact_quads(const __grid_constant__ FrameSet fs);

@@ -33,9 +33,14 @@ __device__ __forceinline__ uint32_t global_lookup(const FrameDesc& F, unsigned l
     }
     return INVALID;
 }
-__device__ __forceinline__ uint32_t global_flush(const FrameDesc& F, uint32_t gs, uint32_t cnt, uint32_t xmin,
-                                                 uint32_t xmax, uint32_t ymin, uint32_t ymax, int gx, int gy,
-                                                 unsigned long long pxgx) {
+
+// Merge cnt > 0 points of a key into its slot.  The first merge also appends
+// the key to the frame's list of distinct keys, unsorted, in the part of
+// cluster_keys behind the clusters' own (k_pairs_finalize reads CNT_PAIRS of
+// it instead of scanning the table).
+__device__ __forceinline__ uint32_t global_flush(const FrameDesc& F, unsigned long long key, uint32_t gs,
+                                                 uint32_t cnt, uint32_t xmin, uint32_t xmax, uint32_t ymin,
+                                                 uint32_t ymax, int gx, int gy, unsigned long long pxgx) {
     uint32_t old = atomicAdd(&F.pair_count[gs], cnt);
     uint32_t* bb = reinterpret_cast<uint32_t*>(&F.pair_bbox[gs]);
     atomicMin(bb + 0, xmin);
@@ -46,6 +51,7 @@ __device__ __forceinline__ uint32_t global_flush(const FrameDesc& F, uint32_t gs
     if (gx) atomicAdd(gsum + 0, gx);
     if (gy) atomicAdd(gsum + 1, gy);
     if (pxgx) atomicAdd(&F.pair_pxgx[gs], pxgx);
+    if (old == 0) F.cluster_keys[F.cluster_cap + atomicAdd(F.counters + CNT_PAIRS, 1u)] = key;
     return old;
 }
 

@@ -310,7 +310,7 @@ struct atag_detector {
     // header carve-out
     FrameDesc* d_tables = nullptr;   // RING x max_frames
     FrameDesc* d_captured = nullptr; // CAPTURE_SLOTS x max_frames: tables of captured calls
-    uint32_t* d_work = nullptr;      // per lane: offsets (WORK_LISTS x (max_frames + 1)) + WORK_LISTS counters
+    uint32_t* d_work = nullptr;      // per lane: offsets (WORK_LISTS x (max_frames + 1)) + WORK_LISTS cursors and tickets
     cudaStream_t lane_stream[MAX_LANES] = {};    // streams of lanes 1.. (lane 0 runs on the caller's)
     cudaStream_t side[MAX_LANES] = {};           // per lane: stream of the large-cluster kernel
     cudaEvent_t fork[MAX_LANES] = {}, join[MAX_LANES] = {};
@@ -608,17 +608,13 @@ atag_status atag_cluster(const atag_boundary_point* points, const uint64_t* keys
     atag_config c;
     atag_config_default(&c);
     const PipelineParams p = make_params(c);
-    k_reset_frames<<<grid2(cdiv(d.pair_cap, 256), 1), 256, 0, s>>>(fs);
+    k_reset_frames<<<grid2(cdiv(d.pair_cap, 256), 1), 256, 0, s>>>(fs, wc, 3);
     LAUNCHED();
     k_planes_pairs<<<(unsigned)std::min<size_t>(cdiv(n, 256), (size_t)sms * 8), 256, 0, s>>>(
         fs, reinterpret_cast<const uint32_t*>(points), reinterpret_cast<const unsigned long long*>(keys), n);
     LAUNCHED();
-    k_pairs_finalize<<<1, 1024, 0, s>>>(fs, p, CF_SMALL_CAP);
-    LAUNCHED();
-    {
-        BatchOffsets bo{{CNT_SMALL, CNT_LARGE, CNT_RUNS, 0}, {off_small, off_large, off_runs, nullptr}, wc};
-        k_batch_offsets<<<1, 1024, 0, s>>>(fs, 1, bo);
-    }
+    const BatchOffsets lists{{CNT_SMALL, CNT_LARGE, CNT_RUNS}, {off_small, off_large, off_runs}, wc + 2};
+    k_pairs_finalize<<<1, 1024, 0, s>>>(fs, p, CF_SMALL_CAP, lists);
     LAUNCHED();
     k_planes_scatter<<<(unsigned)std::min<size_t>(cdiv(n, 256), (size_t)sms * 8), 256, 0, s>>>(
         fs, reinterpret_cast<const uint32_t*>(points), reinterpret_cast<const unsigned long long*>(keys), n);
@@ -919,7 +915,8 @@ static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, con
     const PipelineParams& p = det->pp;
     const int sms = det->dev->num_sms;
     // batch-wide work lists of this lane: small clusters, large clusters,
-    // point runs, clusters with peaks; one queue cursor each
+    // point runs, clusters with peaks; then the two sorts' queue cursors and the
+    // tickets of the kernels that make the lists
     uint32_t* work = det->d_work + (size_t)lane * (WORK_LISTS * (det->max_frames + 1) + WORK_LISTS);
     uint32_t* off_small = work;
     uint32_t* off_large = work + (n + 1);
@@ -951,7 +948,7 @@ static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, con
     fs.overlap = overlap ? 1u : 0u;
 #define PIXEL(k) (overlap ? k##_overlapped : k)
     STAGE(0);
-    k_reset_frames<<<grid2(cdiv(max_pair, 256), n), 256, 0, s>>>(fs);
+    k_reset_frames<<<grid2(cdiv(max_pair, 256), n), 256, 0, s>>>(fs, wc, (uint32_t)WORK_LISTS);
     LAUNCHED();
     STAGE(1);
     if (any_decim) {
@@ -986,12 +983,8 @@ static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, con
         launch(overlap, PIXEL(k_boundaries_pairs_r16), dim3((unsigned)n, (unsigned)cdiv(mw, 64), (unsigned)cdiv(mh, 16)), 16 * 16, 0, s, fs, p.min_component_size);
     LAUNCHED();
     STAGE(7);
-    launch(overlap, k_pairs_finalize, (unsigned)n, 1024, 0, s, fs, p, (uint32_t)tu.small_cluster_max);
-    LAUNCHED();
-    {
-        BatchOffsets bo{{CNT_SMALL, CNT_LARGE, CNT_RUNS, 0}, {off_small, off_large, off_runs, nullptr}, wc};
-        launch(overlap, k_batch_offsets, 1, 1024, 0, s, fs, (uint32_t)n, bo);
-    }
+    const BatchOffsets lists{{CNT_SMALL, CNT_LARGE, CNT_RUNS}, {off_small, off_large, off_runs}, wc + 2};
+    launch(overlap, k_pairs_finalize, (unsigned)n, 1024, 0, s, fs, p, (uint32_t)tu.small_cluster_max, lists);
     LAUNCHED();
     STAGE(8);
     launch(overlap, k_scatter_points, grid2(std::min<size_t>(cdiv(max_points, 256), 1024), n), 256, 0, s, fs);
@@ -1016,12 +1009,8 @@ static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, con
     LAUNCHED();
     STAGE(11);
     STAGE(12);
-    launch(overlap, k_peaks_scan, (unsigned)n, 1024, 0, s, fs, p);
-    LAUNCHED();
-    {
-        BatchOffsets bo{{CNT_PEAKCLU, 0, 0, 0}, {off_peaks, nullptr, nullptr, nullptr}, wc + 3};
-        launch(overlap, k_batch_offsets, 1, 1024, 0, s, fs, (uint32_t)n, bo);
-    }
+    const BatchOffsets with_peaks{{CNT_PEAKCLU, 0, 0}, {off_peaks, nullptr, nullptr}, wc + 3};
+    launch(overlap, k_peaks_scan, (unsigned)n, 1024, 0, s, fs, with_peaks);
     LAUNCHED();
     STAGE(13);
     launch(overlap, k_index_quads, sms * std::max(1, tu.index_ctas_per_sm), 256, 0, s, fs, off_peaks, (uint32_t)n, p);

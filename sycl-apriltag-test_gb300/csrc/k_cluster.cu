@@ -34,8 +34,10 @@ namespace atag {
 // ---------------------------------------------------------------------------
 // reset
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_reset_frames(const __grid_constant__ FrameSet fs) {
+__global__ void __launch_bounds__(256) k_reset_frames(const __grid_constant__ FrameSet fs, uint32_t* cursors,
+                                                      uint32_t n_cursors) {
     if (fs.overlap) await_previous_kernel();
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < n_cursors) cursors[threadIdx.x] = 0u;
     const FrameDesc& F = fs.get(blockIdx.y);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < F.pair_cap; i += gridDim.x * blockDim.x) {
         F.pair_keys[i] = EMPTY_KEY;
@@ -360,7 +362,7 @@ __device__ __forceinline__ void boundaries_pairs_impl(const FrameSet& fs, uint32
                         atomicOr(status, ATAG_DEVFLAG_PAIR_OVERFLOW);
                     } else {
                         const int g = dir ? 1 : -1;
-                        global_flush(F, gs, 1, xd, xd, yd, yd, g, 0, (unsigned long long)(long long)((int)xd * g));
+                        global_flush(F, key, gs, 1, xd, xd, yd, yd, g, 0, (unsigned long long)(long long)((int)xd * g));
                         const uint32_t at = atomicAdd(F.counters + CNT_POINTS, 1u);
                         if (at < F.point_cap) F.points[at] = ((unsigned long long)gs << 32) | stage_packed(e, x0, y0);
                         else atomicOr(status, ATAG_DEVFLAG_POINT_OVERFLOW);
@@ -384,7 +386,7 @@ __device__ __forceinline__ void boundaries_pairs_impl(const FrameSet& fs, uint32
         if (key == EMPTY_KEY) continue;
         const uint32_t gs = T.gslot[i];  // INVALID: the frame's table was full (flagged)
         if (gs == INVALID) continue;
-        uint32_t old = global_flush(F, gs, T.cnt[i], T.xmin[i], T.xmax[i], T.ymin[i], T.ymax[i], T.gx[i], 0,
+        uint32_t old = global_flush(F, key, gs, T.cnt[i], T.xmin[i], T.xmax[i], T.ymin[i], T.ymax[i], T.gx[i], 0,
                                     (unsigned long long)(long long)T.pxgx[i]);
         T.gslot[i] = (old + T.cnt[i] > max_pixels) ? INVALID : gs;
         // the flush that crosses the limit publishes the pair, so that later
@@ -481,30 +483,132 @@ __device__ __forceinline__ void block_exclusive_scan_multi(uint32_t (&v)[K], uin
     }
 }
 
+// Ascending sort of n <= 1024 E keys at src into dst (shared memory, 1024 E
+// words) by a CTA of 1024 threads: the flip form of the bitonic network with E
+// keys a thread in registers.  Partners up to 32 E positions apart are in the
+// thread or its warp; only the others go through shared memory and barriers
+// (10 of 45 steps for 512 keys).
+template <int E>
+__device__ __forceinline__ void sort_keys(const unsigned long long* src, unsigned long long* dst, uint32_t n) {
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    const uint32_t t = threadIdx.x;
+    unsigned long long k[E];
+#pragma unroll
+    for (int e = 0; e < E; e++) k[e] = t * E + e < n ? src[t * E + e] : ~0ull;
+    uint32_t lg = 0;
+    while ((1u << lg) < n) lg++;
+    const bool act = (t & ~31u) * E < n;  // warps of padding only keep the barriers
+    for (uint32_t lk = 1; lk <= lg; lk++) {
+        for (int lj = (int)lk - 1; lj >= 0; lj--) {
+            // position i meets i ^ m; the one without bit lj keeps the smaller
+            const bool flip = lj == (int)lk - 1;
+            const uint32_t m = flip ? (1u << lk) - 1u : 1u << lj, mt = m / E;
+            auto order = [&](unsigned long long& a, unsigned long long& b) {
+                const unsigned long long lo = a < b ? a : b, hi = a < b ? b : a;
+                a = lo;
+                b = hi;
+            };
+            if (m < E) {
+                if constexpr (E == 2) order(k[0], k[1]);
+                if constexpr (E == 4) {
+                    if (m == 1) order(k[0], k[1]), order(k[2], k[3]);
+                    else if (m == 2) order(k[0], k[2]), order(k[1], k[3]);
+                    else order(k[0], k[3]), order(k[1], k[2]);
+                }
+                continue;
+            }
+            unsigned long long o[E];
+            if (mt < 32) {
+                if (!act) continue;
+#pragma unroll
+                for (int e = 0; e < E; e++) o[e] = __shfl_xor_sync(FULL, k[e], (int)mt);
+            } else {
+                if (act)
+#pragma unroll
+                    for (int e = 0; e < E; e++) dst[e * 1024 + t] = k[e];
+                __syncthreads();
+                if (act)
+#pragma unroll
+                    for (int e = 0; e < E; e++) o[e] = (t ^ mt) * E < n ? dst[e * 1024 + (t ^ mt)] : ~0ull;
+                __syncthreads();
+                if (!act) continue;
+            }
+            const bool upper = ((t * E) >> lj) & 1u;
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                const unsigned long long v = flip ? o[E - 1 - e] : o[e];
+                k[e] = (v < k[e]) != upper ? v : k[e];
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < E; e++)
+        if (t * E + e < n) dst[t * E + e] = k[e];
+    __syncthreads();
+}
+
+// The end of a kernel of one CTA per frame: the CTA that finishes last makes
+// the prefix offsets of the per-frame counters over the batch (the flattened
+// work spaces of the per-cluster kernels), a warp per list.
+__device__ __forceinline__ void batch_offsets(const FrameSet& fs, const BatchOffsets& a) {
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    const uint32_t n_frames = gridDim.x, lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();  // this thread wrote the frame's counters
+        last = n_frames == 1 || atomicAdd(a.ticket, 1u) == n_frames - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!last || k >= 3) return;
+    uint32_t* offsets = k == 0 ? a.offsets[0] : (k == 1 ? a.offsets[1] : a.offsets[2]);
+    const uint32_t which = k == 0 ? a.which[0] : (k == 1 ? a.which[1] : a.which[2]);
+    if (!offsets) return;
+    uint32_t carry = 0;
+    for (uint32_t f0 = 0; f0 < n_frames; f0 += 32) {
+        const uint32_t f = f0 + lane, v = f < n_frames ? __ldcg(fs.get(f).counters + which) : 0u;
+        uint32_t x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, x, o);
+            if (lane >= (uint32_t)o) x += y;
+        }
+        if (f < n_frames) offsets[f] = carry + x - v;
+        carry += __shfl_sync(FULL, x, 31);
+    }
+    if (lane == 0) offsets[n_frames] = carry;
+}
+
+// One CTA per frame, bound by the latency of its serial steps: reading the key
+// list instead of counting and gathering the table's used slots, the sort in
+// registers and the batch's work lists made here took a lone 1080p frame's 333
+// keys from 28 to 21 us and a 4K frame's 1254 from 56 to 36 (with the list
+// kernel that followed).
 __global__ void __launch_bounds__(PF_THREADS) k_pairs_finalize(const __grid_constant__ FrameSet fs,
-                                                               PipelineParams p, uint32_t small_max) {
+                                                               PipelineParams p, uint32_t small_max,
+                                                               BatchOffsets a) {
     if (fs.overlap) await_previous_kernel();
     const FrameDesc& F = fs.get(blockIdx.x);
     uint32_t* status = F.counters + CNT_STATUS;
     __shared__ unsigned long long s_keys[PF_SMEM_KEYS];
     __shared__ uint32_t red4[4][33];
-    uint32_t* red = red4[0];
-    __shared__ uint32_t s_n;
-    if (threadIdx.x == 0) s_n = 0;
-    __syncthreads();
-    // the sorted key list lives in shared memory when it fits, else in the
-    // frame's cluster_keys buffer's tail (pair_cap entries reserved there)
-    uint32_t npairs_upper = 0;
-    for (uint32_t i = threadIdx.x; i < F.pair_cap; i += blockDim.x) npairs_upper += F.pair_keys[i] != EMPTY_KEY;
-    uint32_t C = block_sum_u32(npairs_upper, red);
-    unsigned long long* keys = C <= (uint32_t)PF_SMEM_KEYS ? s_keys : F.cluster_keys + F.cluster_cap;
-    for (uint32_t i = threadIdx.x; i < F.pair_cap; i += blockDim.x) {
-        unsigned long long k = F.pair_keys[i];
-        if (k != EMPTY_KEY) keys[atomicAdd(&s_n, 1u)] = k;
+    // the frame's distinct keys, listed in any order: sorted in shared memory
+    // when they fit, else in place
+    const uint32_t C = F.counters[CNT_PAIRS];
+    unsigned long long* list = F.cluster_keys + F.cluster_cap;
+    unsigned long long* keys = C <= (uint32_t)PF_SMEM_KEYS ? s_keys : list;
+    if (C <= 1024u) sort_keys<1>(list, s_keys, C);
+    else if (C <= 2048u) sort_keys<2>(list, s_keys, C);
+    else if (C <= 4096u) sort_keys<4>(list, s_keys, C);
+    else {
+        if (keys == s_keys)
+            for (uint32_t i = threadIdx.x; i < C; i += blockDim.x) keys[i] = list[i];
+        __syncthreads();
+        bitonic_sort_u64(keys, C);
+        __syncthreads();
     }
-    __syncthreads();
-    bitonic_sort_u64(keys, C);
-    __syncthreads();
     FilterParams fp;
     fp.min_cluster_pixels = p.min_cluster_pixels;
     fp.max_cluster_pixels = 2u * (2u * F.width + 2u * F.height);
@@ -607,32 +711,7 @@ __global__ void __launch_bounds__(PF_THREADS) k_pairs_finalize(const __grid_cons
         F.stats->n_clusters = nfit;
         F.stats->n_cluster_points = carry_fit;
     }
-}
-
-// Prefix offsets of per-frame counts over the batch (the flattened work
-// spaces of the per-cluster kernels) and reset of their queue cursors.
-__global__ void k_batch_offsets(const __grid_constant__ FrameSet fs, uint32_t n_frames, BatchOffsets a) {
-    if (fs.overlap) await_previous_kernel();
-    __shared__ uint32_t red[33];
-    for (int k = 0; k < 4; k++) {
-        const uint32_t which = a.which[k];
-        uint32_t* offsets = a.offsets[k];
-        uint32_t* work_counters = a.work_counters;
-        if (!offsets) continue;
-        uint32_t carry = 0;
-        for (uint32_t f0 = 0; f0 < n_frames; f0 += blockDim.x) {
-            uint32_t f = f0 + threadIdx.x;
-            uint32_t v = f < n_frames ? fs.get(f).counters[which] : 0u;
-            uint32_t tot;
-            uint32_t e = block_exclusive_scan_u32(v, red, &tot);
-            if (f < n_frames) offsets[f] = carry + e;
-            carry += tot;
-        }
-        if (threadIdx.x == 0) {
-            offsets[n_frames] = carry;
-            work_counters[k] = 0;
-        }
-    }
+    batch_offsets(fs, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -1149,7 +1228,7 @@ __global__ void __launch_bounds__(32 * CE_WARPS, 4) k_cluster_prefix(const __gri
 // ---------------------------------------------------------------------------
 // 5. peak extents (D10-D12), do_indexing + corners, ordered quads
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) k_peaks_scan(const __grid_constant__ FrameSet fs, PipelineParams p) {
+__global__ void __launch_bounds__(1024) k_peaks_scan(const __grid_constant__ FrameSet fs, BatchOffsets a) {
     if (fs.overlap) await_previous_kernel();
     const FrameDesc& F = fs.get(blockIdx.x);
     __shared__ uint32_t red[33];
@@ -1173,6 +1252,7 @@ __global__ void __launch_bounds__(1024) k_peaks_scan(const __grid_constant__ Fra
         F.stats->n_corners = carry_k;
         F.stats->n_peak_clusters = carry_q;
     }
+    batch_offsets(fs, a);
 }
 
 // The 10 best corner candidates of a cluster by (error desc, index asc), one

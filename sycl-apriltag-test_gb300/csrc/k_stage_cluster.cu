@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(256) k_planes_pairs(const __grid_constant__ Fr
         if (v && (int)lane == leader) {
             const uint32_t gs = global_insert(F, key);
             if (gs == INVALID) atomicOr(status, ATAG_DEVFLAG_PAIR_OVERFLOW);
-            else global_flush(F, gs, (uint32_t)__popc(m), xmn, xmx, ymn, ymx, sgx, sgy,
+            else global_flush(F, key, gs, (uint32_t)__popc(m), xmn, xmx, ymn, ymx, sgx, sgy,
                               (unsigned long long)(long long)spx);
         }
     }
