@@ -214,6 +214,7 @@ __global__ void k_fit_lines_windowed(const atag_line_fit_point* points, const ui
 __global__ void k_do_indexing(const atag_peak_extents* extents, size_t count, const atag_corner* corners,
                               const atag_line_fit_point* points, const atag_cluster_extents* cluster_extents,
                               float max_mse, float cos_critical, atag_fitted_quad* fitted);
+constexpr uint32_t PQ_CTAS = 8;  // blocks of k_process_quads, one cluster
 __global__ void k_process_quads(const atag_fitted_quad* fitted, size_t count, PipelineParams p,
                                 atag_quad_corners* out, size_t cap, uint32_t* count_out);
 

@@ -546,7 +546,7 @@ atag_status atag_process_fitted_quads(const atag_fitted_quad* fitted, size_t cou
     if (!d_count || (count && (!fitted || !quads))) return fail(ATAG_ERR_INVALID_ARGUMENT, "process_fitted_quads: null pointer");
     atag_config c;
     if (cfg) c = *cfg; else atag_config_default(&c);
-    k_process_quads<<<1, 1024, 0, (cudaStream_t)stream>>>(fitted, count, make_params(c), quads, cap, d_count);
+    k_process_quads<<<PQ_CTAS, 128, 0, (cudaStream_t)stream>>>(fitted, count, make_params(c), quads, cap, d_count);
     LAUNCHED();
     return ATAG_OK;
 }
@@ -663,12 +663,12 @@ atag_status atag_corner_peaks(const atag_corner* found, const atag_cluster_exten
     const uint32_t ccap = (uint32_t)std::min<size_t>(corner_cap, 0xFFFFFFFFu);
     const uint32_t ecap = (uint32_t)std::min<size_t>(extents_cap, 0xFFFFFFFFu);
     const int sms = dev->num_sms;
-    k_peaks_count<<<(unsigned)std::min<size_t>(cdiv(nc, 8), (size_t)sms * 8), 256, 0, s>>>(found, extents, nc, counts);
+    k_peaks_count<<<(unsigned)std::min<size_t>(nc, (size_t)sms * 2), 1024, 0, s>>>(found, extents, nc, counts);
     LAUNCHED();
     k_peaks_offsets<<<1, 1024, 0, s>>>(counts, nc, offsets, peak_extents, ecap, ccap, d_counts);
     LAUNCHED();
-    k_peaks_sort<<<(unsigned)std::min<size_t>(nc, (size_t)sms * 2), 256, PK_SMEM, s>>>(found, extents, nc, counts,
-                                                                                        offsets, out, ccap, d_counts);
+    k_peaks_sort<<<(unsigned)std::min<size_t>(nc, (size_t)sms), 1024, PK_SMEM, s>>>(found, extents, nc, counts,
+                                                                                     offsets, out, ccap, d_counts);
     LAUNCHED();
     return ATAG_OK;
 }

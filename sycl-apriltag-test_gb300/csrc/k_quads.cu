@@ -1,5 +1,7 @@
 // k_quads.cu — drop-in kernels for the reference's fit_lines and do_indexing,
 // and the corner intersection of process_fitted_quads moved to the device.
+#include <cooperative_groups.h>
+
 #include "atag_kernels.cuh"
 #include "atag_quads.cuh"
 
@@ -96,18 +98,25 @@ __global__ void __launch_bounds__(128) k_do_indexing(const atag_peak_extents* __
 }
 
 // ---------------------------------------------------------------------------
-// process_fitted_quads (main.cpp:1035-1162) up to tag decoding, on one CTA
-// with an ordered compaction: eight lanes per quad, for the latency of one
-// quad's FP64 chain is what it takes.
+// process_fitted_quads (main.cpp:1035-1162) up to tag decoding, on one cluster
+// of PQ_CTAS thread blocks: eight lanes per quad, and an ordered compaction
+// that reads the other blocks' counts from their shared memory.  Bound by the
+// FP64 chain of a quad (lines, corners, lengths, angles), which one block's SM
+// runs for few quads at a time: 65 quads took 38 us on one block with a thread
+// each, 28 with eight lanes each, 11 on the cluster.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) k_process_quads(const atag_fitted_quad* __restrict__ fitted, size_t count,
-                                                        PipelineParams p, atag_quad_corners* __restrict__ out,
-                                                        size_t cap, uint32_t* __restrict__ count_out) {
-    __shared__ uint32_t red[33];
-    const uint32_t g = threadIdx.x & 7;
-    uint32_t base = 0;
-    for (size_t c0 = 0; c0 < count; c0 += 128) {
-        const size_t i = c0 + (threadIdx.x >> 3);
+__global__ void __cluster_dims__(PQ_CTAS, 1, 1) __launch_bounds__(128)
+    k_process_quads(const atag_fitted_quad* __restrict__ fitted, size_t count, PipelineParams p,
+                    atag_quad_corners* __restrict__ out, size_t cap, uint32_t* __restrict__ count_out) {
+    constexpr uint32_t PER = 16;  // quads of a block and round
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    namespace cg = cooperative_groups;
+    cg::cluster_group blocks = cg::this_cluster();
+    __shared__ uint32_t ok_mask[2];  // by round parity: which of the block's quads stand
+    const uint32_t g = threadIdx.x & 7, local = threadIdx.x >> 3, rank = blocks.block_rank(), lane = threadIdx.x & 31;
+    uint32_t base = 0, round = 0;
+    for (size_t c0 = 0; c0 < count; c0 += PQ_CTAS * PER, round ^= 1) {
+        const size_t i = c0 + rank * PER + local;
         float line[4] = {0.0f, 0.0f, 0.0f, 0.0f}, cx, cy, e, mse;
         bool any = false;
         if (i < count) {
@@ -116,9 +125,17 @@ __global__ void __launch_bounds__(1024) k_process_quads(const atag_fitted_quad* 
             if (any && g < 4) fit_line(load_moment(&fq.moments[g]), fq.num_in_moments[g], line, &e, &mse);
         }
         const bool ok = quad_corners8(line, p, cx, cy) && any;
-        uint32_t total;
-        const uint32_t pos = block_exclusive_scan_u32(ok && g == 0 ? 1u : 0u, red, &total);
-        const uint32_t at = base + __shfl_sync(0xFFFFFFFFu, pos, (int)(threadIdx.x & 31) & ~7);
+        if (threadIdx.x == 0) ok_mask[round] = 0;
+        __syncthreads();
+        if (ok && g == 0) atomicOr(&ok_mask[round], 1u << local);
+        // the masks of all blocks; this round's are rewritten two rounds on,
+        // after every block has passed the next round's barrier
+        blocks.sync();
+        const uint32_t mask = lane < PQ_CTAS ? *blocks.map_shared_rank(&ok_mask[round], lane) : 0u;
+        const uint32_t n = (uint32_t)__popc(mask);
+        const uint32_t before = __reduce_add_sync(FULL, lane < rank ? n : 0u), total = __reduce_add_sync(FULL, n);
+        const uint32_t mine = __shfl_sync(FULL, mask, (int)rank);
+        const size_t at = (size_t)base + before + (uint32_t)__popc(mine & ((1u << local) - 1u));
         if (ok && at < cap) {
             atag_quad_corners& qc = out[at];
             if (g < 4) {
@@ -132,7 +149,8 @@ __global__ void __launch_bounds__(1024) k_process_quads(const atag_fitted_quad* 
         }
         base += total;
     }
-    if (threadIdx.x == 0) *count_out = base < cap ? base : (uint32_t)cap;
+    if (rank == 0 && threadIdx.x == 0) *count_out = base < cap ? base : (uint32_t)cap;
+    blocks.sync();  // no block leaves while another may read its masks
 }
 
 }  // namespace atag

@@ -14,75 +14,191 @@
 
 namespace atag {
 
+// The planes are read in groups of PP_GROUP entries per warp, PP_UNROLL of
+// them at once so that their loads are in flight together.
+constexpr uint32_t PP_UNROLL = 4, PP_GROUP = 32 * PP_UNROLL;
+constexpr uint32_t PP_LC = 32;  // pair table of a CTA; more pairs go straight to the frame's
+
+struct PlanePairs {
+    unsigned long long key[PP_LC], pxgx[PP_LC];
+    uint32_t cnt[PP_LC], xmin[PP_LC], xmax[PP_LC], ymin[PP_LC], ymax[PP_LC];
+    int gx[PP_LC], gy[PP_LC];
+};
+
+__device__ __forceinline__ int plane_pairs_insert(PlanePairs& T, unsigned long long key) {
+    uint32_t h = hash_key(key) & (PP_LC - 1);
+    for (uint32_t p = 0; p < PP_LC; p++) {
+        const unsigned long long k = atomicCAS(&T.key[h], EMPTY_KEY, key);
+        if (k == EMPTY_KEY || k == key) return (int)h;
+        h = (h + 1) & (PP_LC - 1);
+    }
+    return -1;
+}
+
 // Stages 4 and 6: copy_if(point != 0) and reduce_by_segment of
 // ClusterBounds::inital_from_point per pair key (cluster_bounds.h:27-45).
 // The sort by key that separates them in the reference only orders the
-// pairs, which k_pairs_finalize does on the distinct keys.  A warp first
-// merges the entries that share a key (match_any), then one lane adds the
-// sums to the pair's slot of the frame's hash table.
+// pairs, which k_pairs_finalize does on the distinct keys.  A CTA takes one
+// stretch of the planes; a warp keeps the sums of one pair in registers, a
+// point per lane, while its entries are of that pair, then adds them to the
+// CTA's table, which goes to the frame's at the end.  Most points of a frame
+// are of the pair of its two largest components: merged per warp and entry
+// group into the frame's table, their atomics on one slot took 277 us for
+// 1292 x 964 (30 now).
 __global__ void __launch_bounds__(256) k_planes_pairs(const __grid_constant__ FrameSet fs,
                                                       const uint32_t* __restrict__ points,
                                                       const unsigned long long* __restrict__ keys, uint32_t n) {
+    constexpr unsigned FULL = 0xFFFFFFFFu;
     const FrameDesc& F = fs.get(0);
     uint32_t* status = F.counters + CNT_STATUS;
-    const uint32_t lane = threadIdx.x & 31;
-    uint32_t found = 0;
-    // warp-uniform trip count: every lane takes part in the warp collectives
-    for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += gridDim.x * blockDim.x) {
-        const uint32_t i = base + lane;
-        const uint32_t p = i < n ? __ldg(points + i) : 0u;
-        const bool v = p != 0u;
-        if (!__any_sync(0xFFFFFFFFu, v)) continue;
-        const unsigned long long key = v ? __ldg(keys + i) : EMPTY_KEY;
-        found += v ? 1u : 0u;
-        const unsigned m = __match_any_sync(0xFFFFFFFFu, key);
-        const int leader = __ffs(m) - 1;
-        const uint32_t xd = bp_xd(p), yd = bp_yd(p);
-        const int gx = bp_gx(p), gy = bp_gy(p);
-        const uint32_t xmn = __reduce_min_sync(m, xd), xmx = __reduce_max_sync(m, xd);
-        const uint32_t ymn = __reduce_min_sync(m, yd), ymx = __reduce_max_sync(m, yd);
-        const int sgx = __reduce_add_sync(m, gx), sgy = __reduce_add_sync(m, gy);
-        const int spx = __reduce_add_sync(m, (int)xd * gx + (int)yd * gy);
-        if (v && (int)lane == leader) {
-            const uint32_t gs = global_insert(F, key);
-            if (gs == INVALID) atomicOr(status, ATAG_DEVFLAG_PAIR_OVERFLOW);
-            else global_flush(F, key, gs, (uint32_t)__popc(m), xmn, xmx, ymn, ymx, sgx, sgy,
-                              (unsigned long long)(long long)spx);
+    __shared__ PlanePairs T;
+    for (uint32_t i = threadIdx.x; i < PP_LC; i += blockDim.x) {
+        T.key[i] = EMPTY_KEY;
+        T.pxgx[i] = 0ull;
+        T.cnt[i] = T.xmax[i] = T.ymax[i] = 0u;
+        T.xmin[i] = T.ymin[i] = FULL;
+        T.gx[i] = T.gy[i] = 0;
+    }
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    unsigned long long cur = EMPTY_KEY;
+    uint32_t cnt = 0, xmn = FULL, xmx = 0, ymn = FULL, ymx = 0, found = 0;
+    int gx = 0, gy = 0, px = 0;
+    auto to_frame = [&](unsigned long long key, uint32_t c, uint32_t x0, uint32_t x1, uint32_t y0, uint32_t y1, int sx,
+                        int sy, unsigned long long sp) {
+        const uint32_t gs = global_insert(F, key);
+        if (gs == INVALID) atomicOr(status, ATAG_DEVFLAG_PAIR_OVERFLOW);
+        else global_flush(F, key, gs, c, x0, x1, y0, y1, sx, sy, sp);
+    };
+    auto flush = [&]() {
+        if (cnt == 0) return;
+        const uint32_t x0 = __reduce_min_sync(FULL, xmn), x1 = __reduce_max_sync(FULL, xmx);
+        const uint32_t y0 = __reduce_min_sync(FULL, ymn), y1 = __reduce_max_sync(FULL, ymx);
+        const int sx = __reduce_add_sync(FULL, gx), sy = __reduce_add_sync(FULL, gy), sp = __reduce_add_sync(FULL, px);
+        if (lane != 0) return;
+        const unsigned long long spx = (unsigned long long)(long long)sp;
+        const int t = plane_pairs_insert(T, cur);
+        if (t < 0) {
+            to_frame(cur, cnt, x0, x1, y0, y1, sx, sy, spx);
+            return;
+        }
+        atomicAdd(&T.cnt[t], cnt);
+        atomicMin(&T.xmin[t], x0);
+        atomicMax(&T.xmax[t], x1);
+        atomicMin(&T.ymin[t], y0);
+        atomicMax(&T.ymax[t], y1);
+        atomicAdd(&T.gx[t], sx);
+        atomicAdd(&T.gy[t], sy);
+        atomicAdd(&T.pxgx[t], spx);
+    };
+    const uint32_t groups = (n + PP_GROUP - 1) / PP_GROUP, per = (groups + gridDim.x - 1) / gridDim.x;
+    const uint32_t g0 = blockIdx.x * per, g1 = min(groups, g0 + per);
+    for (uint32_t g = g0 + (threadIdx.x >> 5); g < g1; g += warps) {
+        uint32_t p[PP_UNROLL];
+        unsigned long long k[PP_UNROLL];
+#pragma unroll
+        for (uint32_t u = 0; u < PP_UNROLL; u++) {
+            const uint32_t i = g * PP_GROUP + 32 * u + lane;
+            p[u] = i < n ? __ldg(points + i) : 0u;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < PP_UNROLL; u++)
+            k[u] = p[u] ? __ldg(keys + (g * PP_GROUP + 32 * u + lane)) : EMPTY_KEY;
+#pragma unroll
+        for (uint32_t u = 0; u < PP_UNROLL; u++) {
+            const bool v = p[u] != 0u;
+            unsigned pend = __ballot_sync(FULL, v);
+            if (!pend) continue;
+            found += (uint32_t)__popc(pend);
+            const uint32_t xd = bp_xd(p[u]), yd = bp_yd(p[u]);
+            const int dx = bp_gx(p[u]), dy = bp_gy(p[u]);
+            // the current pair's points first, so that it is left once
+            unsigned m = __ballot_sync(FULL, v && k[u] == cur);
+            while (true) {
+                if (m) {
+                    pend &= ~m;
+                    cnt += (uint32_t)__popc(m);
+                    if ((m >> lane) & 1u) {
+                        xmn = min(xmn, xd);
+                        xmx = max(xmx, xd);
+                        ymn = min(ymn, yd);
+                        ymx = max(ymx, yd);
+                        gx += dx;
+                        gy += dy;
+                        px += (int)xd * dx + (int)yd * dy;
+                    }
+                }
+                // (a lane's and a warp's sums of up to 16384 points fit 32 bits)
+                if (!pend && cnt < 16384u - 32u) break;
+                flush();
+                if (pend) cur = __shfl_sync(FULL, k[u], __ffs(pend) - 1);
+                cnt = xmx = ymx = 0;
+                xmn = ymn = FULL;
+                gx = gy = px = 0;
+                if (!pend) break;
+                m = __ballot_sync(FULL, v && k[u] == cur);
+            }
         }
     }
-    found = warp_sum_u32(found);
+    flush();
     if (lane == 0 && found) atomicAdd(F.counters + CNT_ALLPOINTS, found);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < PP_LC; i += blockDim.x)
+        if (T.key[i] != EMPTY_KEY)
+            to_frame(T.key[i], T.cnt[i], T.xmin[i], T.xmax[i], T.ymin[i], T.ymax[i], T.gx[i], T.gy[i], T.pxgx[i]);
 }
 
 // Stage 7: each point of a pair that passed the filter goes to its
 // cluster's segment with its calc_theta key (main.cpp:621-675); the
-// cluster sorts then order each segment by (slope, point).
+// cluster sorts then order each segment by (slope, point).  A lane looks a
+// key up only when it differs from its last one, and points of dropped pairs
+// (most) take no part after that.
 __global__ void __launch_bounds__(256) k_planes_scatter(const __grid_constant__ FrameSet fs,
                                                         const uint32_t* __restrict__ points,
                                                         const unsigned long long* __restrict__ keys, uint32_t n) {
+    constexpr unsigned FULL = 0xFFFFFFFFu;
     const FrameDesc& F = fs.get(0);
-    const uint32_t lane = threadIdx.x & 31;
-    for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < n; base += gridDim.x * blockDim.x) {
-        const uint32_t i = base + lane;
-        const uint32_t p = i < n ? __ldg(points + i) : 0u;
-        if (!__any_sync(0xFFFFFFFFu, p != 0u)) continue;
-        uint32_t cid = INVALID;
-        if (p != 0u) {
-            const uint32_t slot = global_lookup(F, __ldg(keys + i));
-            if (slot != INVALID) cid = F.pair_cluster[slot];
+    const uint32_t lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const uint32_t groups = (n + PP_GROUP - 1) / PP_GROUP, per = (groups + gridDim.x - 1) / gridDim.x;
+    const uint32_t g0 = blockIdx.x * per, g1 = min(groups, g0 + per);
+    unsigned long long last = EMPTY_KEY;
+    uint32_t last_cid = INVALID;
+    for (uint32_t g = g0 + (threadIdx.x >> 5); g < g1; g += warps) {
+        uint32_t p[PP_UNROLL];
+        unsigned long long k[PP_UNROLL];
+#pragma unroll
+        for (uint32_t u = 0; u < PP_UNROLL; u++) {
+            const uint32_t i = g * PP_GROUP + 32 * u + lane;
+            p[u] = i < n ? __ldg(points + i) : 0u;
         }
-        const unsigned mask = __match_any_sync(0xFFFFFFFFu, cid);
-        if (cid != INVALID) {
-            const int leader = __ffs(mask) - 1;
-            uint32_t b = 0;
-            if ((int)lane == leader) b = atomicAdd(F.cluster_cursor + cid, (uint32_t)__popc(mask));
-            b = __shfl_sync(mask, b, leader);
-            const uint32_t rank = __popc(mask & ((1u << lane) - 1u));
-            const atag_cluster_extents ext = F.cluster_extents[cid];
-            const float2 ctr = F.cluster_center[cid];
-            const float theta = calc_theta(p, ctr.x, ctr.y);
-            if (b + rank < ext.count)
-                F.sortbuf[ext.start + b + rank] = ((unsigned long long)float_order_key(theta) << 32) | p;
+#pragma unroll
+        for (uint32_t u = 0; u < PP_UNROLL; u++)
+            k[u] = p[u] ? __ldg(keys + (g * PP_GROUP + 32 * u + lane)) : EMPTY_KEY;
+#pragma unroll
+        for (uint32_t u = 0; u < PP_UNROLL; u++) {
+            uint32_t cid = INVALID;
+            if (p[u]) {
+                if (k[u] != last) {
+                    const uint32_t slot = global_lookup(F, k[u]);
+                    last = k[u];
+                    last_cid = slot != INVALID ? F.pair_cluster[slot] : INVALID;
+                }
+                cid = last_cid;
+            }
+            if (!__any_sync(FULL, cid != INVALID)) continue;
+            const unsigned mask = __match_any_sync(FULL, cid);
+            if (cid != INVALID) {
+                const int leader = __ffs(mask) - 1;
+                uint32_t b = 0;
+                if ((int)lane == leader) b = atomicAdd(F.cluster_cursor + cid, (uint32_t)__popc(mask));
+                b = __shfl_sync(mask, b, leader);
+                const uint32_t rank = __popc(mask & ((1u << lane) - 1u));
+                const atag_cluster_extents ext = F.cluster_extents[cid];
+                const float2 ctr = F.cluster_center[cid];
+                const float theta = calc_theta(p[u], ctr.x, ctr.y);
+                if (b + rank < ext.count)
+                    F.sortbuf[ext.start + b + rank] = ((unsigned long long)float_order_key(theta) << 32) | p[u];
+            }
         }
     }
 }
@@ -117,19 +233,24 @@ __global__ void __launch_bounds__(256) k_stage_cluster_out(const __grid_constant
 // over the clusters, then each cluster's corners sorted in shared memory.
 // The reference's sort leaves ties unordered; here they go by position.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_peaks_count(const atag_corner* __restrict__ found,
+// One CTA per cluster, a cluster's errors read PK_UNROLL per thread at a time:
+// bound by the latency of the largest clusters' loads.  With a warp per cluster
+// the counts took 68 us for 1292 x 964 (9 now), the sort on 256 threads 37 (19
+// on 1024).
+constexpr int PK_UNROLL = 4;
+
+__global__ void __launch_bounds__(1024) k_peaks_count(const atag_corner* __restrict__ found,
                                                      const atag_cluster_extents* __restrict__ ext,
                                                      uint32_t n_clusters, uint32_t* __restrict__ counts) {
-    const uint32_t lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    for (uint32_t c = blockIdx.x * wpb + (threadIdx.x >> 5); c < n_clusters; c += gridDim.x * wpb) {
+    __shared__ uint32_t red[33];
+    for (uint32_t c = blockIdx.x; c < n_clusters; c += gridDim.x) {
         const atag_cluster_extents e = ext[c];
         uint32_t k = 0;
-        for (uint32_t i0 = 0; i0 < e.count; i0 += 32) {
-            const uint32_t i = i0 + lane;
-            const bool corner = i < e.count && found[(size_t)e.start + i].error != 0.0f;
-            k += (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, corner));
-        }
-        if (lane == 0) counts[c] = k;
+#pragma unroll PK_UNROLL
+        for (uint32_t i = threadIdx.x; i < e.count; i += blockDim.x)
+            k += found[(size_t)e.start + i].error != 0.0f ? 1u : 0u;
+        k = block_sum_u32(k, red);
+        if (threadIdx.x == 0) counts[c] = k;
     }
 }
 
@@ -158,7 +279,7 @@ __global__ void __launch_bounds__(1024) k_peaks_offsets(const uint32_t* __restri
     }
 }
 
-__global__ void __launch_bounds__(256) k_peaks_sort(const atag_corner* __restrict__ found,
+__global__ void __launch_bounds__(1024) k_peaks_sort(const atag_corner* __restrict__ found,
                                                     const atag_cluster_extents* __restrict__ ext,
                                                     uint32_t n_clusters, const uint32_t* __restrict__ counts,
                                                     const uint32_t* __restrict__ offsets,
@@ -178,11 +299,18 @@ __global__ void __launch_bounds__(256) k_peaks_sort(const atag_corner* __restric
         if (threadIdx.x == 0) s_n = 0;
         __syncthreads();
         // key: error descending (complemented order key), then position
-        for (uint32_t i = threadIdx.x; i < e.count; i += blockDim.x) {
-            const float err = found[(size_t)e.start + i].error;
-            if (err != 0.0f) {
+        for (uint32_t i0 = threadIdx.x; i0 < e.count; i0 += PK_UNROLL * blockDim.x) {
+            float err[PK_UNROLL];
+#pragma unroll
+            for (int u = 0; u < PK_UNROLL; u++) {
+                const uint32_t i = i0 + u * blockDim.x;
+                err[u] = i < e.count ? found[(size_t)e.start + i].error : 0.0f;
+            }
+#pragma unroll
+            for (int u = 0; u < PK_UNROLL; u++) {
+                if (err[u] == 0.0f) continue;
                 const uint32_t at = atomicAdd(&s_n, 1u);
-                if (at < k) pk_keys[at] = ((unsigned long long)(~float_order_key(err)) << 32) | i;
+                if (at < k) pk_keys[at] = ((unsigned long long)(~float_order_key(err[u])) << 32) | (i0 + u * blockDim.x);
             }
         }
         __syncthreads();
