@@ -61,12 +61,12 @@ def decode_quads(image, corners, family: Family, params=None, stream=None):
     else:
         raise ValueError("corners must be float32 corners or uint8 quad records")
     out = torch.empty((n, DECODED.itemsize), dtype=torch.uint8, device=image.device)
-    s = stream if stream is not None else torch.cuda.current_stream()
+    s = stream.cuda_stream if stream is not None else lib.current_stream()
     fam = family.struct()
     prm = params if params is not None else default_params()
     lib.check(L.atag_decode_quads(_P(image.data_ptr()), image.shape[1], image.shape[0], image.shape[1],
                                   _P(corners.data_ptr()), stride, n, ctypes.byref(fam), ctypes.byref(prm),
-                                  _P(out.data_ptr()), _P(s.cuda_stream)), "atag_decode_quads")
+                                  _P(out.data_ptr()), _P(s)), "atag_decode_quads")
     return out
 
 

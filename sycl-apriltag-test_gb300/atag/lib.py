@@ -125,9 +125,14 @@ def init(device: int = None):
     if device is None:
         import torch
         device = torch.cuda.current_device()
-    check(L.atag_use_device(int(device)), "atag_use_device")
-    check(L.atag_init(), "atag_init")
+    check(L.atag_use_device(int(device)), "atag_use_device")  # initialises the device too
     return L
+
+
+def current_stream() -> int:
+    """The handle of torch's current stream, without a Stream object."""
+    import torch
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def launch_count() -> int:

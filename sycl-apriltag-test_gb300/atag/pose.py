@@ -31,9 +31,9 @@ def estimate_pose(corners, fx, fy, cx, cy, tag_size, max_iterations=20, stream=N
     else:
         raise ValueError("corners must be float32 corners or uint8 quad records")
     out = torch.empty((n, POSE.itemsize), dtype=torch.uint8, device=corners.device)
-    s = stream if stream is not None else torch.cuda.current_stream()
+    s = stream.cuda_stream if stream is not None else lib.current_stream()
     lib.check(L.atag_estimate_pose(_P(corners.data_ptr()), stride, n, float(fx), float(fy), float(cx), float(cy),
-                                   float(tag_size), int(max_iterations), _P(out.data_ptr()), _P(s.cuda_stream)),
+                                   float(tag_size), int(max_iterations), _P(out.data_ptr()), _P(s)),
               "atag_estimate_pose")
     return out
 

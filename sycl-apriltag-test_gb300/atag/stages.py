@@ -19,7 +19,7 @@ _P = ctypes.c_void_p
 
 
 def _stream():
-    return _P(torch.cuda.current_stream().cuda_stream)
+    return _P(lib.current_stream())
 
 
 def _ptr(t):
@@ -43,6 +43,18 @@ def _dev(a):
 
 def _bytes(n, dtype, fill=0):
     return torch.full((max(int(n), 1) * np.dtype(dtype).itemsize,), fill, dtype=torch.uint8, device="cuda")
+
+
+def _blocks(*specs):
+    """Zeroed byte tensors of (n, dtype) records each, on 256-byte boundaries
+    of one allocation: one fill of wide words for all of them (a fill per
+    output took 190 us of host time in a chain of stage calls)."""
+    sizes = [max(int(n), 1) * np.dtype(dtype).itemsize for n, dtype in specs]
+    at = [0]
+    for s in sizes:
+        at.append(at[-1] + (s + 255) // 256 * 256)
+    buf = torch.zeros(at[-1] // 8, dtype=torch.int64, device="cuda").view(torch.uint8)
+    return [buf[o:o + s] for o, s in zip(at, sizes)]
 
 
 def decimate(src: torch.Tensor, factor: int) -> torch.Tensor:
@@ -149,12 +161,11 @@ def process_fitted_quads(fitted, width: int, height: int, config=None, n: int = 
     cfg = config or lib.default_config()
     if n is None:
         n = len(fitted)
-    d_out = _bytes(n, QUAD_CORNERS)
-    d_cnt = torch.zeros(1, dtype=torch.int32, device="cuda")
+    d_out, d_cnt = _blocks((n, QUAD_CORNERS), (1, np.int32))
     d_f = _dev(fitted) if n else torch.zeros(1, dtype=torch.uint8, device="cuda")
     lib.check(L.atag_process_fitted_quads(_ptr(d_f), n, width, height, ctypes.byref(cfg), _ptr(d_out), max(n, 1),
                                           _ptr(d_cnt), _stream()), "atag_process_fitted_quads")
-    cnt = int(d_cnt.item())
+    cnt = int(to_host(d_cnt, np.int32)[0])
     return to_host(d_out, QUAD_CORNERS)[:cnt]
 
 
@@ -178,11 +189,12 @@ def cluster(points: torch.Tensor, keys: torch.Tensor, grey: torch.Tensor, cluste
               "atag_cluster_workspace_size")
     ws = torch.empty(size.value, dtype=torch.uint8, device="cuda")
     cc = min(cluster_capacity, 65535)
-    out = {"pair_bounds": _bytes(pair_capacity, CLUSTER_BOUNDS), "pair_keys": _bytes(pair_capacity, np.uint64),
-           "filtered_bounds": _bytes(cc, CLUSTER_BOUNDS), "filtered_keys": _bytes(cc, np.uint64),
-           "cluster_extents": _bytes(cc, CLUSTER_EXTENTS), "cluster_points": _bytes(point_capacity, CLUSTER_POINT),
-           "cluster_indices": _bytes(point_capacity, np.uint16), "line_fit": _bytes(point_capacity, LINE_FIT_POINT),
-           "counts": _bytes(1, FRAME_STATS)}
+    specs = {"pair_bounds": (pair_capacity, CLUSTER_BOUNDS), "pair_keys": (pair_capacity, np.uint64),
+             "filtered_bounds": (cc, CLUSTER_BOUNDS), "filtered_keys": (cc, np.uint64),
+             "cluster_extents": (cc, CLUSTER_EXTENTS), "cluster_points": (point_capacity, CLUSTER_POINT),
+             "cluster_indices": (point_capacity, np.uint16), "line_fit": (point_capacity, LINE_FIT_POINT),
+             "counts": (1, FRAME_STATS)}
+    out = dict(zip(specs, _blocks(*specs.values())))
     o = ClusterOutputs(_ptr(out["pair_bounds"]), _ptr(out["pair_keys"]), pair_capacity,
                        _ptr(out["filtered_bounds"]), _ptr(out["filtered_keys"]), _ptr(out["cluster_extents"]), cc,
                        _ptr(out["cluster_points"]), _ptr(out["cluster_indices"]), _ptr(out["line_fit"]),
@@ -204,13 +216,11 @@ def corner_peaks(found: torch.Tensor, cluster_extents: torch.Tensor, n_clusters:
     size = ctypes.c_size_t()
     lib.check(L.atag_corner_peaks_workspace_size(n_clusters, ctypes.byref(size)), "atag_corner_peaks_workspace_size")
     ws = torch.empty(size.value, dtype=torch.uint8, device="cuda")
-    d_corners = _bytes(corner_capacity, CORNER)
-    d_pe = _bytes(extents_capacity, PEAK_EXTENTS)
-    d_counts = torch.zeros(3, dtype=torch.int32, device="cuda")
+    d_corners, d_pe, d_counts = _blocks((corner_capacity, CORNER), (extents_capacity, PEAK_EXTENTS), (3, np.uint32))
     lib.check(L.atag_corner_peaks(_ptr(found), _ptr(cluster_extents), n_clusters, _ptr(ws), size.value,
                                   _ptr(d_corners), corner_capacity, _ptr(d_pe), extents_capacity, _ptr(d_counts),
                                   _stream()), "atag_corner_peaks")
-    k, cp, status = (int(v) for v in d_counts.cpu().numpy().view(np.uint32))
+    k, cp, status = (int(v) for v in to_host(d_counts, np.uint32))
     return d_corners, d_pe, (k, cp, status)
 
 
