@@ -196,43 +196,33 @@ __device__ __forceinline__ BlockLinks block_links(PixelAt px, int x, int y, int 
     return BlockLinks{info, wm, bm};
 }
 
-// Root of n, following at most `cap` parents; *capped is set when the cap
-// ends the walk before a root.
-__device__ __forceinline__ uint32_t find_root_volatile(volatile uint32_t* p, uint32_t n, uint32_t cap, bool* capped) {
-    // path halving: every write replaces a parent by one of its ancestors,
-    // which stays valid under concurrent unions (only roots are re-linked)
-    for (uint32_t it = 0; it < cap; it++) {
-        uint32_t q = p[n];
-        if (q == n) return n;
-        uint32_t g = p[q];
-        if (g != q) p[n] = g;
-        n = g;
-    }
-    *capped = true;
-    return n;
-}
-
-// Lock-free union toward the smaller root (union_find.h:50-77) with
-// iteration caps; returns false if a cap was hit.  With a non-root in hand
-// the union still only lowers parents (atomicMin), so the forest stays
-// acyclic and every later walk ends.
+// Lock-free union toward the smaller root (union_find.h:50-77) with an
+// iteration cap; returns false if it was hit.  The border pass is bound by the
+// latency of these chains of parents, so both walks go in lock step, two levels
+// at a time with path halving (a parent is replaced by one of its ancestors,
+// which stays valid under concurrent unions), and end where they meet.  Walking
+// one after the other, each to its root, the pass took 26 us for one 1080p
+// frame (18 now), 55 for a 4K frame (28) and 244 for 64 1080p frames (207).
+// With a non-root in hand the union still only lowers parents (atomicMin), so
+// the forest stays acyclic and every later walk ends.
 template <typename Ptr>
 __device__ __forceinline__ bool uf_union(Ptr par, uint32_t a, uint32_t b, uint32_t cap) {
-    bool capped = false;
     for (uint32_t it = 0; it < cap; it++) {
-        a = find_root_volatile(par, a, cap, &capped);
-        b = find_root_volatile(par, b, cap, &capped);
-        if (capped) return false;
-        if (a == b) return true;
-        if (a < b) {
-            uint32_t old = atomicMin((uint32_t*)&par[b], a);
-            if (old == b) return true;
-            b = old;
-        } else {
-            uint32_t old = atomicMin((uint32_t*)&par[a], b);
-            if (old == a) return true;
-            a = old;
+        const uint32_t pa = par[a], pb = par[b];
+        if (pa == pb) return true;
+        if (pa != a || pb != b) {
+            const uint32_t ga = par[pa], gb = par[pb];
+            if (ga != pa) par[a] = ga;
+            if (gb != pb) par[b] = gb;
+            a = ga;
+            b = gb;
+            continue;
         }
+        const uint32_t lo = min(a, b), hi = max(a, b);
+        const uint32_t old = atomicMin((uint32_t*)&par[hi], lo);
+        if (old == hi) return true;
+        a = old;
+        b = lo;
     }
     return false;
 }
