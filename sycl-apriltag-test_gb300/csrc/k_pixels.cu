@@ -233,12 +233,12 @@ __device__ __forceinline__ bool uf_union(Ptr par, uint32_t a, uint32_t b, uint32
 __device__ __forceinline__ void tile_union(volatile uint32_t* par, uint32_t a, uint32_t b, uint32_t cap) {
     for (uint32_t it = 0; it < cap; it++) {
         const uint32_t pa = par[a], pb = par[b];
+        if (pa == pb) return;
         if (pa != a || pb != b) {
             a = pa;
             b = pb;
             continue;
         }
-        if (a == b) return;
         const uint32_t hi = max(a, b), lo = min(a, b);
         const uint32_t old = atomicMin((uint32_t*)&par[hi], lo);
         if (old == hi) return;
