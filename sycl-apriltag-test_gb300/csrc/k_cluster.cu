@@ -136,7 +136,7 @@ __device__ __forceinline__ void boundaries_pairs_impl(const FrameSet& fs, uint32
     // CTAs are dispatched frame-fastest, so the tiles in flight at once span
     // every frame of the batch and a frame's later tiles start after its
     // first ones published their over-limit pairs
-    const FrameDesc& F = fs.get(blockIdx.x);
+    const FrameDesc& F = fs.of_table(blockIdx.x);
     const int w = F.width, h = F.height;
     const int ntx = (w + BP_W - 1) / BP_W, nty = (h + BP_H - 1) / BP_H;
     if ((int)blockIdx.y >= ntx || (int)blockIdx.z >= nty) return;
@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(PF_THREADS) k_pairs_finalize(const __grid_cons
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_scatter_points(const __grid_constant__ FrameSet fs) {
     if (fs.overlap) await_previous_kernel();
-    const FrameDesc& F = fs.get(blockIdx.y);
+    const FrameDesc& F = fs.of_table(blockIdx.y);
     uint32_t n = F.counters[CNT_POINTS];
     if (n > F.point_cap) n = F.point_cap;
     const uint32_t lane = threadIdx.x & 31;
@@ -1212,7 +1212,7 @@ __global__ void __launch_bounds__(32 * CE_WARPS, 4) k_cluster_lines(const __grid
     RunSums* S = reinterpret_cast<RunSums*>(smem_runs) + wid;
     for (uint32_t item = blockIdx.x + gridDim.x * wid; item < total; item += gridDim.x * CE_WARPS) {
         const uint32_t fidx = find_frame(run_offsets, n_frames, item);
-        const FrameDesc& F = fs.get(fidx);
+        const FrameDesc& F = fs.of_table(fidx);
         cluster_run<true>(F, F.runs[item - run_offsets[fidx]], S);
     }
 }
@@ -1230,7 +1230,7 @@ __global__ void __launch_bounds__(32 * CE_WARPS, 4) k_cluster_prefix(const __gri
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) k_peaks_scan(const __grid_constant__ FrameSet fs, BatchOffsets a) {
     if (fs.overlap) await_previous_kernel();
-    const FrameDesc& F = fs.get(blockIdx.x);
+    const FrameDesc& F = fs.of_table(blockIdx.x);
     __shared__ uint32_t red[33];
     const uint32_t C = F.counters[CNT_CLUSTERS];
     uint32_t carry_q = 0, carry_k = 0;
@@ -1298,7 +1298,7 @@ __global__ void __launch_bounds__(256) k_index_quads(const __grid_constant__ Fra
     const uint32_t total = work_offsets[n_frames];
     for (uint32_t item = blockIdx.x + gridDim.x * wid; item < total; item += gridDim.x * 8) {
         const uint32_t fidx = find_frame(work_offsets, n_frames, item);
-        const FrameDesc& F = fs.get(fidx);
+        const FrameDesc& F = fs.of_table(fidx);
         const uint32_t q = item - work_offsets[fidx];
         const uint32_t cid = F.peak_clusters[q], count = F.peak_count[cid];
         const atag_cluster_extents ce = F.cluster_extents[p.compat_peak_index ? q : cid];
@@ -1341,7 +1341,7 @@ __global__ void __launch_bounds__(256) k_index_quads(const __grid_constant__ Fra
 
 __global__ void __launch_bounds__(1024) k_compact_quads(const __grid_constant__ FrameSet fs) {
     if (fs.overlap) await_previous_kernel();
-    const FrameDesc& F = fs.get(blockIdx.x);
+    const FrameDesc& F = fs.of_table(blockIdx.x);
     __shared__ uint32_t red[33];
     const uint32_t Cp = F.counters[CNT_PEAKCLU];
     uint32_t carry = 0, nfit = 0;

@@ -263,7 +263,7 @@ __device__ __forceinline__ void ccl_local_impl(const FrameSet& fs) {
     constexpr unsigned FULL = 0xFFFFFFFFu;
     // grid (tile column, tile row, frame): the frame's tile from the block
     // indices, no division
-    const FrameDesc& F = fs.get(blockIdx.z);
+    const FrameDesc& F = EXACT ? fs.get(blockIdx.z) : fs.of_table(blockIdx.z);
     const int w = F.width, h = F.height;
     const int ntx = ccl_tiles_x(w), nty = ccl_tiles_y<CCL_BY>(h);
     if ((int)blockIdx.x >= ntx || (int)blockIdx.y >= nty) return;
@@ -538,7 +538,7 @@ template <int CCL_BY>
 __device__ __forceinline__ void ccl_border_edges_impl(const FrameSet& fs) {
     constexpr int PER = CCL_BX + 2 * (CCL_BY - 1);
     constexpr uint32_t EW = ccl_edge_words(CCL_BY), SLOT = 0xFFFFFFu;
-    const FrameDesc& F = fs.get(blockIdx.y);
+    const FrameDesc& F = fs.of_table(blockIdx.y);
     const int w = F.width, h = F.height;
     const int ntx = ccl_tiles_x(w), nty = ccl_tiles_y<CCL_BY>(h);
     const int total = ntx * nty * PER;

@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(32 * RF_WARPS) k_refine_forward(const float* _
 __global__ void __launch_bounds__(32 * RF_WARPS) k_refine_detected(const __grid_constant__ FrameSet fs) {
     if (fs.overlap) await_previous_kernel();
     __shared__ EdgeSums sums[4];
-    const FrameDesc& F = fs.get(blockIdx.x);
+    const FrameDesc& F = fs.of_table(blockIdx.x);
     const uint32_t nq = min(F.stats->n_quads, F.quad_cap);
     const U8Image img{F.grey};
     const int e = threadIdx.x >> 5, lane = threadIdx.x & 31, e1 = (e + 1) & 3;
