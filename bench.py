@@ -172,8 +172,7 @@ def survey_bytes(stats):
         "scatter_points": 12 * P + 32 * C + 10 * Pf,
         "cluster_sort": 2 * 10 * Pf + (8 + 4 + 48) * Pf + 2 * 48 * Pf,
         "cluster_errors": 48 * Pf * 2 + 2 * Pf + 12 * K,
-        "cluster_peaks": 2 * 12 * K,
-        "index_quads": Cp * (8 + 120 + 4 * 2 * 48) + 272 * Cp,
+        "index_quads": 2 * 12 * K + Cp * (8 + 120 + 4 * 2 * 48) + 272 * Cp,  # with the choice of the 10 best peaks
     }
 
 

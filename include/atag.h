@@ -636,8 +636,8 @@ atag_status atag_decode_quads(const uint8_t *d_image, size_t width, size_t heigh
 typedef struct atag_tuning {
     int32_t ccl_tile_rows;        /* 8, 16 or 32 rows of 2x2 blocks per CCL tile (16) */
     int32_t boundary_tile_rows;   /* 8 or 16 pixel rows per boundary tile (16)      */
-    int32_t small_cluster_max;    /* clusters up to this size use the 128-thread
-                                     kernel, larger ones the 512-thread one
+    int32_t small_cluster_max;    /* clusters up to this size use the 256-thread
+                                     kernel, larger ones the 1024-thread one
                                      (1..2048, default 2048)                        */
     int32_t small_ctas_per_sm;    /* persistent CTAs of the small-cluster kernel (8) */
     int32_t large_ctas_divisor;   /* large-cluster CTAs = SMs / divisor (2)         */

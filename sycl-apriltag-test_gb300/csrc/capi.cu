@@ -1007,7 +1007,7 @@ static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, con
     STAGE(10);
     k_cluster_lines<<<sms * 4, 128, CE_LINES_SMEM, s>>>(fs, off_runs, (uint32_t)n);
     LAUNCHED();
-    STAGE(11);
+    STAGE(11);  // the 10 best peaks: no kernel of their own, k_index_quads chooses them
     STAGE(12);
     const BatchOffsets with_peaks{{CNT_PEAKCLU, 0, 0}, {off_peaks, nullptr, nullptr}, wc + 3};
     launch(overlap, k_peaks_scan, (unsigned)n, 1024, 0, s, fs, with_peaks);
