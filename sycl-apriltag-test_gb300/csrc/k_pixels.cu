@@ -202,7 +202,8 @@ __device__ __forceinline__ BlockLinks block_links(PixelAt px, int x, int y, int 
 // at a time with path halving (a parent is replaced by one of its ancestors,
 // which stays valid under concurrent unions), and end where they meet.  Walking
 // one after the other, each to its root, the pass took 26 us for one 1080p
-// frame (18 now), 55 for a 4K frame (28) and 244 for 64 1080p frames (207).
+// frame (18 now), 55 for a 4K frame (27) and 244 for 64 1080p frames (180; 205
+// with 40 registers, six CTAs per SM instead of eight).
 // With a non-root in hand the union still only lowers parents (atomicMin), so
 // the forest stays acyclic and every later walk ends.
 template <typename Ptr>
@@ -757,15 +758,15 @@ __global__ void __launch_bounds__(256) k_boundaries_dense(const __grid_constant_
         BEFORE;                                                                                                 \
         ccl_local_impl<32, false>(fs);                                                                          \
     }                                                                                                           \
-    __global__ void __launch_bounds__(256) k_ccl_border_edges_r8##SUFFIX(const __grid_constant__ FrameSet fs) { \
+    __global__ void __launch_bounds__(256, 8) k_ccl_border_edges_r8##SUFFIX(const __grid_constant__ FrameSet fs) { \
         BEFORE;                                                                                                 \
         ccl_border_edges_impl<8>(fs);                                                                           \
     }                                                                                                           \
-    __global__ void __launch_bounds__(256) k_ccl_border_edges_r16##SUFFIX(const __grid_constant__ FrameSet fs) { \
+    __global__ void __launch_bounds__(256, 8) k_ccl_border_edges_r16##SUFFIX(const __grid_constant__ FrameSet fs) { \
         BEFORE;                                                                                                 \
         ccl_border_edges_impl<16>(fs);                                                                          \
     }                                                                                                           \
-    __global__ void __launch_bounds__(256) k_ccl_border_edges_r32##SUFFIX(const __grid_constant__ FrameSet fs) { \
+    __global__ void __launch_bounds__(256, 8) k_ccl_border_edges_r32##SUFFIX(const __grid_constant__ FrameSet fs) { \
         BEFORE;                                                                                                 \
         ccl_border_edges_impl<32>(fs);                                                                          \
     }                                                                                                           \
