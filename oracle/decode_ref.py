@@ -228,6 +228,9 @@ def decode_one(img, corners, layout, codes, max_hamming=2, sharpening=0.25, refi
     p = [[float(v) for v in c] for c in np.asarray(corners, np.float64)]
     out = {"code": 0, "id": -1, "hamming": 0xFFFFFFFF, "rotation": 0, "status": 0, "decision_margin": 0.0,
            "black": 0.0, "white": 0.0, "corners": np.array(p)}
+    if not np.isfinite(out["corners"]).all():
+        out["status"] |= DEGENERATE
+        return out
     area2 = sum(p[i][0] * p[(i + 1) & 3][1] - p[(i + 1) & 3][0] * p[i][1] for i in range(4))
     if area2 < 0.0:
         p[1], p[3] = p[3], p[1]

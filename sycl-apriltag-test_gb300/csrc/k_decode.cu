@@ -31,8 +31,8 @@
 //      non-negative decision margin.
 // Beyond the library: a quad wound the other way is read with corners 0, 3,
 // 2, 1 (flagged); the refinement's normal points outward by the quad's
-// signed area; a projection behind the camera (z <= 0) marks the quad
-// degenerate.
+// signed area; a projection behind the camera (z <= 0) or a corner that is not
+// finite marks the quad degenerate.
 //
 // One warp per quad, FP64 throughout: lanes take the refinement's points,
 // the grey-model samples, the bits and the codes.  FP64 issues at 2 lanes per
@@ -306,8 +306,10 @@ __global__ void __launch_bounds__(32 * DECODE_WARPS) k_decode_quads(
     double* vals = s_vals[wid];
     const float* cf = reinterpret_cast<const float*>(quads + (size_t)q * stride);
     double px[4], py[4];
+    bool finite = true;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
+        finite &= isfinite(cf[2 * i]) && isfinite(cf[2 * i + 1]);
         px[i] = (double)cf[2 * i];
         py[i] = (double)cf[2 * i + 1];
     }
@@ -337,8 +339,11 @@ __global__ void __launch_bounds__(32 * DECODE_WARPS) k_decode_quads(
             out[q] = R;
         }
     };
+    // With finite corners every projected coordinate below is finite (z is 1
+    // plus bounded terms, so not denormal); homography_ok itself never reads
+    // corner 0.
     double den;
-    bool ok = homography_ok(px, py, &den);
+    bool ok = finite && homography_ok(px, py, &den);
     if (ok && prm.refine) {
         refine_edges(img, w, h, pitch, px, py, F.reversed_border != 0, prm.quad_decimate);
         ok = homography_ok(px, py, &den);
@@ -370,8 +375,10 @@ __global__ void __launch_bounds__(32 * DECODE_WARPS) k_decode_quads(
             behind = true;
             continue;
         }
+        // (-1, 0) truncates to 0; the conversion saturates and takes NaN to
+        // INT_MIN, which the unsigned test rejects too
         const int ix = __double2int_rz(x), iy = __double2int_rz(y);
-        if (x <= -1.0 || y <= -1.0 || ix >= w || iy >= h) continue;
+        if ((unsigned)ix >= (unsigned)w || (unsigned)iy >= (unsigned)h) continue;
         const int v = img[(size_t)iy * pitch + ix], ta = hx - Wb, tb = hy - Wb;
         const int t[9] = {ta * ta, ta * tb, ta, tb * tb, tb, 1, ta * v, tb * v, v};
 #pragma unroll
