@@ -51,6 +51,7 @@
 // 1,178 us before; 597 and 219 us now (FP64 pipe 74% busy).
 #include <vector>
 
+#include "atag_edge_samples.cuh"
 #include "atag_internal.h"
 #include "atag_kernels.cuh"
 
@@ -194,7 +195,10 @@ __device__ void refine_edges(const uint8_t* __restrict__ img, int w, int h, size
         nx = -nx;
         ny = -ny;
     }
-    const int nsamples = max(16, (int)(mag / 8.0));
+    const int nsamples = edge_sample_count(mag);
+    SampleRange S{0, nsamples};
+    if (__any_sync(0xFFFFFFFFu, nsamples > EDGE_SAMPLES_WHOLE))
+        S = edge_sample_range(ax, ay, bx, by, nsamples, quad_decimate + 2, w, h);
     const int r4 = 4 * (quad_decimate + 1);  // search range in quarter pixels
     // FP64 positions where a corner is far out or two coincide (warp-uniform)
     constexpr double FAR = 4000.0;
@@ -208,7 +212,7 @@ __device__ void refine_edges(const uint8_t* __restrict__ img, int w, int h, size
     const double mx = 0.5 * (ax + bx), my = 0.5 * (ay + by);
     double m[5] = {0, 0, 0, 0, 0};  // x, y, xx, xy, yy
     int count = 0;
-    for (int s = sub; s < nsamples; s += 8) {
+    for (int s = S.lo + sub; s < S.hi; s += 8) {
         const double alpha = (1.0 + s) / (nsamples + 1);
         W.x0 = alpha * ax + (1.0 - alpha) * bx;
         W.y0 = alpha * ay + (1.0 - alpha) * by;
