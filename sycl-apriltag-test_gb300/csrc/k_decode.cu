@@ -42,13 +42,14 @@
 //   * the four edges are refined side by side, eight lanes each, so edge set-up,
 //     line fit and corner intersection are issued once, not four times, and
 //     the sums reduce over eight lanes;
-//   * positions along an edge's normal step in exact integers (Q50), each
-//     grey value is fetched once (the step at n pairs offsets n + 1 and n - 1),
-//     and weights and grey-model sums are integers, exact;
+//   * positions along an edge's normal step in exact integers (Q50), but for
+//     those on pixel borders; each grey value is fetched once (the step at n
+//     pairs offsets n + 1 and n - 1), and weights and grey-model sums are
+//     integers, exact;
 //   * the edge's direction comes from square roots, not atan2/sin/cos;
 //   * both grey models are solved at once, on even and odd lanes.
 // 4,096 quads against 587 codes: 4,072 FP64 warp instructions per quad and
-// 1,178 us before; 597 and 219 us now (FP64 pipe 74% busy).
+// 1,178 us before; about 600 and 223 us now (219 without the care at borders).
 #include <vector>
 
 #include "atag_edge_samples.cuh"
@@ -151,7 +152,10 @@ __device__ __forceinline__ bool trunc_in(double v, int n, int* out) {
 // Grey values along one refinement point's normal: offset k quarter pixels,
 // the pixel at the truncated coordinate - 0.5; -1 outside the image.  Within
 // 4,000 px of the origin positions are Q50 integers: an FP64 point from 4 px
-// on converts exactly, and steps without rounding error.  Beyond, FP64.
+// on converts exactly, and steps without rounding error.  A coordinate within
+// 2^-32 px of a pixel's border, where the FP64 sum's rounding (below 2^-40)
+// may fall on the other side of it, is taken from that sum, as beyond 4,000 px:
+// quads along the axes with corners on whole pixels put many points there.
 struct NormalWalk {
     const uint8_t* __restrict__ img;
     int w, h;
@@ -159,12 +163,13 @@ struct NormalWalk {
     bool fixed;
     long long X, Y, NX, NY;  // Q50 position - 0.5, Q52 normal
     double x0, y0, nx, ny;
+    __device__ __forceinline__ static bool at_border(long long v) { return (uint32_t)(v >> 18) + 1u <= 1u; }
     __device__ __forceinline__ int at(int k) const {
         int ix, iy;
-        if (fixed) {
-            // k / 4 * n in Q50: k * Q52 >> 4; truncation toward zero takes
-            // (-1, 0) to 0
-            const long long x = X + ((k * NX) >> 4), y = Y + ((k * NY) >> 4);
+        // k / 4 * n in Q50: k * Q52 >> 4
+        const long long x = X + ((k * NX) >> 4), y = Y + ((k * NY) >> 4);
+        if (fixed && !at_border(x) && !at_border(y)) {
+            // truncation toward zero takes (-1, 0) to 0
             constexpr long long ONE = 1ll << 50;
             if (x <= -ONE || y <= -ONE) return -1;
             ix = x < 0 ? 0 : (int)(x >> 50);
