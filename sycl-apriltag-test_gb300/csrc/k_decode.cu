@@ -49,7 +49,8 @@
 //   * the edge's direction comes from square roots, not atan2/sin/cos;
 //   * both grey models are solved at once, on even and odd lanes.
 // 4,096 quads against 587 codes: 4,072 FP64 warp instructions per quad and
-// 1,178 us before; about 600 and 223 us now (219 without the care at borders).
+// 1,178 us before; about 620 and 229 us now (597 and 219 without the FP64
+// positions on pixel borders and the quotients and cell centres of `project`).
 #include <vector>
 
 #include "atag_edge_samples.cuh"
@@ -61,6 +62,10 @@ namespace {
 
 constexpr int DECODE_WARPS = 4;
 constexpr int MAX_TW = 16;  // total_width limit: the value grid lives in shared memory
+// Cells -1 .. width_at_border (the white ring's) and those of the bits, which
+// start at (width_at_border - total_width) / 2 >= -6: bit cells are int8, so
+// widths are at most 2 * 127 + MAX_TW.
+constexpr int CELL_BASE = 8, MAX_CELLS = CELL_BASE + 2 * 127 + MAX_TW + 2;
 
 struct FamilyDesc {
     int8_t bit_x[64], bit_y[64];
@@ -110,9 +115,8 @@ __device__ __forceinline__ Homography make_homography(const double* px, const do
 __device__ __forceinline__ bool project(const Homography& H, double u, double v, double* x, double* y) {
     const double z = H.g * u + H.h * v + 1.0;
     if (!(z > 0.0)) return false;
-    const double iz = 1.0 / z;
-    *x = (H.a * u + H.b * v + H.c) * iz;
-    *y = (H.d * u + H.e * v + H.f) * iz;
+    *x = (H.a * u + H.b * v + H.c) / z;
+    *y = (H.d * u + H.e * v + H.f) / z;
     return true;
 }
 
@@ -309,6 +313,16 @@ __global__ void __launch_bounds__(32 * DECODE_WARPS) k_decode_quads(
     uint32_t n, const unsigned long long* __restrict__ codes, const __grid_constant__ FamilyDesc F,
     DecodeParams prm, atag_decoded* __restrict__ out) {
     __shared__ double s_vals[DECODE_WARPS][MAX_TW * MAX_TW];
+    // unit-square coordinate of each cell's centre, by way of the tag coordinate
+    // and its roundings: a quad along the axes puts many samples on the borders
+    // between pixels, where the last bit chooses the pixel
+    __shared__ double s_centre[MAX_CELLS];
+    for (int i = threadIdx.x; i < CELL_BASE + max(F.width_at_border, F.total_width) + 2; i += blockDim.x) {
+        const double t = 2.0 * (((double)(i - CELL_BASE) + 0.5) / F.width_at_border - 0.5);
+        s_centre[i] = 0.5 * (t + 1.0);
+    }
+    __syncthreads();
+    const double* centre = s_centre + CELL_BASE;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t q = blockIdx.x * DECODE_WARPS + wid;
     if (q >= n) return;  // warp-uniform
@@ -367,7 +381,6 @@ __global__ void __launch_bounds__(32 * DECODE_WARPS) k_decode_quads(
     // half cells, hx = 2 (x0 + i), so that tx = (hx - W) / W and the sums
     // over hx - W are integers
     const int Wb = F.width_at_border, T = F.total_width;
-    const double half_cell = 0.5 / Wb;
     int sums[2][9];  // black, white
 #pragma unroll
     for (int k = 0; k < 9; k++) sums[0][k] = sums[1][k] = 0;
@@ -380,7 +393,7 @@ __global__ void __launch_bounds__(32 * DECODE_WARPS) k_decode_quads(
         const int edge = (pat & 2) ? 2 * Wb + (white ? 1 : -1) : (white ? -1 : 1);
         const int hx = vertical ? edge : 2 * i + 1, hy = vertical ? 2 * i + 1 : edge;
         double x, y;
-        if (!project(H, half_cell * hx, half_cell * hy, &x, &y)) {
+        if (!project(H, centre[hx >> 1], centre[hy >> 1], &x, &y)) {
             behind = true;
             continue;
         }
@@ -440,7 +453,7 @@ __global__ void __launch_bounds__(32 * DECODE_WARPS) k_decode_quads(
         const int bx = F.bit_x[i], by = F.bit_y[i], hx = 2 * bx + 1, hy = 2 * by + 1;
         cell[j] = (by - m) * T + (bx - m);
         double x, y;
-        if (!project(H, half_cell * hx, half_cell * hy, &x, &y)) {
+        if (!project(H, centre[bx], centre[by], &x, &y)) {
             behind = true;
             continue;
         }

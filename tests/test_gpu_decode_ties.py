@@ -59,3 +59,26 @@ def test_edges_walked_along_pixel_borders():
     g = _decode([q for q, _ in REFINED], 8, 1)
     # the values above are rounded to 1e-4
     assert np.abs(g["corners"] - np.array([c for _, c in REFINED])).max() <= 1e-3
+
+
+# (cells of a side, quad, white, black)
+MODELS = [
+    (8, [[233, 351], [311, 350], [307, 370], [230, 366]], 139.84375, 148.0),
+    (7, [[74, 339], [270, 339], [270, 400], [74, 400]], 133.25, 124.67857),
+    (7, [[52, 164], [248, 164], [248, 267], [52, 267]], 102.5, 131.07143),
+    (7, [[39, 70], [218, 70], [218, 252], [39, 252]], 127.57143, 130.10715),
+    (7, [[190, 13], [262, 13], [262, 97], [190, 97]], 119.57143, 141.0),
+    (6, [[9, 398], [81, 398], [81, 443], [9, 443]], 116.58334, 115.91666),
+    (6, [[33, 321], [153, 321], [153, 344], [33, 344]], 145.91667, 97.5),
+    (6, [[43, 35], [143, 35], [143, 167], [43, 167]], 108.66666, 149.16667),
+    (6, [[39, 29], [231, 29], [231, 102], [39, 102]], 104.66666, 152.25),
+]
+
+
+@pytest.mark.parametrize("width", [6, 7, 8])
+def test_grey_model_samples_on_pixel_borders(width):
+    rows = [m for m in MODELS if m[0] == width]
+    g = _decode([m[1] for m in rows], width, 0)
+    # a sample's grey value changes a model by at least 1 / 32 of a grey level
+    assert np.abs(g["white"] - [m[2] for m in rows]).max() <= 1e-3
+    assert np.abs(g["black"] - [m[3] for m in rows]).max() <= 1e-3
