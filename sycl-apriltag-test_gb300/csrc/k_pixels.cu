@@ -153,13 +153,16 @@ constexpr int CCL_BX = 32;  // blocks per tile row; CCL_BY (8, 16 or 32) rows is
 // tiles.  So a chain, and the retries of one union (each moves to a
 // strictly smaller root), are bounded by uf_bound(w, h); a loop that gets
 // there flags ATAG_DEVFLAG_UF_ITERATION_CAP instead of spinning.
-// FrameDesc::uf_cap may lower the bound (0 keeps it).
+// FrameDesc::uf_cap may lower the bound (0 keeps it).  Loops may take twice the
+// cap: unions that end where their walks meet compress the forest less than
+// walks to the root would, so chains are up to twice as long as those.
 __device__ __forceinline__ uint32_t uf_bound(uint32_t w, uint32_t h) {
     const uint32_t tiles = ((w / 2 + CCL_BX - 1) / CCL_BX) * ((h / 2 + 7) / 8);
     return 2u * (2u * CCL_BX + 2u * 8u) * tiles + 2u;
 }
 __device__ __forceinline__ uint32_t uf_cap_of(const FrameDesc& F) {
-    return F.uf_cap ? F.uf_cap : uf_bound(F.width, F.height);
+    const uint32_t bound = uf_bound(F.width, F.height);
+    return 2u * (F.uf_cap ? min(F.uf_cap, bound) : bound);
 }
 
 // Which neighbour blocks (bit 0 P, 1 Q, 2 R, 3 S) a block links to in the
@@ -196,8 +199,8 @@ __device__ __forceinline__ BlockLinks block_links(PixelAt px, int x, int y, int 
     return BlockLinks{info, wm, bm};
 }
 
-// Lock-free union toward the smaller root (union_find.h:50-77) with an
-// iteration cap; returns false if it was hit.  The border pass is bound by the
+// Lock-free union toward the smaller root (union_find.h:50-77); returns false
+// if a walk to the roots or the retries took `cap` iterations.  The border pass is bound by the
 // latency of these chains of parents, so both walks go in lock step, two levels
 // at a time with path halving (a parent is replaced by one of its ancestors,
 // which stays valid under concurrent unions), and end where they meet.  Walking
@@ -208,7 +211,9 @@ __device__ __forceinline__ BlockLinks block_links(PixelAt px, int x, int y, int 
 // the forest stays acyclic and every later walk ends.
 template <typename Ptr>
 __device__ __forceinline__ bool uf_union(Ptr par, uint32_t a, uint32_t b, uint32_t cap) {
-    for (uint32_t it = 0; it < cap; it++) {
+    uint32_t steps = cap, tries = cap;  // left to this pair of walks, and to the union
+    while (true) {
+        if (steps == 0 || tries == 0) return false;
         const uint32_t pa = par[a], pb = par[b];
         if (pa == pb) return true;
         if (pa != a || pb != b) {
@@ -217,6 +222,7 @@ __device__ __forceinline__ bool uf_union(Ptr par, uint32_t a, uint32_t b, uint32
             if (gb != pb) par[b] = gb;
             a = ga;
             b = gb;
+            steps--;
             continue;
         }
         const uint32_t lo = min(a, b), hi = max(a, b);
@@ -224,8 +230,9 @@ __device__ __forceinline__ bool uf_union(Ptr par, uint32_t a, uint32_t b, uint32
         if (old == hi) return true;
         a = old;
         b = lo;
+        steps = cap;
+        tries--;
     }
-    return false;
 }
 
 // The same within a tile's shared-memory forest: both walks in lock step, so
@@ -637,7 +644,7 @@ __device__ __forceinline__ void ccl_final_impl(const FrameSet& fs) {
     const int w = F.width, h = F.height;
     const int npx = w / 4, by = blockIdx.y, px = blockIdx.x * CCL_FINAL_THREADS + threadIdx.x;  // w % 4 == 0
     const uint32_t* par = F.scratch;
-    const uint32_t cap = uf_cap_of(F);
+    const uint32_t cap = 2u * uf_cap_of(F);  // of one parent, a union's iterations being of two
     if (by < h / 2 && px < npx) {
         const size_t id = (size_t)(by * 2) * w + (size_t)px * 4;
         const uint4 p4 = *reinterpret_cast<const uint4*>(F.scratch + id);
