@@ -457,9 +457,9 @@ typedef struct atag_limits {
                                         (ATAG_DEVFLAG_PAIR_OVERFLOW)                              */
     uint32_t cluster_capacity;       /* filtered clusters (ATAG_DEVFLAG_CLUSTER_OVERFLOW)           */
     uint32_t cluster_point_capacity; /* points of filtered clusters (ATAG_DEVFLAG_CLUSTER_OVERFLOW) */
-    uint32_t uf_iteration_cap;       /* twice this many iterations of one frame-wide union-find walk
-                                        (two parents each) and retries of one union, counted apart,
-                                        raise ATAG_DEVFLAG_UF_ITERATION_CAP; the default is
+    uint32_t uf_iteration_cap;       /* four times this many iterations of one frame-wide union (steps
+                                        of both walks and retries) or of one final walk raise
+                                        ATAG_DEVFLAG_UF_ITERATION_CAP; the default is
                                         the bound the CCL tile count gives for a w x h frame,
                                         2 + 160 ceil(w / 64) ceil(h / 16)                       */
     uint32_t reserved[3];

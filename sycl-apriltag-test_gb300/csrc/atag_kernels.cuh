@@ -70,7 +70,7 @@ struct FrameDesc {
     // whose running point count is already above the cluster size limit; null
     // when not tracked
     unsigned long long* dead_pairs;
-    // iteration cap of the frame-wide union-find loops (0: the bound the
+    // iteration cap of the frame-wide union-find loops (0: the default that the
     // tile count gives, see k_pixels.cu)
     uint32_t uf_cap;
     // optional (stage entry point): every pair's ClusterBounds and key in

@@ -836,7 +836,10 @@ static void apply_limits(const atag_limits& L, FrameDesc* d) {
     }
     if (L.cluster_capacity) d->cluster_cap = std::min(d->cluster_cap, L.cluster_capacity);
     if (L.cluster_point_capacity) d->cpoint_cap = std::min(d->cpoint_cap, L.cluster_point_capacity);
-    d->uf_cap = L.uf_iteration_cap;
+    // loops take four times a caller's cap: a union's iterations are those of both
+    // its walks and of all retries, and unions that end where the walks meet leave
+    // longer chains than walks to the roots would
+    d->uf_cap = 4u * std::min(L.uf_iteration_cap, 1u << 28);
 }
 
 // The device table of frame descriptors a call's kernels read.  Eager calls

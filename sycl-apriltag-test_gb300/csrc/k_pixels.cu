@@ -150,19 +150,16 @@ constexpr int CCL_BX = 32;  // blocks per tile row; CCL_BY (8, 16 or 32) rows is
 // step from its tile root, and the border pass only links roots of
 // components that touch a tile edge: at most two (one per colour) per edge
 // block, 2 (2 CCL_BX + 2 rows) edge blocks per tile, largest for 8-row
-// tiles.  So a chain, and the retries of one union (each moves to a
-// strictly smaller root), are bounded by uf_bound(w, h); a loop that gets
-// there flags ATAG_DEVFLAG_UF_ITERATION_CAP instead of spinning.
-// FrameDesc::uf_cap may lower the bound (0 keeps it).  Loops may take twice the
-// cap: unions that end where their walks meet compress the forest less than
-// walks to the root would, so chains are up to twice as long as those.
+// tiles.  So a chain is bounded by uf_bound(w, h), and a union, of whose two
+// slots each iteration lowers at least one (a retry too), by twice that.  A loop
+// that gets to the cap flags ATAG_DEVFLAG_UF_ITERATION_CAP instead of spinning.
+// FrameDesc::uf_cap may lower it (0 keeps the default, four times the bound).
 __device__ __forceinline__ uint32_t uf_bound(uint32_t w, uint32_t h) {
     const uint32_t tiles = ((w / 2 + CCL_BX - 1) / CCL_BX) * ((h / 2 + 7) / 8);
     return 2u * (2u * CCL_BX + 2u * 8u) * tiles + 2u;
 }
 __device__ __forceinline__ uint32_t uf_cap_of(const FrameDesc& F) {
-    const uint32_t bound = uf_bound(F.width, F.height);
-    return 2u * (F.uf_cap ? min(F.uf_cap, bound) : bound);
+    return F.uf_cap ? F.uf_cap : 4u * uf_bound(F.width, F.height);
 }
 
 // Which neighbour blocks (bit 0 P, 1 Q, 2 R, 3 S) a block links to in the
@@ -199,21 +196,19 @@ __device__ __forceinline__ BlockLinks block_links(PixelAt px, int x, int y, int 
     return BlockLinks{info, wm, bm};
 }
 
-// Lock-free union toward the smaller root (union_find.h:50-77); returns false
-// if a walk to the roots or the retries took `cap` iterations.  The border pass is bound by the
-// latency of these chains of parents, so both walks go in lock step, two levels
-// at a time with path halving (a parent is replaced by one of its ancestors,
-// which stays valid under concurrent unions), and end where they meet.  Walking
-// one after the other, each to its root, the pass took 26 us for one 1080p
-// frame (18 now), 55 for a 4K frame (27) and 244 for 64 1080p frames (180; 205
-// with 40 registers, six CTAs per SM instead of eight).
+// Lock-free union toward the smaller root (union_find.h:50-77) with a cap on the
+// iterations of both walks and all retries; returns false if it was hit.  The
+// border pass is bound by the latency of these chains of parents, so both walks
+// go in lock step, two levels at a time with path halving (a parent is replaced
+// by one of its ancestors, which stays valid under concurrent unions), and end
+// where they meet.  Walking one after the other, each to its root, the pass took
+// 26 us for one 1080p frame (18 now), 55 for a 4K frame (27) and 244 for 64 1080p
+// frames (180; 205 with 40 registers, six CTAs per SM instead of eight).
 // With a non-root in hand the union still only lowers parents (atomicMin), so
 // the forest stays acyclic and every later walk ends.
 template <typename Ptr>
 __device__ __forceinline__ bool uf_union(Ptr par, uint32_t a, uint32_t b, uint32_t cap) {
-    uint32_t steps = cap, tries = cap;  // left to this pair of walks, and to the union
-    while (true) {
-        if (steps == 0 || tries == 0) return false;
+    for (uint32_t it = 0; it < cap; it++) {
         const uint32_t pa = par[a], pb = par[b];
         if (pa == pb) return true;
         if (pa != a || pb != b) {
@@ -222,7 +217,6 @@ __device__ __forceinline__ bool uf_union(Ptr par, uint32_t a, uint32_t b, uint32
             if (gb != pb) par[b] = gb;
             a = ga;
             b = gb;
-            steps--;
             continue;
         }
         const uint32_t lo = min(a, b), hi = max(a, b);
@@ -230,9 +224,8 @@ __device__ __forceinline__ bool uf_union(Ptr par, uint32_t a, uint32_t b, uint32
         if (old == hi) return true;
         a = old;
         b = lo;
-        steps = cap;
-        tries--;
     }
+    return false;
 }
 
 // The same within a tile's shared-memory forest: both walks in lock step, so
@@ -644,7 +637,7 @@ __device__ __forceinline__ void ccl_final_impl(const FrameSet& fs) {
     const int w = F.width, h = F.height;
     const int npx = w / 4, by = blockIdx.y, px = blockIdx.x * CCL_FINAL_THREADS + threadIdx.x;  // w % 4 == 0
     const uint32_t* par = F.scratch;
-    const uint32_t cap = 2u * uf_cap_of(F);  // of one parent, a union's iterations being of two
+    const uint32_t cap = uf_cap_of(F);
     if (by < h / 2 && px < npx) {
         const size_t id = (size_t)(by * 2) * w + (size_t)px * 4;
         const uint4 p4 = *reinterpret_cast<const uint4*>(F.scratch + id);

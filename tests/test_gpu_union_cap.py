@@ -1,6 +1,6 @@
-"""The union-find iteration cap counts a union's walks and its retries apart: a
-cap that leaves room for both is not raised by unions that contend for long
-chains, call after call, and the labels are complete."""
+"""A union-find iteration cap with room for a union's two walks and its retries
+is not raised by unions that contend for long chains, call after call, and the
+labels are complete."""
 import numpy as np
 import pytest
 
