@@ -794,13 +794,25 @@ struct Buckets {
     }
 };
 
+constexpr uint32_t SPLIT_STEPS = 48, SPLIT_MIN = 512;
+
 // Sort of one cluster per CTA by (theta, packed point), the reference's
 // (cluster, slope) order (main.cpp:737-750) with ties fixed by the point, as
 // a bucket sort: count the buckets, prefix the counts, place the keys bucket
-// by bucket, then rank each key among its bucket's few keys (rounding of
-// theta leaves up to ~25 equal ones in the largest clusters): O(n), against
-// the log2(threads) merge rounds, and radix passes in global memory above
-// 16,384 keys, that it replaced.  Bound by instruction issue and the latency
+// by bucket, then rank each key among its bucket's.  In compact clusters those
+// are few (rounding of theta leaves up to ~25 equal ones in the largest): O(n),
+// against the log2(threads) merge rounds, and radix passes in global memory
+// above 16,384 keys, that it replaced.  On a thin slanted line theta takes few
+// values, and thousands of keys share one.  Where the buckets of one warp alone
+// would take SPLIT_STEPS comparisons per key of the cluster, the buckets are made
+// anew, cut by MAX_NB / 4 of the keys themselves, evenly sampled and sorted: a
+// key's bucket is then found by binary search, and whatever the shape a bucket
+// holds 4 n / MAX_NB keys on average.  A line of 10,700 keys takes 72 us (471
+// without, 90 by the merge sort), one of 15,200 keys 115 (1,235; 127), one of
+// 31,700 keys, past the shared memory, 281 (8,289; 584).  At 32, 64 and 128 steps
+// a key these and the frames below take the same; up to SPLIT_MIN keys, where all
+// of them in one bucket take some 5 us, nothing is counted.
+// Bound by instruction issue and the latency
 // of one CTA; sort and prefix sums of a lone 1080p frame 82 -> 42 us, of a 4K
 // stress frame 343 -> 100 us, of 64 1080p frames 750 -> 492 us (stage alone).
 // Keys are placed in shared memory, or for clusters over `cap` keys (frames
@@ -817,6 +829,9 @@ __device__ __forceinline__ void cluster_sort(const FrameSet& fs, const uint32_t*
     __shared__ long long red_m[6][MAX_RUNS];
     __shared__ uint32_t red32[W];
     __shared__ uint32_t s_item;
+    // of split clusters: MAX_NB / 4 counters, and the sorted samples
+    constexpr uint32_t SPLIT = MAX_NB / 4;
+    unsigned long long* cuts = reinterpret_cast<unsigned long long*>(hist + MAX_NB / 2);
     const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t total = work_offsets[n_frames];
     // a CTA's first cluster is its own index, later ones come from the queue
@@ -831,7 +846,14 @@ __device__ __forceinline__ void cluster_sort(const FrameSet& fs, const uint32_t*
         unsigned long long* X = n <= cap ? smem_keys : reinterpret_cast<unsigned long long*>(F.errbuf) + start;
         // about one bucket per key
         const uint32_t nb = min(max(256u, 1u << (32 - __clz((int)(n - 1u)))), MAX_NB);
-        const Buckets bucket(nb);
+        const Buckets theta_buckets(nb);
+        auto by_theta = [&](unsigned long long k) { return theta_buckets((uint32_t)(k >> 32)); };
+        auto by_cuts = [&](unsigned long long k) {  // the cuts above the first that are at most the key
+            uint32_t b = 0;
+#pragma unroll
+            for (uint32_t step = SPLIT / 2; step; step >>= 1) b += cuts[b + step] <= k ? step : 0u;
+            return b;
+        };
         for (uint32_t i = threadIdx.x; i < nb; i += THREADS) hist[i] = 0u;
         if (threadIdx.x == 0) s_item = gridDim.x + atomicAdd(work_counter, 1u);
         __syncthreads();
@@ -844,23 +866,31 @@ __device__ __forceinline__ void cluster_sort(const FrameSet& fs, const uint32_t*
             const uint32_t i = threadIdx.x + u * THREADS;
             key[u] = i < n ? __ldcg(src + i) : 0ull;
         }
+        // counts the buckets; a warp's part of them is [h0, h1).  False, where
+        // the buckets may be made anew, if ranking would take too many steps.
+        auto count = [&](auto bucket, uint32_t h0, uint32_t h1, bool may_split) {
 #pragma unroll
-        for (int u = 0; u < KEEP; u++) {
-            const uint32_t i = threadIdx.x + u * THREADS;
-            bkt[u] = bucket((uint32_t)(key[u] >> 32));
-            if (i < n) atomicAdd(&hist[bkt[u]], 1u);
-        }
-        for (uint32_t i = threadIdx.x + KEEP * THREADS; i < n; i += THREADS)
-            atomicAdd(&hist[bucket((uint32_t)(__ldcg(src + i) >> 32))], 1u);
-        __syncthreads();
-        // exclusive prefix: each warp takes a contiguous part, in rows of 32
-        {
-            const uint32_t per = max(nb / W, 32u), h0 = w * per, h1 = min(nb, h0 + per);
+            for (int u = 0; u < KEEP; u++) {
+                const uint32_t i = threadIdx.x + u * THREADS;
+                bkt[u] = bucket(key[u]);
+                if (i < n) atomicAdd(&hist[bkt[u]], 1u);
+            }
+            for (uint32_t i = threadIdx.x + KEEP * THREADS; i < n; i += THREADS) atomicAdd(&hist[bucket(__ldcg(src + i))], 1u);
+            __syncthreads();
             uint32_t sum = 0;
             for (uint32_t h = h0 + lane; h < h1; h += 32) sum += hist[h];
             sum = __reduce_add_sync(0xFFFFFFFFu, sum);
             if (lane == 0) red32[w] = sum;
-            __syncthreads();
+            if (!may_split) {
+                __syncthreads();
+                return true;
+            }
+            uint32_t steps = 0;  // n^2 < 2^31
+            for (uint32_t h = h0 + lane; h < h1; h += 32) steps += hist[h] * hist[h];
+            return !__syncthreads_or(__reduce_add_sync(0xFFFFFFFFu, steps) > SPLIT_STEPS * n);
+        };
+        // prefixes the counts, places the keys and ranks each in its bucket
+        auto order = [&](auto bucket, uint32_t h0, uint32_t h1) {
             uint32_t carry = __reduce_add_sync(0xFFFFFFFFu, lane < w ? red32[lane] : 0u);
             for (uint32_t h = h0 + lane; h < h1; h += 32) {
                 const uint32_t v = hist[h];
@@ -873,48 +903,64 @@ __device__ __forceinline__ void cluster_sort(const FrameSet& fs, const uint32_t*
                 hist[h] = carry + x - v;
                 carry += __shfl_sync(0xFFFFFFFFu, x, 31);
             }
-        }
-        __syncthreads();
+            __syncthreads();
 #pragma unroll
-        for (int u = 0; u < KEEP; u++)
-            if (threadIdx.x + u * THREADS < n) X[atomicAdd(&hist[bkt[u]], 1u)] = key[u];
-        for (uint32_t i = threadIdx.x + KEEP * THREADS; i < n; i += THREADS) {
-            const unsigned long long k = __ldcg(src + i);
-            X[atomicAdd(&hist[bucket((uint32_t)(k >> 32))], 1u)] = k;
-        }
-        __syncthreads();
-        // hist[b] is now the end of bucket b.  Two keys per thread and step,
-        // so their image reads overlap.
-        for (uint32_t i0 = threadIdx.x; i0 < n; i0 += 2 * THREADS) {
-            unsigned long long k[2];
-            uint32_t rank[2];
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const uint32_t i = i0 + u * THREADS;
-                k[u] = 0ull;
-                rank[u] = INVALID;
-                if (i >= n) continue;
-                k[u] = X[i];
-                const uint32_t b = bucket((uint32_t)(k[u] >> 32)), lo = b ? hist[b - 1] : 0u, hi = hist[b];
-                uint32_t r = lo;
-                for (uint32_t q = lo; q < i; q++) r += X[q] <= k[u] ? 1u : 0u;
-                for (uint32_t q = i + 1; q < hi; q++) r += X[q] < k[u] ? 1u : 0u;
-                rank[u] = r;
+            for (int u = 0; u < KEEP; u++)
+                if (threadIdx.x + u * THREADS < n) X[atomicAdd(&hist[bkt[u]], 1u)] = key[u];
+            for (uint32_t i = threadIdx.x + KEEP * THREADS; i < n; i += THREADS) {
+                const unsigned long long k = __ldcg(src + i);
+                X[atomicAdd(&hist[bucket(k)], 1u)] = k;
             }
-            unsigned long long v[2];
+            __syncthreads();
+            // hist[b] is now the end of bucket b.  Two keys per thread and step,
+            // so their image reads overlap.
+            for (uint32_t i0 = threadIdx.x; i0 < n; i0 += 2 * THREADS) {
+                unsigned long long k[2];
+                uint32_t rank[2];
 #pragma unroll
-            for (int u = 0; u < 2; u++) v[u] = linefit_rxyw((uint32_t)k[u], F.width, F.height, F.grey);
+                for (int u = 0; u < 2; u++) {
+                    const uint32_t i = i0 + u * THREADS;
+                    k[u] = 0ull;
+                    rank[u] = INVALID;
+                    if (i >= n) continue;
+                    k[u] = X[i];
+                    const uint32_t b = bucket(k[u]), lo = b ? hist[b - 1] : 0u, hi = hist[b];
+                    uint32_t r = lo;
+                    for (uint32_t q = lo; q < i; q++) r += X[q] <= k[u] ? 1u : 0u;
+                    for (uint32_t q = i + 1; q < hi; q++) r += X[q] < k[u] ? 1u : 0u;
+                    rank[u] = r;
+                }
+                unsigned long long v[2];
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                if (rank[u] == INVALID) continue;
-                const uint32_t packed = (uint32_t)k[u];
-                atag_cluster_point cp;
-                cp.packed_x = (uint16_t)packed;
-                cp.packed_y = (uint16_t)(packed >> 16);
-                cp.slope = float_from_order_key((uint32_t)(k[u] >> 32));
-                F.cluster_points[start + rank[u]] = cp;
-                __stcg(src + rank[u], v[u]);
+                for (int u = 0; u < 2; u++) v[u] = linefit_rxyw((uint32_t)k[u], F.width, F.height, F.grey);
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    if (rank[u] == INVALID) continue;
+                    const uint32_t packed = (uint32_t)k[u];
+                    atag_cluster_point cp;
+                    cp.packed_x = (uint16_t)packed;
+                    cp.packed_y = (uint16_t)(packed >> 16);
+                    cp.slope = float_from_order_key((uint32_t)(k[u] >> 32));
+                    F.cluster_points[start + rank[u]] = cp;
+                    __stcg(src + rank[u], v[u]);
+                }
             }
+        };
+        // each warp takes a contiguous part of the buckets, in rows of 32
+        const uint32_t per = max(nb / W, 32u), h0 = w * per, h1 = min(nb, h0 + per);
+        if (count(by_theta, h0, h1, n > SPLIT_MIN)) {
+            order(by_theta, h0, h1);
+        } else {
+            for (uint32_t i = threadIdx.x; i < SPLIT; i += THREADS) {
+                hist[i] = 0u;
+                cuts[i] = __ldcg(src + i * n / SPLIT);
+            }
+            __syncthreads();
+            bitonic_sort_u64(cuts, SPLIT);
+            static_assert(SPLIT % (32 * W) == 0, "rows of 32 buckets per warp");
+            const uint32_t s0 = w * (SPLIT / W), s1 = s0 + SPLIT / W;
+            count(by_cuts, s0, s1, false);
+            order(by_cuts, s0, s1);
         }
         __syncthreads();
         // moments of each run of CE_RUN points: W, Mx and My fit 32 bits (W <=
