@@ -233,24 +233,48 @@ __global__ void __launch_bounds__(256) k_stage_cluster_out(const __grid_constant
 // over the clusters, then each cluster's corners sorted in shared memory.
 // The reference's sort leaves ties unordered; here they go by position.
 // ---------------------------------------------------------------------------
-// One CTA per cluster, a cluster's errors read PK_UNROLL per thread at a time:
-// bound by the latency of the largest clusters' loads.  With a warp per cluster
-// the counts took 68 us for 1292 x 964 (9 now), the sort on 256 threads 37 (19
-// on 1024).
+// Bound by the latency of the loads.  Clusters of up to PK_WARP points take a
+// warp each, larger ones a CTA of 1024 threads, PK_UNROLL points per thread at
+// once.  Clusters go round the CTAs first, then their warps, so that a few use
+// every SM.  With a warp for clusters of any size the counts of 1292 x 964 took
+// 68 us (9 now), the sort on 256 threads 37 (19 on 1024); with a CTA for clusters
+// of any size 65,535 clusters of 24 points took 887 us in all (107 now, 671 on
+// warps and 256 threads), 4,000 of them 69 (17, 57).
 constexpr int PK_UNROLL = 4;
+constexpr uint32_t PK_WARP = 32 * PK_UNROLL * 2, PK_WARPS = 32;
 
-__global__ void __launch_bounds__(1024) k_peaks_count(const atag_corner* __restrict__ found,
+__global__ void __launch_bounds__(32 * PK_WARPS) k_peaks_count(const atag_corner* __restrict__ found,
                                                      const atag_cluster_extents* __restrict__ ext,
                                                      uint32_t n_clusters, uint32_t* __restrict__ counts) {
-    __shared__ uint32_t red[33];
-    for (uint32_t c = blockIdx.x; c < n_clusters; c += gridDim.x) {
-        const atag_cluster_extents e = ext[c];
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    __shared__ uint32_t red[33], s_large[PK_WARPS];
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    auto count = [&](const atag_cluster_extents& e, uint32_t first, uint32_t step) {
         uint32_t k = 0;
 #pragma unroll PK_UNROLL
-        for (uint32_t i = threadIdx.x; i < e.count; i += blockDim.x)
-            k += found[(size_t)e.start + i].error != 0.0f ? 1u : 0u;
-        k = block_sum_u32(k, red);
-        if (threadIdx.x == 0) counts[c] = k;
+        for (uint32_t i = first; i < e.count; i += step) k += found[(size_t)e.start + i].error != 0.0f ? 1u : 0u;
+        return k;
+    };
+    for (uint32_t c0 = blockIdx.x; c0 < n_clusters; c0 += gridDim.x * PK_WARPS) {
+        const uint32_t c = c0 + gridDim.x * wid;
+        uint32_t large = INVALID;
+        if (c < n_clusters) {
+            const atag_cluster_extents e = ext[c];
+            if (e.count > PK_WARP) {
+                large = c;
+            } else {
+                const uint32_t k = __reduce_add_sync(FULL, count(e, lane, 32));
+                if (lane == 0) counts[c] = k;
+            }
+        }
+        if (lane == 0) s_large[wid] = large;
+        __syncthreads();
+        for (unsigned m = __ballot_sync(FULL, s_large[lane] != INVALID); m; m &= m - 1) {
+            const uint32_t cl = s_large[__ffs(m) - 1];
+            const uint32_t k = block_sum_u32(count(ext[cl], threadIdx.x, blockDim.x), red);
+            if (threadIdx.x == 0) counts[cl] = k;
+        }
+        __syncthreads();
     }
 }
 
@@ -279,45 +303,81 @@ __global__ void __launch_bounds__(1024) k_peaks_offsets(const uint32_t* __restri
     }
 }
 
-__global__ void __launch_bounds__(1024) k_peaks_sort(const atag_corner* __restrict__ found,
+__global__ void __launch_bounds__(32 * PK_WARPS) k_peaks_sort(const atag_corner* __restrict__ found,
                                                     const atag_cluster_extents* __restrict__ ext,
                                                     uint32_t n_clusters, const uint32_t* __restrict__ counts,
                                                     const uint32_t* __restrict__ offsets,
                                                     atag_corner* __restrict__ out, uint32_t corner_cap,
                                                     uint32_t* __restrict__ d_counts) {
+    constexpr unsigned FULL = 0xFFFFFFFFu;
     extern __shared__ unsigned long long pk_keys[];
-    __shared__ uint32_t s_n;
-    for (uint32_t c = blockIdx.x; c < n_clusters; c += gridDim.x) {
-        const uint32_t k = counts[c];
-        if (k == 0) continue;  // uniform over the block
-        if (k > PK_SORT_CAP) {
-            // more corners than a cluster of valid points can have
-            if (threadIdx.x == 0) atomicOr(d_counts + 2, ATAG_DEVFLAG_SORT_OVERFLOW);
-            continue;
-        }
-        const atag_cluster_extents e = ext[c];
-        if (threadIdx.x == 0) s_n = 0;
-        __syncthreads();
-        // key: error descending (complemented order key), then position
-        for (uint32_t i0 = threadIdx.x; i0 < e.count; i0 += PK_UNROLL * blockDim.x) {
-            float err[PK_UNROLL];
-#pragma unroll
-            for (int u = 0; u < PK_UNROLL; u++) {
-                const uint32_t i = i0 + u * blockDim.x;
-                err[u] = i < e.count ? found[(size_t)e.start + i].error : 0.0f;
+    __shared__ uint32_t s_n, s_large[PK_WARPS];
+    static_assert(PK_WARPS * PK_WARP <= PK_SORT_CAP, "a warp's share of the keys");
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    // key: error descending (complemented order key), then position
+    auto key_of = [](float err, uint32_t i) { return ((unsigned long long)(~float_order_key(err)) << 32) | i; };
+    for (uint32_t c0 = blockIdx.x; c0 < n_clusters; c0 += gridDim.x * PK_WARPS) {
+        const uint32_t cw = c0 + gridDim.x * wid, kw = cw < n_clusters ? counts[cw] : 0u;
+        uint32_t large = INVALID;
+        if (kw) {
+            const atag_cluster_extents e = ext[cw];
+            if (e.count > PK_WARP) {
+                large = cw;
+            } else {
+                // keys listed by ballots, each corner put at its key's rank
+                unsigned long long* keys = pk_keys + wid * PK_WARP;
+                uint32_t n = 0;
+#pragma unroll PK_UNROLL
+                for (uint32_t i0 = 0; i0 < e.count; i0 += 32) {
+                    const uint32_t i = i0 + lane;
+                    const float err = i < e.count ? found[(size_t)e.start + i].error : 0.0f;
+                    const unsigned m = __ballot_sync(FULL, err != 0.0f);
+                    if (err != 0.0f) keys[n + (uint32_t)__popc(m & ((1u << lane) - 1u))] = key_of(err, i);
+                    n += (uint32_t)__popc(m);
+                }
+                __syncwarp();
+                const uint32_t off = offsets[cw];
+                for (uint32_t j = lane; j < n; j += 32) {
+                    const unsigned long long key = keys[j];
+                    uint32_t r = 0;
+                    for (uint32_t q = 0; q < n; q++) r += keys[q] < key ? 1u : 0u;
+                    if (off + r < corner_cap) out[off + r] = found[(size_t)e.start + (uint32_t)key];
+                }
             }
-#pragma unroll
-            for (int u = 0; u < PK_UNROLL; u++) {
-                if (err[u] == 0.0f) continue;
-                const uint32_t at = atomicAdd(&s_n, 1u);
-                if (at < k) pk_keys[at] = ((unsigned long long)(~float_order_key(err[u])) << 32) | (i0 + u * blockDim.x);
-            }
         }
+        if (lane == 0) s_large[wid] = large;
         __syncthreads();
-        bitonic_sort_u64(pk_keys, k);
-        const uint32_t off = offsets[c];
-        for (uint32_t j = threadIdx.x; j < k; j += blockDim.x)
-            if (off + j < corner_cap) out[off + j] = found[(size_t)e.start + (uint32_t)pk_keys[j]];
+        for (unsigned m = __ballot_sync(FULL, s_large[lane] != INVALID); m; m &= m - 1) {
+            const uint32_t c = s_large[__ffs(m) - 1], k = counts[c];
+            if (k > PK_SORT_CAP) {
+                // more corners than a cluster of valid points can have
+                if (threadIdx.x == 0) atomicOr(d_counts + 2, ATAG_DEVFLAG_SORT_OVERFLOW);
+                continue;
+            }
+            const atag_cluster_extents e = ext[c];
+            if (threadIdx.x == 0) s_n = 0;
+            __syncthreads();
+            for (uint32_t i0 = threadIdx.x; i0 < e.count; i0 += PK_UNROLL * blockDim.x) {
+                float err[PK_UNROLL];
+#pragma unroll
+                for (int u = 0; u < PK_UNROLL; u++) {
+                    const uint32_t i = i0 + u * blockDim.x;
+                    err[u] = i < e.count ? found[(size_t)e.start + i].error : 0.0f;
+                }
+#pragma unroll
+                for (int u = 0; u < PK_UNROLL; u++) {
+                    if (err[u] == 0.0f) continue;
+                    const uint32_t at = atomicAdd(&s_n, 1u);
+                    if (at < k) pk_keys[at] = key_of(err[u], i0 + u * blockDim.x);
+                }
+            }
+            __syncthreads();
+            bitonic_sort_u64(pk_keys, k);
+            const uint32_t off = offsets[c];
+            for (uint32_t j = threadIdx.x; j < k; j += blockDim.x)
+                if (off + j < corner_cap) out[off + j] = found[(size_t)e.start + (uint32_t)pk_keys[j]];
+            __syncthreads();
+        }
         __syncthreads();
     }
 }
