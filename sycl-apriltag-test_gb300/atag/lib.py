@@ -130,9 +130,13 @@ def init(device: int = None):
 
 
 def current_stream() -> int:
-    """The handle of torch's current stream, without a Stream object."""
+    """The handle of torch's current stream; without a Stream object where this
+    torch has the call for that."""
     import torch
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is None:
+        return torch.cuda.current_stream().cuda_stream
+    return raw(torch.cuda.current_device())
 
 
 def launch_count() -> int:
