@@ -310,7 +310,9 @@ __device__ __forceinline__ float bounds_dot(uint32_t xmin, uint32_t xmax, uint32
     return r;
 }
 
-// ValidBlobFilter, cluster_bounds.h:85-120
+// ValidBlobFilter, cluster_bounds.h:85-120.  No cluster below its fixed gate is
+// kept, which k_cluster_lines counts on.
+constexpr uint32_t MIN_CLUSTER_POINTS = 24;
 struct FilterParams {
     uint32_t min_cluster_pixels;
     uint32_t max_cluster_pixels;  // 2 * (2 w + 2 h)
@@ -321,7 +323,7 @@ __device__ __forceinline__ bool valid_blob(const FilterParams& f, uint32_t count
                                            uint32_t xmax, uint32_t ymin, uint32_t ymax, int gx_sum,
                                            int gy_sum, long long pxgx) {
     if (count < f.min_cluster_pixels) return false;
-    if (count < 24) return false;
+    if (count < MIN_CLUSTER_POINTS) return false;
     if (count > f.max_cluster_pixels) return false;
     if ((uint32_t)((int)(xmax - xmin) * (int)(ymax - ymin)) < f.tag_width) return false;
     bool reversed = bounds_dot(xmin, xmax, ymin, ymax, gx_sum, gy_sum, pxgx) < 0.0f;

@@ -1056,7 +1056,7 @@ __global__ void __launch_bounds__(CF_LARGE_THREADS, 1) k_cluster_sort_large(cons
 // 64 frames of 1080p took 125 + 197 us and a lone frame 10 + 30 us, now 277 and
 // 20 us (with the cheaper hypotf and conversions in both: 125 + 235 and 10 + 16).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t cyclic(int i, int n) {  // i in [-n, 3n)
+__device__ __forceinline__ uint32_t cyclic(int i, int n) {  // i in [-n, 3n): n is at least CE_MARGIN
     if (i < 0) i += n;
     while (i >= n) i -= n;
     return (uint32_t)i;
@@ -1101,6 +1101,9 @@ __device__ __forceinline__ float window_fit_error(const ShortMoment& m, uint32_t
 }
 
 constexpr uint32_t CE_MARGIN = 24;                           // window (20) and filter (3) reach, and a neighbour
+// A run's margins go round the cluster at most once, and its windows reach at
+// least two points to either side (fewer give no error, fit_quad.cpp:202-225).
+static_assert(CE_MARGIN <= MIN_CLUSTER_POINTS && MIN_CLUSTER_POINTS / 12 >= 2, "smallest cluster of the window errors");
 constexpr uint32_t CE_SPAN = CE_RUN + 2 * CE_MARGIN;         // points a warp scans
 constexpr uint32_t CE_ERRS = CE_RUN + 8;                     // errors of positions -4 .. CE_RUN + 3
 // Sums of the points before local index j at [CE_BASE + j]: the base keeps a
