@@ -90,7 +90,9 @@ __global__ void __launch_bounds__(128) k_do_indexing(const atag_peak_extents* __
     for (size_t q = blockIdx.x + (size_t)gridDim.x * wid; q < count; q += (size_t)gridDim.x * 4) {
         const atag_peak_extents pe = extents[q];
         const atag_cluster_extents ce = cluster_extents[q];
-        const uint32_t idx = lane < min(pe.count, 10u) ? corners[pe.start + lane].line_fit_point_index : 0u;
+        // fewer than four corners make no quad and are not read
+        const uint32_t used = pe.count < 4u ? 0u : min(pe.count, 10u);
+        const uint32_t idx = lane < used ? corners[pe.start + lane].line_fit_point_index : 0u;
         QuadSide side;
         index_one_cluster(pe.count, idx, points + ce.start, ce.count, max_mse, cos_critical, T[wid], fitted + q, side);
         __syncwarp();
