@@ -14,14 +14,19 @@ __device__ __forceinline__ uint32_t hash_key(unsigned long long k) {
     return (uint32_t)((k * 0x9E3779B97F4A7C15ull) >> 32);
 }
 
-__device__ __forceinline__ uint32_t global_insert(const FrameDesc& F, unsigned long long key) {
+// The slot of a key, inserted if it is new; INVALID after `probes` slots of
+// other keys.
+__device__ __forceinline__ uint32_t global_insert(const FrameDesc& F, unsigned long long key, uint32_t probes) {
     uint32_t mask = F.pair_cap - 1, h = hash_key(key) & mask;
-    for (uint32_t p = 0; p < F.pair_cap; p++) {
+    for (uint32_t p = 0; p < probes; p++) {
         unsigned long long k = atomicCAS(&F.pair_keys[h], EMPTY_KEY, key);
         if (k == EMPTY_KEY || k == key) return h;
         h = (h + 1) & mask;
     }
     return INVALID;
+}
+__device__ __forceinline__ uint32_t global_insert(const FrameDesc& F, unsigned long long key) {
+    return global_insert(F, key, F.pair_cap);
 }
 __device__ __forceinline__ uint32_t global_lookup(const FrameDesc& F, unsigned long long key) {
     uint32_t mask = F.pair_cap - 1, h = hash_key(key) & mask;

@@ -331,13 +331,13 @@ __device__ __forceinline__ void boundaries_pairs_impl(const FrameSet& fs, uint32
                     if (lane == 0) {
                         // a key new to the tile also takes its slot in the frame's
                         // table now, so the merge below needs one round trip less
+                        // (0.3% of a batch); by one try only, since a full table
+                        // has all its slots tried: the merge does that with a
+                        // thread per key, where a warp after the other's first
+                        // lane took 99 instead of 54 ms for 32 overflowing frames
                         bool fresh = false;
                         ls = local_insert(T, key, &fresh);
-                        if (fresh) {
-                            const uint32_t gs = global_insert(F, key);
-                            if (gs == INVALID) atomicOr(F.counters + CNT_STATUS, ATAG_DEVFLAG_PAIR_OVERFLOW);
-                            T.gslot[ls] = gs;
-                        }
+                        if (fresh) T.gslot[ls] = global_insert(F, key, 1);
                     }
                     ls = __shfl_sync(FULL, ls, 0);
                     cnt = rows = xmx = 0u;
@@ -384,8 +384,14 @@ __device__ __forceinline__ void boundaries_pairs_impl(const FrameSet& fs, uint32
     for (int i = threadIdx.x; i < BP_LC; i += blockDim.x) {
         unsigned long long key = T.key[i];
         if (key == EMPTY_KEY) continue;
-        const uint32_t gs = T.gslot[i];  // INVALID: the frame's table was full (flagged)
-        if (gs == INVALID) continue;
+        uint32_t gs = T.gslot[i];
+        if (gs == INVALID) {  // its first slot held another key
+            gs = global_insert(F, key);
+            if (gs == INVALID) {  // the frame's table is full
+                atomicOr(F.counters + CNT_STATUS, ATAG_DEVFLAG_PAIR_OVERFLOW);
+                continue;
+            }
+        }
         uint32_t old = global_flush(F, key, gs, T.cnt[i], T.xmin[i], T.xmax[i], T.ymin[i], T.ymax[i], T.gx[i], 0,
                                     (unsigned long long)(long long)T.pxgx[i]);
         T.gslot[i] = (old + T.cnt[i] > max_pixels) ? INVALID : gs;
