@@ -143,8 +143,8 @@ def stage_bytes(stats, n_src_px):
         "boundaries_pairs": 4 * N + 8 * Pf,     # read labels; write the listed points (>= surviving ones)
         "pairs_finalize": 48 * C,
         "scatter_points": 8 * Pf + 8 * Pf,      # read listed points, write sort keys
-        "cluster_sort": (8 + 4 + 8 + 64) * Pf,  # keys, grey taps, ClusterPoints, prefix sums
-        "cluster_errors": 48 * Pf,              # each prefix sum read once
+        "cluster_sort": (8 + 4 + 8 + 8) * Pf,   # keys, grey taps, ClusterPoints, line-fit inputs
+        "cluster_errors": (8 + 64) * Pf,        # read the inputs, write the prefix sums
         "index_quads": Cp * (120 + 90 * 2 * 48 + 272),
     }
 
@@ -170,8 +170,8 @@ def survey_bytes(stats):
         "boundaries_pairs": 4 * N + 4 * N + 12 * P,
         "pairs_finalize": 32 * C,
         "scatter_points": 12 * P + 32 * C + 10 * Pf,
-        "cluster_sort": 2 * 10 * Pf + (8 + 4 + 48) * Pf + 2 * 48 * Pf,
-        "cluster_errors": 48 * Pf * 2 + 2 * Pf + 12 * K,
+        "cluster_sort": 2 * 10 * Pf + (8 + 4 + 48) * Pf,
+        "cluster_errors": 2 * 48 * Pf + 48 * Pf * 2 + 2 * Pf + 12 * K,  # with the scan of the prefix sums
         "index_quads": 2 * 12 * K + Cp * (8 + 120 + 4 * 2 * 48) + 272 * Cp,  # with the choice of the 10 best peaks
     }
 
