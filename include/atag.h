@@ -563,8 +563,8 @@ atag_status atag_estimate_pose(const float *d_corners, size_t corner_stride, siz
 /* library's own terms.                                                  */
 /* ------------------------------------------------------------------ */
 #define ATAG_DECODE_REORDERED 0x1u    /* corners were wound the other way        */
-#define ATAG_DECODE_DEGENERATE 0x2u   /* no homography, or part of the tag
-                                         projects behind the camera            */
+#define ATAG_DECODE_DEGENERATE 0x2u   /* no homography, a corner that is not finite, or part
+                                         of the tag projects behind the camera */
 #define ATAG_DECODE_LOW_CONTRAST 0x4u /* white minus black grey model at the tag
                                          centre below min_contrast, or a model
                                          without enough samples: no bits read  */

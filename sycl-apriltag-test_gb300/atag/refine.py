@@ -63,7 +63,7 @@ class RefineCorners(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, image, corners):
-        # the samples and their gradient (4 KB each per quad) are not asked for
+        # the samples and their gradient (1 KB each per quad) are not asked for
         refined, residual, _ = _forward(image.detach(), corners.detach(), False)
         ctx.save_for_backward(image, corners)
         return refined, residual

@@ -119,8 +119,9 @@ struct FrameSet {
 // The compiler may move a read-only load (__ldg, const __restrict__) up across
 // the wait, so one of data that an earlier kernel wrote goes through a
 // descriptor's pointer that is itself read, by a plain load, after it.
-// Large lanes run without: the calls alone made their pixel kernels, of up to
-// half a million short CTAs, 1-4% slower, so those are compiled both ways.
+// Large lanes beside others run without (launch_lane), and so do captures: the
+// calls alone made their pixel kernels, of up to half a million short CTAs, 1-4%
+// slower, so those are compiled both ways.
 __device__ __forceinline__ void await_previous_kernel() {
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();

@@ -943,7 +943,11 @@ static atag_status launch_lane(atag_detector* det, const FrameDesc* d_table, con
     // 185, but 960x540 128 -> 135 and 3840x2160 348 -> 358).  The waiting CTAs
     // also keep another lane's off the SMs: with two lanes of 8 megapixels and
     // more, batches of unequal frames lost up to 4% (64 frames 2907 -> 3036
-    // us), while lanes below 6 gained.
+    // us), while lanes below 6 gained.  A lone lane has no other beside it and
+    // gains at every size of 1080p and 4K batches (4, 8, 32, 64 frames of 1080p
+    // 325 -> 304, 505 -> 484, 1558 -> 1534, 2934 -> 2917 us; 8 of 4K 1668 ->
+    // 1665); only very many small frames lose (64 of 640x480 496 -> 500, 128 860
+    // -> 897).
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(s, &cs));
     const bool overlap =

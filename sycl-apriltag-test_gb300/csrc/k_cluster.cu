@@ -123,7 +123,11 @@ __device__ __forceinline__ unsigned long long pair_labels(unsigned long long key
 // key's lanes were ~480 instructions per 32 points.  A strip's points belong
 // to 1.4 pairs on average, so a warp keeps one pair's sums in registers across
 // its rounds and reduces them when the pair changes.  64 frames of 1080p 926
-// -> 877 us.
+// -> 877 us.  Strips of many pairs pay for the changes: 32 frames of diagonal
+// stripes, 6 px wide, take 2,090 us instead of 1,500.  Lanes that add their own
+// points there need 650, but choosing between the two costs the others 5-25% of
+// the pass: the kernel has 32 registers (eight CTAs per SM) and spills 44 bytes
+// already.
 template <int BP_H>
 __device__ __forceinline__ void boundaries_pairs_impl(const FrameSet& fs, uint32_t min_size) {
     constexpr int BP_SH = BP_H + 1;

@@ -49,8 +49,8 @@
 //   * the edge's direction comes from square roots, not atan2/sin/cos;
 //   * both grey models are solved at once, on even and odd lanes.
 // 4,096 quads against 587 codes: 4,072 FP64 warp instructions per quad and
-// 1,178 us before; about 620 and 229 us now (597 and 219 without the FP64
-// positions on pixel borders and the quotients and cell centres of `project`).
+// 1,178 us before; 615 and 229 us now (597 and 219 without the FP64 positions
+// on pixel borders and the quotients and cell centres of `project`).
 #include <vector>
 
 #include "atag_edge_samples.cuh"

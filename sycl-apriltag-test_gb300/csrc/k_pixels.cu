@@ -203,7 +203,8 @@ __device__ __forceinline__ BlockLinks block_links(PixelAt px, int x, int y, int 
 // by one of its ancestors, which stays valid under concurrent unions), and end
 // where they meet.  Walking one after the other, each to its root, the pass took
 // 26 us for one 1080p frame (18 now), 55 for a 4K frame (27) and 244 for 64 1080p
-// frames (180; 205 with 40 registers, six CTAs per SM instead of eight).
+// frames (180; 205 with 40 registers, six CTAs per SM instead of eight; at 32 the
+// 16- and 32-row forms spill 24 bytes).
 // With a non-root in hand the union still only lowers parents (atomicMin), so
 // the forest stays acyclic and every later walk ends.
 template <typename Ptr>
