@@ -819,12 +819,12 @@ constexpr uint32_t SPLIT_STEPS = 48, SPLIT_MIN = 512;
 // key's bucket is then found by binary search, and whatever the shape a bucket
 // holds 4 n / MAX_NB keys on average.  A line of 10,700 keys takes 72 us (471
 // without, 90 by the merge sort), one of 15,200 keys 115 (1,235; 127), one of
-// 31,700 keys, past the shared memory, 281 (8,289; 584).  At 32, 64 and 128 steps
-// a key these and the frames below take the same; up to SPLIT_MIN keys, where all
-// of them in one bucket take some 5 us, nothing is counted.
-// Bound by instruction issue and the latency
-// of one CTA; sort and prefix sums of a lone 1080p frame 82 -> 42 us, of a 4K
-// stress frame 343 -> 100 us, of 64 1080p frames 750 -> 492 us (stage alone).
+// 31,700 keys, past the shared memory, 281 (8,289; 584).  With 32 to 128 steps a
+// key these take about the same, lines of 1,650 keys 29 to 24; up to SPLIT_MIN
+// keys, where all of them in one bucket cost some 5 us, nothing is counted.
+// Bound by instruction issue and the latency of one CTA; sort and prefix sums of
+// a lone 1080p frame 82 -> 42 us, of a 4K stress frame 343 -> 100 us, of 64 1080p
+// frames 750 -> 492 us (stage alone, the prefix sums by a kernel of their own).
 // Keys are placed in shared memory, or for clusters over `cap` keys (frames
 // larger than 4K) in their segment of errbuf.  Results: ClusterPoints and, in
 // the segment of sortbuf, each point's line-fit inputs in sorted order; and
